@@ -600,7 +600,8 @@ __global__ void __launch_bounds__(kFThreads, 4)
       if (atomicAdd(o.done, 1ull) == (unsigned long long)n_groups - 1ull) {
         __threadfence();
         const int64_t m = *reinterpret_cast<volatile int64_t*>(o.total);
-        const int64_t err = (int64_t)f_load(&o.state[1]);
+        const int64_t err =
+            (int64_t)(f_load(&o.state[1]) | (b.bin_scan ? f_load(&b.bin_scan[1]) : 0ull));
         f_report(o, m, err);
       }
     }

@@ -25,7 +25,6 @@ namespace {
 constexpr int kSortThreads = 128;
 constexpr int kSortCap = 2048;  // elements sorted entirely in shared memory
 constexpr int64_t kRankSortMax = 512;  // bins up to this size: rank placement
-constexpr int kPlaceSplit = 8;         // threads per atom in the rank placement
 
 // Grid points p (0 <= p_a < nb_a) whose Morton code is smaller than that of c.
 __device__ int64_t morton_rank(const int32_t c[3], const int32_t nb[3]) {
@@ -120,6 +119,105 @@ __device__ void cta_bin_scan(const int32_t* __restrict__ bin_count, int64_t nb,
     grun += (v + 31) / 32;
   }
   if (tid == kPrepThreads - 1) bin_start[nb] = before + x;
+}
+
+// The same two scans over several CTAs, for grids above kPrepBinScanMax bins:
+// tiles of kBinTile bins by ticket, a bounded decoupled look-back over the
+// tiles before it.  Atoms and groups share one 62-bit value (31 bits each:
+// neither exceeds the 2^31 atoms of a system).  state (zeroed): [0] ticket,
+// [1] error word, [2 + t] tile t's look-back word.
+constexpr int kBinPer = 8;
+constexpr int kBinTile = kPrepThreads * kBinPer;
+constexpr int kBinShift = 62;
+constexpr uint64_t kBinAggregate = 1ull << kBinShift;
+constexpr uint64_t kBinInclusive = 2ull << kBinShift;
+constexpr uint64_t kBinValue = (1ull << kBinShift) - 1;
+constexpr uint64_t kBinAtoms = (1ull << 31) - 1;
+constexpr int kBinSpins = 1 << 22;
+
+__global__ void __launch_bounds__(kPrepThreads)
+    k_bin_scan(const int32_t* __restrict__ bin_count, int64_t nb, int64_t* __restrict__ bin_start,
+               int32_t* __restrict__ group_start, uint64_t* __restrict__ state) {
+  __shared__ uint64_t warp_tot[kPrepThreads / 32];
+  __shared__ uint64_t s_prefix;
+  __shared__ int64_t s_tile;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
+  if (tid == 0) s_tile = (int64_t)atomicAdd(reinterpret_cast<unsigned long long*>(state), 1ull);
+  __syncthreads();
+  const int64_t t = s_tile;
+  const int64_t b0 = t * kBinTile + (int64_t)tid * kBinPer;
+  uint64_t v[kBinPer], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kBinPer; ++k) {
+    const uint64_t c = b0 + k < nb ? (uint64_t)bin_count[b0 + k] : 0ull;
+    v[k] = ((c + 31) / 32) << 31 | c;
+    sum += v[k];
+  }
+  uint64_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_tot[warp] = x;
+  __syncthreads();
+  uint64_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kPrepThreads / 32; ++w) {
+    before += w < warp ? warp_tot[w] : 0ull;
+    all += warp_tot[w];
+  }
+  if (warp == 0) {
+    volatile uint64_t* tiles = state + 2;
+    if (lane == 0) {
+      __threadfence();
+      tiles[t] = (t == 0 ? kBinInclusive : kBinAggregate) | all;
+    }
+    uint64_t prefix = 0;
+    for (int64_t tt = t - 1; tt >= 0; tt -= 32) {
+      const int64_t pred = tt - lane;
+      uint64_t w = kBinInclusive;
+      if (pred >= 0) {
+        int spins = 0;
+        w = tiles[pred];
+        while ((w >> kBinShift) == 0 && spins < kBinSpins) {
+          __nanosleep(32);
+          w = tiles[pred];
+          ++spins;
+        }
+      }
+      if (__any_sync(0xffffffffu, (w >> kBinShift) == 0)) {
+        if (lane == 0) atomicExch(reinterpret_cast<unsigned long long*>(&state[1]), 1ull);
+        break;
+      }
+      const unsigned inc = __ballot_sync(0xffffffffu, (w >> kBinShift) == 2);
+      const int stop = __ffs(inc) - 1;
+      uint64_t add = pred >= 0 && lane <= (stop < 0 ? 31 : stop) ? (w & kBinValue) : 0ull;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+      prefix += add;
+      if (stop >= 0) break;
+    }
+    if (lane == 0) {
+      if (t > 0) {
+        __threadfence();
+        tiles[t] = kBinInclusive | (prefix + all);
+      }
+      s_prefix = prefix;
+    }
+  }
+  __syncthreads();
+  uint64_t run = s_prefix + before + x - sum;
+#pragma unroll
+  for (int k = 0; k < kBinPer; ++k) {
+    if (b0 + k < nb) {
+      bin_start[b0 + k] = (int64_t)(run & kBinAtoms);
+      group_start[b0 + k] = (int32_t)(run >> 31);
+    }
+    run += v[k];
+    if (b0 + k == nb - 1) bin_start[nb] = (int64_t)(run & kBinAtoms);
+  }
 }
 
 // Per atom: wrap, Morton key, bin rank, histogram.  With `done`, the last
@@ -403,14 +501,20 @@ __device__ void sort_bin(const GridParams& g, const double* __restrict__ pos, in
   if (p32 && threadIdx.x == 0) store_groups(g, r, s, e, lin0, groups, counters, group_start);
 }
 
-// Places every atom at its slot.  Blocks [0, atom_blocks): kPlaceSplit
-// threads per entry p of the bin segments k_scatter wrote (arbitrary order
-// inside a segment); for bins of at most kRankSortMax atoms the atom's place in its
+// Places every atom at its slot.  Blocks [0, atom_blocks): SPLIT threads per
+// entry p of the bin segments k_scatter wrote (arbitrary order inside a
+// segment); for bins of at most kRankSortMax atoms the atom's place in its
 // bin is the number of the bin's (key, index) pairs below its own (a rank
 // sort: the bin's pairs are read by each of its atoms, from L1), and the
 // thread writes the slot there directly; the atom placed first writes the
-// bin's group records.  Blocks from atom_blocks on: block atom_blocks + r
-// sorts bin r when it is larger (sort_bin).
+// bin's group records.  Blocks from atom_blocks on look at bin_span bins
+// each and sort the larger ones (sort_bin).
+//
+// SPLIT: small systems fill few warps and wait for the bin's loads, so 8
+// threads share an atom's count; large ones fill the chip, and there the
+// slot's FP64 work, done by one of the SPLIT threads, wants whole warps
+// (kPlaceWhole, launch_grid_build).
+template <int SPLIT>
 __global__ void __launch_bounds__(kSortThreads)
     k_place(GridParams g, const double* __restrict__ pos, int64_t n,
             const int32_t* __restrict__ rank, const int64_t* __restrict__ bin_start,
@@ -421,21 +525,32 @@ __global__ void __launch_bounds__(kSortThreads)
             GroupRec* __restrict__ groups, int32_t* __restrict__ irr_list,
             uint8_t* __restrict__ irr, int32_t* __restrict__ counters,
             float4* __restrict__ cbox, const int32_t* __restrict__ group_start,
-            int32_t atom_blocks) {
+            int32_t atom_blocks, int32_t bin_span) {
   __shared__ uint64_t sk[kSortCap];
   __shared__ int32_t sv[kSortCap];
   pdl_wait();
   if ((int32_t)blockIdx.x >= atom_blocks) {
-    const int64_t r = (int64_t)blockIdx.x - atom_blocks;
-    if (bin_start[r + 1] - bin_start[r] <= kRankSortMax) return;
-    sort_bin(g, pos, r, bin_start, skey, sidx, skey2, sidx2, px, py, pz, meta, p32, sbin, groups,
-             irr_list, irr, counters, cbox, group_start, sk, sv);
+    const int64_t r0 = (int64_t)(blockIdx.x - atom_blocks) * bin_span;
+    const int64_t end = r0 + bin_span < g.total_bins ? r0 + bin_span : g.total_bins;
+    for (int64_t r1 = r0; r1 < end; r1 += kSortThreads) {
+      if (bin_span > 1) {
+        const int64_t rt = r1 + threadIdx.x;
+        const bool big = rt < end && bin_start[rt + 1] - bin_start[rt] > kRankSortMax;
+        if (!__syncthreads_or(big)) continue;
+      }
+      for (int64_t r = r1; r < r1 + kSortThreads && r < end; ++r) {
+        if (bin_start[r + 1] - bin_start[r] <= kRankSortMax) continue;
+        sort_bin(g, pos, r, bin_start, skey, sidx, skey2, sidx2, px, py, pz, meta, p32, sbin,
+                 groups, irr_list, irr, counters, cbox, group_start, sk, sv);
+        __syncthreads();
+      }
+    }
     return;
   }
-  // (kPlaceSplit consecutive threads per entry, each counting a strided
-  // share of the bin: more loads in flight than one thread per atom)
-  const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kPlaceSplit;
-  const int part = (int)(threadIdx.x % kPlaceSplit);
+  // (SPLIT consecutive threads per entry, each counting a strided share of
+  // the bin: more loads in flight than one thread per atom)
+  const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / SPLIT;
+  const int part = (int)(threadIdx.x % SPLIT);
   if (p >= n) return;  // (the same for the entry's threads, as below)
   const uint64_t k = skey[p];
   const int32_t i = sidx[p];
@@ -443,12 +558,15 @@ __global__ void __launch_bounds__(kSortThreads)
   const int64_t s = bin_start[r], e = bin_start[r + 1];
   if (e - s > kRankSortMax) return;
   int32_t below = 0;
-  for (int64_t q = s + part; q < e; q += kPlaceSplit)
+#pragma unroll(SPLIT > 1 ? 1 : 4)
+  for (int64_t q = s + part; q < e; q += SPLIT)
     below += pair_less(__ldg(&skey[q]), __ldg(&sidx[q]), k, i) ? 1 : 0;
-  const unsigned group = ((1u << kPlaceSplit) - 1u) << (threadIdx.x & 31 & ~(kPlaceSplit - 1));
+  if (SPLIT > 1) {
+    const unsigned group = (unsigned)(((1ull << SPLIT) - 1ull) << (threadIdx.x & 31 & ~(SPLIT - 1)));
 #pragma unroll
-  for (int o = 1; o < kPlaceSplit; o <<= 1) below += __shfl_xor_sync(group, below, o);
-  if (part != 0) return;
+    for (int o = 1; o < SPLIT; o <<= 1) below += __shfl_xor_sync(group, below, o);
+    if (part != 0) return;
+  }
   const SlotOut so = store_slot(g, pos, s + below, i, px, py, pz, meta, p32, sbin, irr_list, irr,
                                 counters);
   if (p32 && below == 0) store_groups(g, r, s, e, so.lin, groups, counters, group_start);
@@ -512,7 +630,15 @@ __global__ void __launch_bounds__(kBoundsThreads)
   }
 }
 
+// Atoms from which the placement takes one thread per atom (a million atoms:
+// k_place<8> 215 us, and 42,875 CTAs of it only looked at one bin each).
+constexpr int64_t kPlaceWhole = 65536;
+// Most CTAs that look for bins too large for the rank placement.
+constexpr int64_t kSortBlocks = 1024;
+
 }  // namespace
+
+int64_t bin_scan_words(int64_t total_bins) { return 2 + (total_bins + kBinTile - 1) / kBinTile; }
 
 void launch_bounds(const double* pos, int64_t n, double* out, cudaStream_t s) {
   k_bounds<<<1, kBoundsThreads, 0, s>>>(pos, n, out);
@@ -526,18 +652,31 @@ void launch_grid_build(const GridParams& g, const double* pos, int64_t n, const 
     k_rank_table<<<(unsigned)((g.total_bins + T - 1) / T), T, 0, s>>>(g, b.rank_of_bin);
     note_launches(1);
   }
-  const bool fused = b.build_done != nullptr && g.total_bins <= kFusedBinScanMax;
+  const bool own_scan = b.build_done != nullptr && g.total_bins <= kPrepBinScanMax;
   k_prep<<<(unsigned)((n + kPrepThreads - 1) / kPrepThreads), kPrepThreads, 0, s>>>(
       g, pos, n, b.rank_of_bin, b.key, b.rank, b.bin_count, b.bin_start,
-      fused ? b.build_done : nullptr, fused ? b.group_start : nullptr, b.fill);
-  if (!fused) exclusive_scan_i32(b.bin_count, g.total_bins, b.bin_start, b.scan_tmp, s);
+      own_scan ? b.build_done : nullptr, own_scan ? b.group_start : nullptr, b.fill);
+  if (!own_scan && b.group_start && b.bin_scan) {
+    launch_pdl(k_bin_scan, dim3((unsigned)((g.total_bins + kBinTile - 1) / kBinTile)),
+               dim3(kPrepThreads), 0, s, (const int32_t*)b.bin_count, g.total_bins, b.bin_start,
+               b.group_start, b.bin_scan);
+    note_launches(1);
+  } else if (!own_scan) {
+    exclusive_scan_i32(b.bin_count, g.total_bins, b.bin_start, b.scan_tmp, s);
+  }
+  const bool grouped = b.group_start && (own_scan || b.bin_scan);
   launch_pdl(k_scatter, dim3((unsigned)((n + T - 1) / T)), dim3(T), 0, s, b.key, b.rank, n,
              b.bin_start, b.bin_fill, b.skey, b.sidx, (const int32_t*)b.fill);
-  const int32_t atom_blocks = (int32_t)((kPlaceSplit * n + kSortThreads - 1) / kSortThreads);
-  launch_pdl(k_place, dim3((unsigned)(atom_blocks + g.total_bins)), dim3(kSortThreads), 0, s, g,
+  const bool whole = n >= kPlaceWhole;
+  const int64_t split = whole ? 1 : 8;
+  const int32_t atom_blocks = (int32_t)((split * n + kSortThreads - 1) / kSortThreads);
+  const int64_t span = (g.total_bins + kSortBlocks - 1) / kSortBlocks;
+  const int64_t blocks = atom_blocks + (g.total_bins + span - 1) / span;
+  launch_pdl(whole ? k_place<1> : k_place<8>, dim3((unsigned)blocks), dim3(kSortThreads), 0, s, g,
              pos, n, (const int32_t*)b.rank, (const int64_t*)b.bin_start, b.skey, b.sidx, b.skey2,
              b.sidx2, b.px, b.py, b.pz, b.meta, b.p32, b.sbin, b.groups, b.irr_list, b.irr,
-             b.counters, b.cbox, fused ? (const int32_t*)b.group_start : nullptr, atom_blocks);
+             b.counters, b.cbox, grouped ? (const int32_t*)b.group_start : nullptr,
+             atom_blocks, (int32_t)span);
   note_launches(3);
   if (b.p32 && b.cbox) {
     int dev = 0, sms = 0;

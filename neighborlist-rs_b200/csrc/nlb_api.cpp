@@ -392,11 +392,15 @@ void* Ctx::raw(int slot, size_t bytes) {
     // Every slot comes from the stream-ordered pool (result arrays must, to
     // be handed over; the others so that a grown slot's old memory stays
     // mapped for the next allocation instead of being unmapped by cudaFree
-    // and mapped again by cudaMalloc).  Growth waits for the device first
-    // (the old array may still be in use on another stream, as a cudaFree
-    // would).
+    // and mapped again by cudaMalloc).  Growth waits for this context's own
+    // work: every call has either synchronised its stream before it returned
+    // or is followed by this stream (early_ev).  It must not wait for the
+    // whole device: with several server workers making their streams at the
+    // same time, cudaDeviceSynchronize crashed inside the driver (a null
+    // stream in cuCtxSynchronize, about one process in ten), and it held up
+    // every other worker.
     if (b.p) {
-      cudaDeviceSynchronize();
+      cudaStreamSynchronize(stream);
       if (b.pooled)
         cudaFreeAsync(b.p, stream);
       else
@@ -429,7 +433,8 @@ void release_thread_ctx() {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(c->device);
-    cudaDeviceSynchronize();
+    if (c->early_stream) cudaEventSynchronize(c->early_ev);
+    cudaStreamSynchronize(c->own_stream);
     for (Ctx::Buf& b : c->bufs) {
       if (b.p && b.pooled)
         cudaFreeAsync(b.p, c->own_stream);
@@ -643,7 +648,7 @@ Status count_system(Ctx& c, SystemPlan& sp, const double* d_pos) {
     e = cudaMemcpyAsync(c.h_small + k + 2, sp.gb.mask_top, sizeof(int64_t),
                         cudaMemcpyDeviceToHost, s);
   const bool bin_scan = sp.method == Method::kCellList &&
-                        !(sp.gb.build_done && sp.grid.total_bins <= kFusedBinScanMax);
+                        !(sp.gb.build_done && sp.grid.total_bins <= kPrepBinScanMax);
   c.h_small[k + 3] = 0;
   if (e == cudaSuccess && bin_scan)  // the separate bin scan's error word
     e = cudaMemcpyAsync(c.h_small + k + 3, sp.gb.scan_tmp + 1, sizeof(int64_t),

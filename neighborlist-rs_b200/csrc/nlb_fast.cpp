@@ -124,11 +124,15 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   const int64_t max_groups = n / 32 + std::min<int64_t>(n, nb) + 1;
   sp.fused_words = 2 + max_groups + 2;  // + total, completion count
   sp.zeroed_words = 2 * (size_t)nb + 6 +
-                    2 * (size_t)(sp.fused ? sp.fused_words : scan_tmp_elems(row));
+                    2 * (size_t)(sp.fused ? sp.fused_words : scan_tmp_elems(row)) +
+                    2 * (size_t)(sp.fused && nb > kPrepBinScanMax ? bin_scan_words(nb) : 0);
   int32_t* zeroed = slot<int32_t>(c, kSlotBinCount, sp.zeroed_words);
   sp.scan_state = zeroed ? reinterpret_cast<int64_t*>(zeroed + 2 * nb + 6) : nullptr;
   sp.fused_state = reinterpret_cast<uint64_t*>(sp.scan_state);
   sp.fused_total = sp.fused && zeroed ? sp.scan_state + 2 + max_groups : nullptr;
+  b.bin_scan = sp.fused && nb > kPrepBinScanMax && zeroed
+                   ? reinterpret_cast<uint64_t*>(sp.scan_state + sp.fused_words)
+                   : nullptr;
   b.group_start = sp.fused ? slot<int32_t>(c, kSlotGroupStart, nb) : nullptr;
   b.fill = slot<int32_t>(c, kSlotFill, n);
   b.bin_count = zeroed;
@@ -222,7 +226,7 @@ EmitTargets fast_targets(const SystemPlan& sp, int64_t capacity, int64_t* report
   t.report = report;
   t.mask_top = sp.gb.mask_top;
   // (grids too large for k_prep's own bin scan: the separate scan's error word)
-  t.grid_scan_error = sp.grid.total_bins > kFusedBinScanMax ? sp.gb.scan_tmp + 1 : nullptr;
+  t.grid_scan_error = sp.grid.total_bins > kPrepBinScanMax ? sp.gb.scan_tmp + 1 : nullptr;
   return t;
 }
 
@@ -290,8 +294,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
   FastState& fs = state_for(c);
   const int64_t n_cells = stencil_cells_of(sp.grid);
   sp.fused = single_pipeline_mode() == 0 && n_cells <= kFusedMaxCells &&
-             sp.grid.total_bins > 0 && sp.grid.total_bins <= kFusedBinScanMax &&
-             (double)sp.n / (double)sp.grid.total_bins <= kFusedMaxPerBin;
+             sp.grid.total_bins > 0 && (double)sp.n / (double)sp.grid.total_bins <= kFusedMaxPerBin;
   tl_last_fused = sp.fused ? 0 : 1;
   const double rc = std::sqrt(sp.rc_sq[0]);
   int64_t capacity = std::max<int64_t>(
@@ -415,9 +418,11 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
   // Grids too large for k_prep's own bin scan use a separate scan (state in
   // gb.scan_tmp): its error word too.
   c.h_small[3] = 0;
-  if (e == cudaSuccess && sp.grid.total_bins > kFusedBinScanMax)
-    e = cudaMemcpyAsync(c.h_small + 3, sp.gb.scan_tmp + 1, sizeof(int64_t),
-                        cudaMemcpyDeviceToHost, c.stream);
+  if (e == cudaSuccess && sp.grid.total_bins > kPrepBinScanMax)
+    e = cudaMemcpyAsync(c.h_small + 3,
+                        sp.fused ? reinterpret_cast<int64_t*>(sp.gb.bin_scan) + 1
+                                 : sp.gb.scan_tmp + 1,
+                        sizeof(int64_t), cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_fail(e, "neighbour-list pipeline");
   if (c.h_small[1] != 0 || c.h_small[3] != 0)

@@ -66,7 +66,7 @@ struct GridBuffers {
   int32_t* counters;
   // Optional (zeroed by the caller before the build): completion counter of
   // k_prep, whose last CTA then scans the bin histogram into bin_start
-  // itself (grids of at most kFusedBinScanMax bins); nullptr: separate scan.
+  // itself (grids of at most kPrepBinScanMax bins); nullptr: separate scan.
   int32_t* build_done;
   // Optional (zeroed by the caller before the build): task counter of the
   // pair-task emit pass, which then hands tasks out dynamically on dense
@@ -91,7 +91,7 @@ struct GridBuffers {
   // pass skips a (group, chunk) pair whose boxes are farther apart than the
   // guard band's upper bound by more than the band's width.
   float4* cbox;
-  // Optional ([total_bins], written by k_prep's own bin scan): canonical
+  // Optional ([total_bins], written by the bin scan): canonical
   // index of each bin's first group; the build then stores groups[] in
   // canonical order (bins in rank order, runs in slot order).
   int32_t* group_start;
@@ -99,12 +99,21 @@ struct GridBuffers {
   // from the histogram (k_scatter then needs no atomics); nullptr: k_scatter
   // takes places from bin_fill.
   int32_t* fill;
+  // Optional: state words of the bin scan of grids above kPrepBinScanMax bins
+  // (bin_scan_words(total_bins), zeroed by the caller before the build; used
+  // when group_start is set); [1] is its error word.
+  uint64_t* bin_scan;
 };
 
 // Grids with at least this many atoms per bin on average get chunk boxes.
 constexpr double kChunkPruneMinPerBin = 64.0;
 
-constexpr int64_t kFusedBinScanMax = 65536;
+// Grids of at most this many bins are scanned by k_prep's last CTA, which
+// saves a launch (about 3 us).  That CTA alone took most of k_prep's 119 us at
+// 42,875 bins (a million atoms); above the line the scan is a launch over
+// several CTAs.
+constexpr int64_t kPrepBinScanMax = 4096;
+int64_t bin_scan_words(int64_t total_bins);
 
 // need_rank_table = false reuses rank_of_bin from a previous build with the
 // same bins per axis.
