@@ -15,9 +15,7 @@ exact-sized edge_index int64 (2, M) and shift int32 (M, 3)).
                (neighborlist_rs.build_neighborlists: numpy positions in, numpy
                edge arrays out), host<->device copies inside the timed region.
 * roofline   : the dominant kernel's algorithmic bytes / its CUDA-event time
-               (the one-launch search on the headline's sparse grid; the emit
-               pass, with the count pass beside it, on grids that keep the
-               three launches).
+               (the emit pass, with the count pass beside it).
 * cpu_baseline: the CPU oracle (C++ restatement of the reference's rayon
                count/fill path) on the host cores, rank 0, bounded sample.
 * extra      : other configurations (rc 14, isolated N=1000, triclinic
@@ -529,36 +527,25 @@ def run_b200(args):
     # per-phase CUDA-event times -> roofline of the dominant kernel
     ph = dt.phases(max(5, args.steps // 3))
     peak, peak_kind = peaks()
-    # Algorithmic bytes per launch: the emit (or the one-launch kernel) writes
-    # the 28 B/edge output and reads the sorted SoA (positions, FP32
-    # coordinates, meta) once; the count pass of the three-launch pipeline
-    # reads the sorted FP32 coordinates and writes one count per (atom,
-    # stencil cell).
-    cells = 27  # stencil cells of this grid (n_search = 1 on every axis)
-    bytes_emit = 28 * m_step + 48 * n
-    bytes_count = 16 * n + 4 * cells * n
-    fused = nl.last_single_pipeline() == 0  # one-launch pipeline (sparse grids)
+    # Algorithmic bytes per launch: the emit pass writes the 28 B/edge output
+    # and reads the sorted meta once; the count pass reads the sorted FP32
+    # coordinates.
+    bytes_emit = 28 * m_step + 16 * n
+    bytes_count = 16 * n
+    grouped = nl.last_single_pipeline() == 0  # two-launch group search
     dominant = "emit"
     alg = bytes_emit
     achieved = alg / (ph[dominant] * 1e-3) / 1e9
     # DRAM bytes (read + write) per launch of the same kernel on the same
     # workload, from an ncu capture (not measured by this run).
-    traffic, capture = ncu_traffic(args.rc, "fused" if fused else dominant)
-    count_traffic, _ = ncu_traffic(args.rc, "count")
-    if fused:
-        kernel_name = ("k_pair_fused (count, offsets by look-back over groups, emit and the move "
-                       "of the destinations behind the sources: one launch)")
-        second = {"note": "no separate count pass or offsets scan: both are inside k_pair_fused"}
-    else:
-        # The emit pass has the largest share of the ncu launch list; the
-        # count pass, within a few us of it in live timing and issue-bound,
-        # is reported beside it.
-        kernel_name = "k_pair_tasks<1> (emit pass)"
-        second = {"kernel": "k_pair_tasks<0> (count pass)",
-                  "bound": "instruction issue (61-78 % issue-active in ncu)",
-                  "algorithmic_bytes": bytes_count, "kernel_ms": ph["count"],
-                  "achieved_gbs": bytes_count / (ph["count"] * 1e-3) / 1e9,
-                  "traffic": count_traffic}
+    names = ("k_group_emit", "k_group_count") if grouped else ("k_pair_tasks<1>", "k_pair_tasks<0>")
+    traffic, capture = ncu_traffic(args.rc, "group_emit" if grouped else "emit")
+    count_traffic, _ = ncu_traffic(args.rc, "group_count" if grouped else "count")
+    kernel_name = f"{names[0]} (emit pass)"
+    second = {"kernel": f"{names[1]} (count pass)", "bound": "instruction issue",
+              "algorithmic_bytes": bytes_count, "kernel_ms": ph["count"],
+              "achieved_gbs": bytes_count / (ph["count"] * 1e-3) / 1e9,
+              "traffic": count_traffic}
     step_bytes = 24 * n + 72 + 28 * m_step
 
     # e2e through the reference-facing call (host buffers)
@@ -585,7 +572,7 @@ def run_b200(args):
                      "algorithmic_bytes": alg, "kernel_ms": ph[dominant], "traffic": traffic,
                      "traffic_source": f"ncu capture {capture} (committed traffic table)"
                      if traffic is not None else None,
-                     "phases_ms": ph, "pipeline": "one launch" if fused else "three launches",
+                     "phases_ms": ph, "pipeline": "group search" if grouped else "pair tasks",
                      "count_pass": second,
                      "whole_step": {"algorithmic_bytes": step_bytes,
                                     "ms": ms_max / args.steps,

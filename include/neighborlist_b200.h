@@ -181,14 +181,13 @@ int64_t nlb_kernel_launches(void);
 int64_t nlb_graph_replays(void);
 
 /* Single-system, single-cutoff pipeline choice (no counterpart in the
- * reference).  mode 0 (the default): sparse grids (at most 64 atoms per bin
- * on average, at most 125 stencil cells) count, place and write their edges
- * in one launch, denser ones in three (count, offsets scan, emit); mode 1:
- * always the three-launch pipeline.  Both give identical results.  mode < 0
- * only queries.  Returns the previous mode, or -1 for an unknown mode. */
+ * reference).  mode 0 (the default): the group search, two launches (count
+ * with hit masks, emit); mode 1: the pair-task pipeline, three launches
+ * (count, offsets scan, emit).  Both give identical results.  mode < 0 only
+ * queries.  Returns the previous mode, or -1 for an unknown mode. */
 int32_t nlb_single_pipeline(int32_t mode);
 /* The pipeline the calling thread's last single-cutoff cell-list build took:
- * 0 = one launch, 1 = three launches, -1 = none yet. */
+ * 0 = group search, 1 = pair tasks, -1 = none yet. */
 int32_t nlb_last_single_pipeline(void);
 
 /* Failure-detection hook (no counterpart in the reference, which has no

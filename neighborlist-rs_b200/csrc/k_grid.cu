@@ -318,7 +318,8 @@ __device__ __forceinline__ SlotOut store_slot(const GridParams& g, const double*
                                              float4* __restrict__ p32, int32_t* __restrict__ sbin,
                                              int32_t* __restrict__ irr_list,
                                              uint8_t* __restrict__ irr,
-                                             int32_t* __restrict__ counters) {
+                                             int32_t* __restrict__ counters,
+                                             int32_t* __restrict__ loose) {
   const AtomWrap w = wrap_atom(g, pos[3 * (int64_t)idx], pos[3 * (int64_t)idx + 1],
                                pos[3 * (int64_t)idx + 2]);
   px[p] = w.wx;
@@ -346,6 +347,13 @@ __device__ __forceinline__ SlotOut store_slot(const GridParams& g, const double*
     so.q = make_float4(__double2float_rn(dsub(w.wx, c[0])), __double2float_rn(dsub(w.wy, c[1])),
                        __double2float_rn(dsub(w.wz, c[2])), __int_as_float(idx));
     p32[p] = so.q;
+    // Half the bin's diagonal bounds an atom's distance from its bin's centre;
+    // 1e-6 of it is far above rounding and far below the guard band's width.
+    if (loose) {
+      const double far = dmul(g.radius, 1.000001);
+      if (!(norm2(dsub(w.wx, c[0]), dsub(w.wy, c[1]), dsub(w.wz, c[2])) <= dmul(far, far)))
+        atomicExch(loose, 1);
+    }
     so.lin = w.bin[0] + g.nb[0] * (w.bin[1] + g.nb[1] * w.bin[2]);
     sbin[p] = so.lin;
     // Home stencil centre, recomputed from the wrapped position exactly as
@@ -422,7 +430,8 @@ __device__ void sort_bin(const GridParams& g, const double* __restrict__ pos, in
                          int32_t* __restrict__ sbin, GroupRec* __restrict__ groups,
                          int32_t* __restrict__ irr_list, uint8_t* __restrict__ irr,
                          int32_t* __restrict__ counters, float4* __restrict__ cbox,
-                         const int32_t* __restrict__ group_start, uint64_t* sk, int32_t* sv) {
+                         const int32_t* __restrict__ group_start, int32_t* __restrict__ loose,
+                         uint64_t* sk, int32_t* sv) {
   const int64_t s = bin_start[r];
   const int64_t e = bin_start[r + 1];
   const int64_t cnt = e - s;
@@ -494,7 +503,7 @@ __device__ void sort_bin(const GridParams& g, const double* __restrict__ pos, in
     so.lin = 0;
     if (p < e)
       so = store_slot(g, pos, p, final_idx[p], px, py, pz, meta, p32, sbin, irr_list, irr,
-                      counters);
+                      counters, loose);
     if (p == s) lin0 = so.lin;
     if (p32 && cbox) warp_box(so.q, p < e, cbox + 2 * p0);
   }
@@ -525,7 +534,7 @@ __global__ void __launch_bounds__(kSortThreads)
             GroupRec* __restrict__ groups, int32_t* __restrict__ irr_list,
             uint8_t* __restrict__ irr, int32_t* __restrict__ counters,
             float4* __restrict__ cbox, const int32_t* __restrict__ group_start,
-            int32_t atom_blocks, int32_t bin_span) {
+            int32_t* __restrict__ loose, int32_t atom_blocks, int32_t bin_span) {
   __shared__ uint64_t sk[kSortCap];
   __shared__ int32_t sv[kSortCap];
   pdl_wait();
@@ -541,7 +550,7 @@ __global__ void __launch_bounds__(kSortThreads)
       for (int64_t r = r1; r < r1 + kSortThreads && r < end; ++r) {
         if (bin_start[r + 1] - bin_start[r] <= kRankSortMax) continue;
         sort_bin(g, pos, r, bin_start, skey, sidx, skey2, sidx2, px, py, pz, meta, p32, sbin,
-                 groups, irr_list, irr, counters, cbox, group_start, sk, sv);
+                 groups, irr_list, irr, counters, cbox, group_start, loose, sk, sv);
         __syncthreads();
       }
     }
@@ -558,7 +567,7 @@ __global__ void __launch_bounds__(kSortThreads)
   const int64_t s = bin_start[r], e = bin_start[r + 1];
   if (e - s > kRankSortMax) return;
   int32_t below = 0;
-#pragma unroll(SPLIT > 1 ? 1 : 4)
+#pragma unroll 4
   for (int64_t q = s + part; q < e; q += SPLIT)
     below += pair_less(__ldg(&skey[q]), __ldg(&sidx[q]), k, i) ? 1 : 0;
   if (SPLIT > 1) {
@@ -568,7 +577,7 @@ __global__ void __launch_bounds__(kSortThreads)
     if (part != 0) return;
   }
   const SlotOut so = store_slot(g, pos, s + below, i, px, py, pz, meta, p32, sbin, irr_list, irr,
-                                counters);
+                                counters, loose);
   if (p32 && below == 0) store_groups(g, r, s, e, so.lin, groups, counters, group_start);
 }
 
@@ -675,7 +684,7 @@ void launch_grid_build(const GridParams& g, const double* pos, int64_t n, const 
   launch_pdl(whole ? k_place<1> : k_place<8>, dim3((unsigned)blocks), dim3(kSortThreads), 0, s, g,
              pos, n, (const int32_t*)b.rank, (const int64_t*)b.bin_start, b.skey, b.sidx, b.skey2,
              b.sidx2, b.px, b.py, b.pz, b.meta, b.p32, b.sbin, b.groups, b.irr_list, b.irr,
-             b.counters, b.cbox, grouped ? (const int32_t*)b.group_start : nullptr,
+             b.counters, b.cbox, grouped ? (const int32_t*)b.group_start : nullptr, b.loose,
              atom_blocks, (int32_t)span);
   note_launches(3);
   if (b.p32 && b.cbox) {

@@ -907,13 +907,13 @@ Status run_single(const double* pos, int64_t n, const double* cell9, const uint8
   if (!st.ok()) return st;
   if (fast_eligible(sp)) {
     int64_t m = 0;
-    // (host copies: no [src | dst] layout needed; the copies follow the
-    // search on the stream, so the call goes on as soon as M is known)
-    st = run_fast(*c, sp, d_pos, &m, false, true);
+    // (the copies follow the search on the stream, so the call goes on as
+    // soon as M is known)
+    st = run_fast(*c, sp, d_pos, &m, true);
     if (!st.ok()) return st;
     DevLists L;
     L.src.assign(1, sp.out_src);
-    L.dst.assign(1, sp.out_dst);
+    L.dst.assign(1, sp.out_src + m);
     L.sh.assign(1, sp.out_sh);
     st = download_results(*c, std::vector<int64_t>(1, m), L, sp.order, outs);
     if (!st.ok()) nlb_result_free(&outs[0]);

@@ -1,21 +1,16 @@
 // nlb_fast.cpp -- single-system, single-cutoff cell-list builds without a
 // host round trip in the middle, replayed as a CUDA graph.
 //
-// The pipeline (bin histogram memset, atom prep, bin scan, scatter, per-bin
-// sort + gather, pair-task count, offset scan, pair-task emit) is issued
-// back to back on the caller's stream.  The emit pass reads the edge total
-// from device memory and writes into a capacity-bounded arena (the previous
-// total x 1.25, or a density estimate); the host synchronises once at the
-// end, and only if the arena was too small does it grow it and run the emit
-// pass again (the counts and offsets are still in place).
+// The pipeline (bin histogram memset, atom prep, bin scan, scatter, placement,
+// group count, group emit) is issued back to back on the caller's stream.
+// The emit pass reads the edge total from device memory and writes into a
+// capacity-bounded arena (the previous total x 1.25, or a density estimate);
+// the host learns the total from the count pass, and only if the arena or
+// the count's records were too small does it grow them and run the missing
+// passes again.
 //
-// On sparse grids (at most 64 atoms per bin on average, at most 125 stencil
-// cells) the count, offsets scan and emit are one launch instead
-// (k_fused.cu): the build stores the groups in canonical order, one CTA per
-// group counts, finds its output offset by a look-back over the groups
-// before it and writes its block; the edge total again comes from device
-// memory, and an arena that was too small makes the host grow it and run the
-// fused launch again.
+// Mode 1 (nlb_single_pipeline) takes the pair-task kernels of the
+// multi-cutoff path instead: count per (atom, stencil cell), scan, emit.
 //
 // The first call with a given set of launch parameters runs the work
 // directly; a repeated call with identical parameters (same positions
@@ -46,8 +41,7 @@ struct FastKey {
   int64_t mask_cap;
   int32_t need_rank;
   int32_t prof;
-  int32_t fused;
-  int32_t contiguous;
+  int32_t split;  // segments per group (0: pair tasks)
 };
 
 struct FastState {
@@ -57,6 +51,7 @@ struct FastState {
   int launches = 0;  // kernels per replay
   int64_t last_m = 0;
   int64_t last_mask_words = 0;
+  int64_t last_records = 0;  // records the last group search asked for
 };
 
 thread_local FastState tl_states[16];
@@ -65,6 +60,11 @@ FastState& state_for(Ctx& c) { return tl_states[c.device & 15]; }
 
 int64_t stencil_cells_of(const GridParams& g) {
   return (int64_t)(2 * g.ns[0] + 1) * (2 * g.ns[1] + 1) * (2 * g.ns[2] + 1);
+}
+
+// 64-bit words of the group search's zeroed state.
+int64_t group_state_words(int64_t max_groups) {
+  return 16 + 16 * kGroupRegions + group_blocks(max_groups) + (max_groups + 1) / 2;
 }
 
 // Expected edges for sizing the first arena: half the pairs within rc at the
@@ -85,11 +85,11 @@ std::atomic<int32_t> g_pipeline_mode{0};
 }  // namespace
 
 namespace {
-thread_local int32_t tl_last_fused = -1;  // pipeline of this thread's last fast-path build
+thread_local int32_t tl_last_pipeline = -1;  // pipeline of this thread's last fast-path build
 }  // namespace
 
 int32_t single_pipeline_mode() { return g_pipeline_mode.load(); }
-int32_t last_single_pipeline() { return tl_last_fused; }
+int32_t last_single_pipeline() { return tl_last_pipeline; }
 int32_t set_single_pipeline_mode(int32_t mode) { return g_pipeline_mode.exchange(mode); }
 
 void release_fast_states() {
@@ -113,41 +113,74 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   b.rank_of_bin = slot<int32_t>(c, kSlotRankTab, nb);
   sp.rank_cached = b.rank_of_bin == tab_before && tab_cap > 0 && c.rank_nb[0] == sp.grid.nb[0] &&
                    c.rank_nb[1] == sp.grid.nb[1] && c.rank_nb[2] == sp.grid.nb[2];
-  // Zeroed block: bin histogram, scatter cursors, 2 task counters, 64-bit
-  // mask cursor (8-byte aligned: 2 nb + 2 is even), build completion count,
-  // emit task counter, then the offsets scan's state (8-byte aligned at
-  // 2 nb + 6), so a single
-  // memset at the start clears everything and the kernels follow each other
-  // directly.
-  // (Fused launch: its ticket, error and look-back words and its total take
-  // the scan state's place.)
+  // Zeroed block, so that a single memset at the start clears everything and
+  // the kernels follow each other directly: bin histogram, scatter cursors, 2
+  // task counters, 64-bit mask cursor (8-byte aligned: 2 nb + 2 is even),
+  // build completion count, emit task counter, loose flag and padding, then
+  // (8-byte aligned) the offsets scan's state, or the group search's ticket,
+  // error word, total, completion count, record cursor, block sums and segment
+  // counts and the bin scan's state.
   const int64_t max_groups = n / 32 + std::min<int64_t>(n, nb) + 1;
-  sp.fused_words = 2 + max_groups + 2;  // + total, completion count
-  sp.zeroed_words = 2 * (size_t)nb + 6 +
-                    2 * (size_t)(sp.fused ? sp.fused_words : scan_tmp_elems(row)) +
-                    2 * (size_t)(sp.fused && nb > kPrepBinScanMax ? bin_scan_words(nb) : 0);
+  const bool bin_scan = sp.grouped && nb > kPrepBinScanMax;
+  const int64_t group_words = group_state_words(max_groups);
+  const int64_t words64 = sp.grouped ? group_words + (bin_scan ? bin_scan_words(nb) : 0)
+                                     : scan_tmp_elems(row);
+  sp.zeroed_words = 2 * (size_t)nb + 8 + 2 * (size_t)words64;
   int32_t* zeroed = slot<int32_t>(c, kSlotBinCount, sp.zeroed_words);
-  sp.scan_state = zeroed ? reinterpret_cast<int64_t*>(zeroed + 2 * nb + 6) : nullptr;
-  sp.fused_state = reinterpret_cast<uint64_t*>(sp.scan_state);
-  sp.fused_total = sp.fused && zeroed ? sp.scan_state + 2 + max_groups : nullptr;
-  b.bin_scan = sp.fused && nb > kPrepBinScanMax && zeroed
-                   ? reinterpret_cast<uint64_t*>(sp.scan_state + sp.fused_words)
-                   : nullptr;
-  b.group_start = sp.fused ? slot<int32_t>(c, kSlotGroupStart, nb) : nullptr;
-  b.fill = slot<int32_t>(c, kSlotFill, n);
+  if (!zeroed) return fail(NLB_ERR_NOMEM, "device allocation failed");
   b.bin_count = zeroed;
-  b.bin_fill = zeroed ? zeroed + nb : nullptr;
-  b.counters = zeroed ? zeroed + 2 * nb : nullptr;
-  b.mask_top = zeroed ? reinterpret_cast<unsigned long long*>(zeroed + 2 * nb + 2) : nullptr;
-  b.build_done = zeroed ? zeroed + 2 * nb + 4 : nullptr;
-  b.emit_queue = zeroed ? reinterpret_cast<uint32_t*>(zeroed + 2 * nb + 5) : nullptr;
-  const int64_t max_tasks = (n / 32 + std::min<int64_t>(n, nb) + 1) * cells;
-  // (The fused launch needs no task headers, masks, counts or offsets.)
-  b.task_hdr = slot<int4>(c, kSlotTaskHdr, sp.fused ? 1 : max_tasks);
-  b.masks = slot<uint32_t>(c, kSlotMasks, sp.fused ? 1 : mask_cap);
-  const bool chunk_boxes = nb > 0 && (double)n / (double)nb >= kChunkPruneMinPerBin;
+  b.bin_fill = zeroed + nb;
+  b.counters = zeroed + 2 * nb;
+  b.mask_top = reinterpret_cast<unsigned long long*>(zeroed + 2 * nb + 2);
+  b.build_done = zeroed + 2 * nb + 4;
+  b.emit_queue = reinterpret_cast<uint32_t*>(zeroed + 2 * nb + 5);
+  b.loose = zeroed + 2 * nb + 6;
+  int64_t* state = reinterpret_cast<int64_t*>(zeroed + 2 * nb + 8);
+  sp.scan_state = state;
+  b.bin_scan = bin_scan ? reinterpret_cast<uint64_t*>(state + group_words) : nullptr;
+  b.group_start = sp.grouped ? slot<int32_t>(c, kSlotGroupStart, nb) : nullptr;
+  b.fill = slot<int32_t>(c, kSlotFill, n);
+  const int64_t max_tasks = max_groups * cells;
+  // (The group search needs no task headers, masks, counts or offsets.)
+  b.task_hdr = slot<int4>(c, kSlotTaskHdr, sp.grouped ? 1 : max_tasks);
+  if (sp.grouped) {
+    GroupSearch& o = sp.search;
+    const int32_t split = o.split;
+    std::memset(&o, 0, sizeof(o));
+    o.split = split;
+    o.state = reinterpret_cast<uint64_t*>(state);
+    o.total = state + 2;
+    o.done = reinterpret_cast<int32_t*>(state + 3);
+    o.records = state + 4;
+    o.chunk_top = reinterpret_cast<unsigned long long*>(state + 16);
+    o.block_sum = reinterpret_cast<uint64_t*>(state + 16 + 16 * kGroupRegions);
+    o.group_done =
+        reinterpret_cast<int32_t*>(state + 16 + 16 * kGroupRegions + group_blocks(max_groups));
+    o.chunk_cap = mask_cap / 32;
+    o.masks = slot<uint32_t>(c, kSlotMasks, mask_cap);
+    o.cand = slot<uint32_t>(c, kSlotCand, mask_cap);
+    o.cshift = slot<uint32_t>(c, kSlotCshift, mask_cap);
+    o.block_base = slot<int64_t>(c, kSlotGroupBase, group_blocks(max_groups));
+    o.group_total = slot<int64_t>(c, kSlotGroupTotal, max_groups);
+    o.atom_base = slot<int64_t>(c, kSlotAtomBase, 32 * (size_t)max_groups);
+    o.seg_cnt = slot<uint32_t>(c, kSlotSegCnt, (size_t)max_groups * split * 32);
+    o.seg_rec = slot<longlong2>(c, kSlotSegRec, (size_t)max_groups * split);
+    o.max_groups = max_groups;
+    o.withhold = -1;
+    o.spin_limit = kGroupSpinLimit;
+    o.report = c.prof ? nullptr : c.d_report;
+    if (!o.masks || !o.cand || !o.cshift || !o.block_base || !o.group_total || !o.atom_base || !o.seg_cnt || !o.seg_rec ||
+        !b.group_start)
+      return fail(NLB_ERR_NOMEM, "device allocation failed");
+    b.masks = nullptr;
+    b.mask_cap = 0;
+  } else {
+    b.masks = slot<uint32_t>(c, kSlotMasks, mask_cap);
+    b.mask_cap = mask_cap;
+    if (!b.masks) return fail(NLB_ERR_NOMEM, "device allocation failed");
+  }
+  const bool chunk_boxes = !sp.grouped && nb > 0 && (double)n / (double)nb >= kChunkPruneMinPerBin;
   b.cbox = chunk_boxes ? slot<float4>(c, kSlotCbox, 2 * (size_t)n) : nullptr;
-  b.mask_cap = sp.fused ? 0 : mask_cap;
   b.bin_start = slot<int64_t>(c, kSlotBinStart, nb + 1);
   b.key = slot<uint64_t>(c, kSlotKey, n);
   b.rank = slot<int32_t>(c, kSlotRank, n);
@@ -164,55 +197,52 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   b.groups = slot<GroupRec>(c, kSlotGroups, n / 32 + std::min<int64_t>(n, nb) + 1);
   b.irr_list = slot<int32_t>(c, kSlotIrrList, n);
   b.irr = slot<uint8_t>(c, kSlotIrr, n);
-  b.scan_tmp = slot<int64_t>(c, kSlotScanTmp, scan_tmp_elems(std::max<int64_t>(row, nb)));
-  sp.counts = slot<uint32_t>(c, kSlotCounts, sp.fused ? 1 : row);
-  sp.offs = slot<int64_t>(c, kSlotOffs, sp.fused ? 1 : row + 1);
+  b.scan_tmp = slot<int64_t>(c, kSlotScanTmp, scan_tmp_elems(sp.grouped ? nb : std::max<int64_t>(row, nb)));
+  sp.counts = slot<uint32_t>(c, kSlotCounts, sp.grouped ? 1 : row);
+  sp.offs = slot<int64_t>(c, kSlotOffs, sp.grouped ? 1 : row + 1);
   sp.out_src = slot<int64_t>(c, kSlotOutEi, 2 * (size_t)capacity);
   sp.out_sh = slot<int32_t>(c, kSlotOutSh, 3 * (size_t)capacity);
-  int64_t* dst_arena = sp.fused ? slot<int64_t>(c, kSlotOutDst, (size_t)capacity) : nullptr;
-  if (sp.fused && (!dst_arena || !b.group_start))
-    return fail(NLB_ERR_NOMEM, "device allocation failed");
-  if (!b.rank_of_bin || !zeroed || !b.bin_start || !b.key || !b.rank || !b.skey || !b.sidx ||
-      !b.skey2 || !b.sidx2 || !b.px || !b.py || !b.pz || !b.meta || !b.p32 || !b.sbin ||
-      !b.groups || !b.irr_list || !b.irr || !b.scan_tmp || !sp.counts || !sp.offs ||
-      !sp.out_src || !sp.out_sh || !b.task_hdr || !b.masks || (chunk_boxes && !b.cbox) ||
-      !b.fill)
+  if (!b.rank_of_bin || !b.bin_start || !b.key || !b.rank || !b.skey || !b.sidx || !b.skey2 ||
+      !b.sidx2 || !b.px || !b.py || !b.pz || !b.meta || !b.p32 || !b.sbin || !b.groups ||
+      !b.irr_list || !b.irr || !b.scan_tmp || !sp.counts || !sp.offs || !sp.out_src ||
+      !sp.out_sh || !b.task_hdr || (chunk_boxes && !b.cbox) || !b.fill)
     return fail(NLB_ERR_NOMEM, "device allocation failed");
   return Status{NLB_OK};
 }
 
-FusedOut fused_targets(Ctx& c, const SystemPlan& sp, int64_t capacity) {
-  FusedOut o;
-  std::memset(&o, 0, sizeof(o));
-  o.src = sp.out_src;
-  o.dst = static_cast<int64_t*>(c.bufs[kSlotOutDst].p);
-  o.sh = sp.out_sh;
-  o.capacity = capacity;
-  o.state = sp.fused_state;
-  o.total = sp.fused_total;
-  o.done = reinterpret_cast<unsigned long long*>(sp.fused_total + 1);
-  o.report = c.prof ? nullptr : c.d_report;
-  o.spin_limit = kFusedSpinLimit;
-  o.withhold = -1;
-  {
-    const double per_bin = (double)sp.n / (double)std::max<int64_t>(sp.grid.total_bins, 1);
-    const int64_t chunks = (int64_t)std::ceil(1.5 * per_bin / 32.0);
-    const int64_t want = stencil_cells_of(sp.grid) * std::max<int64_t>(chunks, 1) * 32;
-    o.mask_words = (int32_t)std::min<int64_t>(std::max<int64_t>(want, kFusedMaskMin), kFusedMaskMax);
-  }
-  int32_t tile = 0, spins = 0;
-  if (take_scan_stall(&tile, &spins)) {  // failure-detection hook
-    o.withhold = tile;
-    o.spin_limit = spins;
-  }
-  return o;
+// Segments per group.  Grids with large bins (every group tests hundreds of
+// atoms in most cells, none in others): one per stencil cell.  Others: as many
+// as give the chip one round of warps (28 per SM): fewer leave warps idle
+// (10,008 atoms at rc 6: 90 us with two per group, 82 with six to nine), more
+// pay for describing cells twice (88 us with twelve).
+constexpr double kSplitDense = 64.0;
+constexpr int64_t kSplitTarget = 5000;
+int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
+  const int64_t groups = n / 32 + std::min<int64_t>(n, nb) + 1;  // (at most)
+  const int64_t want = (double)n > kSplitDense * (double)nb
+                           ? std::min<int64_t>(cells, ((int64_t)1 << 30) / groups)
+                           : std::min<int64_t>(kSplitTarget / groups, cells);
+  return (int32_t)std::max<int64_t>(want, 1);
 }
 
-// The fused launch (and the move of the destinations behind the sources).
-void issue_fused(Ctx& c, SystemPlan& sp, int64_t capacity, bool contiguous) {
-  FusedOut o = fused_targets(c, sp, capacity);
-  o.move = contiguous ? 1 : 0;
-  launch_pair_fused(sp.grid, sp.gb, (int32_t)stencil_cells_of(sp.grid), sp.band, o, c.stream);
+// The group search's two launches.
+void issue_search(Ctx& c, SystemPlan& sp, int64_t capacity, bool count) {
+  const GroupBand band = group_band(sp.band);
+  const int32_t cells = (int32_t)stencil_cells_of(sp.grid);
+  if (count) {
+    GroupSearch o = sp.search;
+    int32_t tile = 0, spins = 0;
+    if (take_scan_stall(&tile, &spins)) {  // failure-detection hook
+      o.withhold = tile;
+      o.spin_limit = spins;
+    }
+    launch_group_count(sp.grid, sp.gb, cells, band, o, c.stream);
+    c.mark(2);
+    c.mark(3);
+    c.mark(4);
+  }
+  launch_group_emit(sp.grid, sp.gb, cells, band, sp.search, sp.out_src, sp.out_sh, capacity,
+                    c.stream);
 }
 
 EmitTargets fast_targets(const SystemPlan& sp, int64_t capacity, int64_t* report = nullptr) {
@@ -231,21 +261,16 @@ EmitTargets fast_targets(const SystemPlan& sp, int64_t capacity, int64_t* report
 }
 
 // Issues the whole pipeline on c.stream (no host synchronisation).
-void issue_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t capacity,
-                bool contiguous) {
+void issue_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t capacity) {
   cudaStream_t s = c.stream;
   const int64_t n = sp.n;
   c.mark(0);
   cudaMemsetAsync(sp.gb.bin_count, 0, sizeof(int32_t) * sp.zeroed_words, s);
   launch_grid_build(sp.grid, d_pos, n, sp.gb, s, !sp.rank_cached);
   c.mark(1);
-  if (sp.fused) {
-    // (Phases: counting and offsets are part of the one launch, timed with
-    // the emit.)
-    c.mark(2);
-    c.mark(3);
-    c.mark(4);
-    issue_fused(c, sp, capacity, contiguous);
+  if (sp.grouped) {
+    // (Phases: the offsets are part of the count pass.)
+    issue_search(c, sp, capacity, true);
     c.mark(5);
     return;
   }
@@ -283,19 +308,20 @@ Status wait_report(Ctx& c) {
 // Runs the fast pipeline for a planned single-cutoff cell-list system and
 // leaves M edges in sp.out_src ([src | dst]) / sp.out_sh.
 //
-// M reaches the host through host-mapped memory as soon as it is known: the
-// one-launch search reports it when its last group is done, the three-launch
-// pipeline when its emit pass starts.  On a caller's stream the call then
-// returns at once: the remaining work (the emit, or the move of the
-// destinations) is queued on that stream ahead of anything the caller queues
-// there.  On the library's own stream it also waits for that work.
-Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, bool contiguous,
+// M reaches the host through host-mapped memory as soon as it is known: when
+// the count pass ends (mode 1: when its emit pass starts).  On a caller's
+// stream the call then returns at once: the emit is queued on that stream
+// ahead of anything the caller queues there.  On the library's own stream it
+// also waits for that work.
+Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
                 bool stream_ordered) {
   FastState& fs = state_for(c);
-  const int64_t n_cells = stencil_cells_of(sp.grid);
-  sp.fused = single_pipeline_mode() == 0 && n_cells <= kFusedMaxCells &&
-             sp.grid.total_bins > 0 && (double)sp.n / (double)sp.grid.total_bins <= kFusedMaxPerBin;
-  tl_last_fused = sp.fused ? 0 : 1;
+  const int64_t cells = stencil_cells_of(sp.grid);
+  // (the group search counts a row of candidates -- at most 32 images of all
+  // atoms -- in 32 bits)
+  sp.grouped = single_pipeline_mode() == 0 && sp.n < ((int64_t)1 << 26);
+  sp.search.split = sp.grouped ? group_split(sp.n, sp.grid.total_bins, cells) : 0;
+  tl_last_pipeline = sp.grouped ? 0 : 1;
   const double rc = std::sqrt(sp.rc_sq[0]);
   int64_t capacity = std::max<int64_t>(
       {4096, (int64_t)(1.25 * (double)fs.last_m), (int64_t)(1.5 * (double)estimate_edges(sp, rc))});
@@ -303,9 +329,22 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
   const size_t have = c.bufs[kSlotOutSh].cap / (3 * sizeof(int32_t));
   if ((int64_t)have > capacity && c.bufs[kSlotOutEi].cap / (2 * sizeof(int64_t)) >= have)
     capacity = (int64_t)have;
-  // Hit-mask arena: the last run's need x 1.25, at least 64 words per atom.
+  // Hit-mask arena: the last run's need x 1.25, at least 64 words per atom;
+  // the group search's records (32 words each): one per 32 candidates of a
+  // segment, with the groups and candidates of a uniform density.
   int64_t mask_cap = std::max<int64_t>(64 * sp.n + 4096, fs.last_mask_words + fs.last_mask_words / 4);
-  const int64_t mask_have = (int64_t)(c.bufs[kSlotMasks].cap / sizeof(uint32_t));
+  if (sp.grouped) {
+    const double per_bin = (double)sp.n / (double)sp.grid.total_bins;
+    const double filled = (double)sp.grid.total_bins * (1.0 - std::exp(-per_bin));
+    const double groups = std::max(filled, (double)sp.n / 32.0 + 0.5 * filled) + 1.0;
+    const double records = groups * ((double)cells * per_bin / 32.0 + sp.search.split);
+    mask_cap = 32 * std::max<int64_t>((int64_t)std::min(1.25 * records, 1e12) + 64 * kGroupRegions,
+                                      fs.last_records + fs.last_records / 8);
+  }
+  int64_t mask_have = (int64_t)(c.bufs[kSlotMasks].cap / sizeof(uint32_t));
+  if (sp.grouped)
+    mask_have = std::min({mask_have, (int64_t)(c.bufs[kSlotCand].cap / sizeof(uint32_t)),
+                          (int64_t)(c.bufs[kSlotCshift].cap / sizeof(uint32_t))});
   if (mask_have > mask_cap) mask_cap = mask_have;
   Status st = prepare_fast(c, sp, capacity, mask_cap);
   if (!st.ok()) return st;
@@ -322,8 +361,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
   key.mask_cap = mask_cap;
   key.need_rank = sp.rank_cached ? 0 : 1;
   key.prof = c.prof ? 1 : 0;
-  key.fused = sp.fused ? 1 : 0;
-  key.contiguous = contiguous ? 1 : 0;
+  key.split = sp.search.split;
 
   const bool report = !c.prof;
   if (report) c.h_report[0] = 0;
@@ -352,7 +390,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
     cudaGraph_t graph = nullptr;
     const int64_t l0 = nlb_kernel_launches();
     if (cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-      issue_fast(c, sp, d_pos, capacity, contiguous);
+      issue_fast(c, sp, d_pos, capacity);
       if (cudaStreamEndCapture(c.stream, &graph) == cudaSuccess && graph) {
         if (cudaGraphInstantiate(&fs.exec, graph, 0) != cudaSuccess) fs.exec = nullptr;
         cudaGraphDestroy(graph);
@@ -371,7 +409,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
       cudaGraphExecDestroy(fs.exec);
       fs.exec = nullptr;
     }
-    issue_fast(c, sp, d_pos, capacity, contiguous);
+    issue_fast(c, sp, d_pos, capacity);
   }
   fs.key = key;
   fs.have_key = true;
@@ -383,7 +421,8 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
     const volatile int64_t* r = c.h_report;
     const int64_t m = r[1];
     if (r[2] != 0) return fail(NLB_ERR_CUDA, "prefix scan gave up waiting for a tile");
-    if (m <= capacity) {
+    if (sp.grouped) fs.last_records = r[3];
+    if (m <= capacity && (!sp.grouped || r[3] <= sp.search.chunk_cap)) {
       if (c.stream == c.own_stream) {
         if (!stream_ordered) {
           const cudaError_t e = cudaStreamSynchronize(c.stream);
@@ -394,33 +433,31 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
         if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
         c.early_stream = c.stream;
       }
-      sp.out_dst = sp.fused && !contiguous ? static_cast<int64_t*>(c.bufs[kSlotOutDst].p)
-                                           : sp.out_src + m;
       fs.last_m = m;
-      fs.last_mask_words = sp.fused ? 0 : r[3];
+      if (!sp.grouped) fs.last_mask_words = r[3];
       *m_out = m;
       return Status{NLB_OK};
     }
-    // (M above the capacity: the synchronous path below grows the arrays.)
+    // (Too little room: the synchronous path below grows the arrays.)
   }
 
-  // Without the report (phase profiling, or M above the capacity): one
+  // Without the report (phase profiling, or too little room): one
   // synchronisation reads the total edges and the scan's wait-error word.
-  cudaError_t e = cudaMemcpyAsync(c.h_small, sp.fused ? sp.fused_total : sp.offs + sp.row,
+  cudaError_t e = cudaMemcpyAsync(c.h_small, sp.grouped ? sp.search.total : sp.offs + sp.row,
                                   sizeof(int64_t), cudaMemcpyDeviceToHost, c.stream);
-  if (e == cudaSuccess)  // the scan's (or the fused look-back's) wait-error word
+  if (e == cudaSuccess)  // the scan's (or the group search's) wait-error word
     e = cudaMemcpyAsync(c.h_small + 1, sp.scan_state + 1, sizeof(int64_t),
                         cudaMemcpyDeviceToHost, c.stream);
   c.h_small[2] = 0;
-  if (e == cudaSuccess && !sp.fused)
-    e = cudaMemcpyAsync(c.h_small + 2, sp.gb.mask_top, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                        c.stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(c.h_small + 2, sp.grouped ? (const void*)sp.search.records : sp.gb.mask_top,
+                        sizeof(int64_t), cudaMemcpyDeviceToHost, c.stream);
   // Grids too large for k_prep's own bin scan use a separate scan (state in
   // gb.scan_tmp): its error word too.
   c.h_small[3] = 0;
   if (e == cudaSuccess && sp.grid.total_bins > kPrepBinScanMax)
     e = cudaMemcpyAsync(c.h_small + 3,
-                        sp.fused ? reinterpret_cast<int64_t*>(sp.gb.bin_scan) + 1
+                        sp.grouped ? reinterpret_cast<int64_t*>(sp.gb.bin_scan) + 1
                                  : sp.gb.scan_tmp + 1,
                         sizeof(int64_t), cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
@@ -433,35 +470,43 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out, boo
     c.prof_pending_emit = true;
     c.harvest();
   }
-  if (m > capacity) {
-    // Arena too small: grow it (outside any capture) and emit again.
-    const int64_t cap2 = m + m / 8 + 1024;
+  const int64_t records = c.h_small[2];
+  const bool recount = sp.grouped && records > sp.search.chunk_cap;
+  if (m > capacity || recount) {
+    // Too little room: grow it (outside any capture) and run what is missing
+    // again.  The records: the count pass once more, its state cleared first.
+    const int64_t cap2 = m > capacity ? m + m / 8 + 1024 : capacity;
     sp.out_src = slot<int64_t>(c, kSlotOutEi, 2 * (size_t)cap2);
     sp.out_sh = slot<int32_t>(c, kSlotOutSh, 3 * (size_t)cap2);
     if (!sp.out_src || !sp.out_sh) return fail(NLB_ERR_NOMEM, "device allocation for the edge lists failed");
-    if (sp.fused) {
-      // The fused launch counts again: clear its ticket, look-back words and
-      // total first.
-      if (!slot<int64_t>(c, kSlotOutDst, (size_t)cap2))
-        return fail(NLB_ERR_NOMEM, "device allocation for the edge lists failed");
-      cudaMemsetAsync(sp.fused_state, 0, sizeof(uint64_t) * (size_t)sp.fused_words, c.stream);
-      issue_fused(c, sp, cap2, contiguous);
-      e = cudaMemcpyAsync(c.h_small + 1, sp.scan_state + 1, sizeof(int64_t),
-                          cudaMemcpyDeviceToHost, c.stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
-      if (e != cudaSuccess) return cuda_fail(e, "fused pass");
-      if (c.h_small[1] != 0) return fail(NLB_ERR_CUDA, "prefix scan gave up waiting for a tile");
-    } else {
-      launch_pair_emit(sp.grid, sp.gb, sp.n, sp.band, sp.offs, fast_targets(sp, cap2), c.stream);
-      e = cudaStreamSynchronize(c.stream);
-      if (e != cudaSuccess) return cuda_fail(e, "emit pass");
+    if (recount) {
+      GroupSearch& o = sp.search;
+      o.masks = slot<uint32_t>(c, kSlotMasks, 32 * (size_t)records);
+      o.cand = slot<uint32_t>(c, kSlotCand, 32 * (size_t)records);
+      o.cshift = slot<uint32_t>(c, kSlotCshift, 32 * (size_t)records);
+      if (!o.masks || !o.cand || !o.cshift) return fail(NLB_ERR_NOMEM, "device allocation failed");
+      o.chunk_cap = records;
+      cudaMemsetAsync(o.state, 0, sizeof(uint64_t) * (size_t)group_state_words(o.max_groups), c.stream);
     }
+    if (sp.grouped)
+      issue_search(c, sp, cap2, recount);
+    else
+      launch_pair_emit(sp.grid, sp.gb, sp.n, sp.band, sp.offs, fast_targets(sp, cap2), c.stream);
+    c.h_small[1] = 0;
+    e = cudaSuccess;
+    if (recount)
+      e = cudaMemcpyAsync(c.h_small + 1, sp.search.state + 1, sizeof(int64_t),
+                          cudaMemcpyDeviceToHost, c.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
+    if (e != cudaSuccess) return cuda_fail(e, "emit pass");
+    if (c.h_small[1] != 0) return fail(NLB_ERR_CUDA, "prefix scan gave up waiting for a tile");
     fs.have_key = false;  // workspace pointers changed
   }
-  sp.out_dst = sp.fused && !contiguous ? static_cast<int64_t*>(c.bufs[kSlotOutDst].p)
-                                       : sp.out_src + m;
   fs.last_m = m;
-  fs.last_mask_words = c.h_small[2];
+  if (sp.grouped)
+    fs.last_records = records;
+  else
+    fs.last_mask_words = records;
   *m_out = m;
   return Status{NLB_OK};
 }

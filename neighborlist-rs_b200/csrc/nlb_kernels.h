@@ -19,8 +19,8 @@ int64_t scan_tmp_elems(int64_t n);
 // (then record the error word and finish).  One-shot.
 void arm_scan_stall(int32_t tile, int32_t spin_limit);
 bool scan_stall_armed();
-// Takes the armed hook for a launch that is not a scan (the fused search's
-// look-back over groups); false when none is armed.
+// Takes the armed hook for a launch that is not a scan (the group
+// search's scan of its blocks); false when none is armed.
 bool take_scan_stall(int32_t* tile, int32_t* spin_limit);
 void exclusive_scan_u32(const uint32_t* in, int64_t n, int64_t* out, int64_t* tmp,
                         cudaStream_t s);
@@ -99,6 +99,10 @@ struct GridBuffers {
   // from the histogram (k_scatter then needs no atomics); nullptr: k_scatter
   // takes places from bin_fill.
   int32_t* fill;
+  // Optional (zeroed by the caller before the build): set when an atom lies
+  // outside its stored bin by more than rounding (positions so far from the
+  // cell that wrapping them loses bits).
+  int32_t* loose;
   // Optional: state words of the bin scan of grids above kPrepBinScanMax bins
   // (bin_scan_words(total_bins), zeroed by the caller before the build; used
   // when group_start is set); [1] is its error word.
@@ -186,47 +190,56 @@ struct PairBands {
 };
 // Stencils above this many cells use the per-atom FP64 kernels.
 constexpr int64_t kPairMaxCells = 1024;
-// ---- k_fused.cu : count + offsets + emit of the single-cutoff list in one
-// launch (one CTA per 32-atom group, decoupled look-back over the groups).
-// Needs the groups in canonical order (GridBuffers::group_start set for the
-// build) and at most kFusedMaxCells stencil cells.
-constexpr int32_t kFusedMaxCells = 125;
-// Grids with more atoms per bin than this keep the three-launch pipeline
-// (measured at 370 atoms per bin, rc 14 on the cluster liquid: one launch
-// 326 us against 189 us for count + scan + emit).
-constexpr double kFusedMaxPerBin = 64.0;
-// Hit-mask words a group keeps in shared memory: enough for every stencil
-// cell at 1.5 x the mean bin occupancy, within these bounds (cells beyond
-// the budget recompute their tests when the group writes).
-constexpr int32_t kFusedMaskMin = 4096;
-constexpr int32_t kFusedMaskMax = 12288;
-struct FusedOut {
-  int64_t* src;       // [capacity] sources
-  int64_t* dst;       // [capacity] destinations (a separate array)
-  int32_t* sh;        // [3 capacity] shifts
-  int64_t capacity;   // a group whose block does not fit writes nothing
-  uint64_t* state;    // zeroed: [0] group ticket, [1] error word, [2 + g] group g's look-back word
-  int64_t* total;     // receives M
-  // Zeroed completion count of the groups; the group that completes it
-  // copies {M, error word} into `report` (host-mapped pinned memory, may be
-  // null) and then sets report[0] = 1, so the host learns M without waiting
-  // for the launch (or the ones queued after it) to end.
-  unsigned long long* done;
-  int64_t* report;
-  // 1: after the last group, the CTAs move the M destinations behind the M
-  // sources (src[M + e] = dst[e]: the [src | dst] layout of device results).
-  int32_t move;
-  int32_t spin_limit; // polls of one look-back wait before it gives up
-  int32_t withhold;   // failure-detection hook: this group never publishes (-1: none)
-  int32_t mask_words; // hit-mask words per group in shared memory
+// ---- k_group.cu : single-cutoff search in two launches (count with hit
+// masks, emit), a segment of a 32-atom group's stencil cells per warp.  Needs
+// the groups in canonical order (GridBuffers::group_start set for the build)
+// and GridBuffers::loose.
+struct GroupBand {
+  double rc_sq;
+  float rc2;       // rc^2, rounded
+  float width;     // pairs with |d2_32 - rc2| <= width are decided in FP64
+  float reach_sq;  // candidates farther than this from the group's box cannot hit
 };
-__host__ __device__ inline size_t fused_cells_bytes(int32_t n_cells) {
-  return ((size_t)88 * (size_t)n_cells + 15) & ~(size_t)15;
+GroupBand group_band(const GuardBand& band);
+struct GroupSearch {
+  uint64_t* state;      // zeroed: [1] error word
+  uint64_t* block_sum;  // zeroed: [group_blocks] edges of each block of kGroupBlock groups
+  int64_t* total;       // receives M
+  // Zeroed completion count of the count pass's CTAs; the last one scans the
+  // blocks, copies {M, error words, records asked for} into `report`
+  // (host-mapped pinned memory, may be null) and then sets report[0] = 1.
+  int32_t* done;
+  int64_t* report;
+  unsigned long long* chunk_top;  // zeroed: [16 r] records asked for in region r
+  int64_t* records;               // receives the room needed for all of them
+  int64_t chunk_cap;              // records there is room for (more: the host grows them)
+  uint32_t* masks;   // [32 chunk_cap] hit mask of each atom of the group over the candidates
+  uint32_t* cand;    // [32 chunk_cap] candidates' slots; top bit: the record has image shifts
+  uint32_t* cshift;  // [32 chunk_cap] image shifts, three signed 10-bit fields
+  int32_t* group_done;  // zeroed: [max_groups] counted segments of each group
+  int64_t* block_base;  // [group_blocks] first output slot of each block
+  int64_t* group_total; // [max_groups] edges of each group
+  int64_t* atom_base;   // [32 max_groups] first slot of each atom within its group
+  uint32_t* seg_cnt;    // [32 max_groups split] hits of each atom in the segments before
+  longlong2* seg_rec;   // [max_groups split] {first record, records}
+  int64_t max_groups;
+  int32_t split;        // segments per group (at most the stencil cells)
+  int32_t spin_limit;   // polls of one wait for a block's groups before it gives up
+  int32_t withhold;     // failure-detection hook: this group never joins its block (-1: none)
+};
+constexpr int32_t kGroupBlock = 64;
+constexpr int32_t kGroupRegions = 32;
+inline int64_t group_blocks(int64_t max_groups) {
+  return (max_groups + kGroupBlock - 1) / kGroupBlock;
 }
-size_t fused_smem_bytes(int32_t n_cells, int32_t mask_words);
-constexpr int32_t kFusedSpinLimit = 1 << 22;
-void launch_pair_fused(const GridParams& g, const GridBuffers& b, int32_t n_cells,
-                       const GuardBand& band, const FusedOut& o, cudaStream_t s);
+constexpr int32_t kGroupSpinLimit = 1 << 22;
+void launch_group_count(const GridParams& g, const GridBuffers& b, int32_t n_cells,
+                        const GroupBand& band, const GroupSearch& o, cudaStream_t s);
+// The list [src | dst] with dst = src + M, and its shifts; nothing when M is
+// above the capacity or the records did not fit.
+void launch_group_emit(const GridParams& g, const GridBuffers& b, int32_t n_cells,
+                       const GroupBand& band, const GroupSearch& o, int64_t* src, int32_t* sh,
+                       int64_t capacity, cudaStream_t s);
 
 // Returns false when the FP32 test cannot be made safe for this grid (the
 // band would be too wide); callers then use the FP64 kernels.

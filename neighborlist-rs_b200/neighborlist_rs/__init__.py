@@ -498,15 +498,15 @@ _lib.nlb_last_single_pipeline.restype = ctypes.c_int32
 
 
 def last_single_pipeline() -> int:
-    """Pipeline of this thread's last single-cutoff cell-list build: 0 = one
-    launch, 1 = three launches, -1 = none yet."""
+    """Pipeline of this thread's last single-cutoff cell-list build: 0 = the
+    group search, 1 = pair tasks, -1 = none yet."""
     return int(_lib.nlb_last_single_pipeline())
 
 
 def set_single_pipeline(mode: int | None) -> int:
-    """Single-system pipeline: 0 (or None) = automatic (one launch for count,
-    offsets and emit on sparse grids), 1 = always the three-launch pair-task
-    pipeline.  Identical results either way; returns the previous mode."""
+    """Single-system pipeline: 0 (or None) = the two-launch group search (count
+    with hit masks, emit), 1 = the three-launch pair-task pipeline.  Identical
+    results either way; returns the previous mode."""
     r = int(_lib.nlb_single_pipeline(0 if mode is None else int(mode)))
     if r < 0:
         raise ValueError(f"no single-system pipeline mode {mode}")
