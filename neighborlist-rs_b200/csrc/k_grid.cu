@@ -581,6 +581,123 @@ __global__ void __launch_bounds__(kSortThreads)
   if (p32 && below == 0) store_groups(g, r, s, e, so.lin, groups, counters, group_start);
 }
 
+// Bucket build (GridBuffers::bucket): wrap, Morton key, bin, and the atom's
+// entry in its bin's bucket (atoms past the bucket's end are found by their
+// rank).
+__global__ void __launch_bounds__(kPrepThreads)
+    k_prep_bucket(const __grid_constant__ GridParams g, const double* __restrict__ pos, int64_t n,
+                  const int32_t* __restrict__ rank_of_bin, uint64_t* __restrict__ key,
+                  int32_t* __restrict__ rank, int32_t* __restrict__ bin_count,
+                  uint64_t* __restrict__ bkey, int32_t* __restrict__ bidx, int32_t bucket) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const AtomWrap w = wrap_atom(g, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]);
+  const int32_t r = rank_of_bin[w.bin[0] + g.nb[0] * (w.bin[1] + g.nb[1] * w.bin[2])];
+  const int32_t at = atomicAdd(&bin_count[r], 1);
+  key[i] = w.key;
+  rank[i] = r;
+  if (at < bucket) {
+    bkey[(int64_t)r * bucket + at] = w.key;
+    bidx[(int64_t)r * bucket + at] = (int32_t)i;
+  }
+}
+
+// Every CTA scans the histogram (bin starts and first groups in shared
+// memory; CTA 0 also stores them), then kBucketSplit threads per atom count
+// the bin's (key, index) pairs below its own and one of them writes the
+// atom's slot; the atom placed first in its bin writes the bin's groups.
+constexpr int kBucketSplit = 8;
+__global__ void __launch_bounds__(kSortThreads)
+    k_place_bucket(const __grid_constant__ GridParams g, const double* __restrict__ pos, int64_t n,
+                   const __grid_constant__ GridBuffers b) {
+  extern __shared__ int32_t s_scan[];
+  __shared__ uint64_t warp_tot[kSortThreads / 32];
+  __shared__ int32_t warp_max[kSortThreads / 32];
+  const int32_t nb = (int32_t)g.total_bins;
+  int32_t* const s_start = s_scan;
+  int32_t* const s_group = s_scan + nb + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
+  const int64_t i = ((int64_t)blockIdx.x * kSortThreads + tid) / kBucketSplit;
+  const int part = tid % kBucketSplit;
+  const uint64_t k = i < n ? b.key[i] : 0ull;
+  const int32_t r = i < n ? b.rank[i] : 0;
+  {
+    const int32_t per = (nb + kSortThreads - 1) / kSortThreads;
+    const int32_t b0 = min(tid * per, nb), b1 = min(b0 + per, nb);
+    uint64_t sum = 0;  // groups above, atoms below
+    int32_t most = 0;
+#pragma unroll 4
+    for (int32_t c = b0; c < b1; ++c) {
+      const int32_t v = b.bin_count[c];
+      most = max(most, v);
+      sum += (uint64_t)((v + 31) / 32) << 32 | (uint64_t)v;
+      s_start[c] = v;
+    }
+    uint64_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 31) {
+      warp_tot[warp] = x;
+      warp_max[warp] = most;
+    }
+    __syncthreads();
+    uint64_t run = x - sum;
+    for (int w = 0; w < warp; ++w) run += warp_tot[w];
+    for (int32_t c = b0; c < b1; ++c) {
+      const int32_t v = s_start[c];
+      s_start[c] = (int32_t)run;
+      s_group[c] = (int32_t)(run >> 32);
+      if (blockIdx.x == 0) b.bin_start[c] = (int64_t)(uint32_t)run;
+      run += (uint64_t)((v + 31) / 32) << 32 | (uint64_t)v;
+    }
+    if (tid == 0) s_start[nb] = (int32_t)n;
+    if (blockIdx.x == 0 && tid == kSortThreads - 1) {
+      b.bin_start[nb] = n;
+      b.counters[0] = (int32_t)(run >> 32);
+      int32_t top = 0;
+      for (int w = 0; w < kSortThreads / 32; ++w) top = max(top, warp_max[w]);
+      *b.max_bin = top;
+    }
+    __syncthreads();
+  }
+  if (i >= n) return;  // (the same for an atom's threads)
+  const int32_t s = s_start[r], cnt = s_start[r + 1] - s;
+  int32_t below = 0;
+  if (cnt <= b.bucket) {
+    const uint64_t* bk = b.skey + (int64_t)r * b.bucket;
+    const int32_t* bi = b.sidx + (int64_t)r * b.bucket;
+#pragma unroll 4
+    for (int32_t q = part; q < cnt; q += kBucketSplit)
+      below += pair_less(bk[q], bi[q], k, (int32_t)i) ? 1 : 0;
+  } else {  // a bin above its bucket: every atom of the system
+    for (int32_t q = part; q < (int32_t)n; q += kBucketSplit)
+      below += b.rank[q] == r && pair_less(b.key[q], q, k, (int32_t)i) ? 1 : 0;
+  }
+  const unsigned mates = ((1u << kBucketSplit) - 1u) << (lane & ~(kBucketSplit - 1));
+#pragma unroll
+  for (int o = 1; o < kBucketSplit; o <<= 1) below += __shfl_xor_sync(mates, below, o);
+  if (part != 0) return;
+  const SlotOut so = store_slot(g, pos, s + below, (int32_t)i, b.px, b.py, b.pz, b.meta, b.p32,
+                                b.sbin, b.irr_list, b.irr, b.counters, b.loose);
+  if (below == 0) {
+    GroupRec gr;
+    gr.end = s + cnt;
+    gr.lin = so.lin;
+    gr.bx = so.lin % g.nb[0];
+    gr.by = (so.lin / g.nb[0]) % g.nb[1];
+    gr.bz = so.lin / (g.nb[0] * g.nb[1]);
+    for (int c = 0; 32 * c < cnt; ++c) {
+      gr.first = s + 32 * c;
+      b.groups[s_group[r] + c] = gr;
+    }
+  }
+}
+
 // Bounding box of every 32-atom group's chunk (one warp per group).
 __global__ void k_chunk_box(const GroupRec* __restrict__ groups,
                             const int32_t* __restrict__ counters, const float4* __restrict__ p32,
@@ -660,6 +777,15 @@ void launch_grid_build(const GridParams& g, const double* pos, int64_t n, const 
   if (need_rank_table) {
     k_rank_table<<<(unsigned)((g.total_bins + T - 1) / T), T, 0, s>>>(g, b.rank_of_bin);
     note_launches(1);
+  }
+  if (b.bucket > 0) {
+    k_prep_bucket<<<(unsigned)((n + kPrepThreads - 1) / kPrepThreads), kPrepThreads, 0, s>>>(
+        g, pos, n, b.rank_of_bin, b.key, b.rank, b.bin_count, b.skey, b.sidx, b.bucket);
+    const size_t smem = sizeof(int32_t) * (2 * (size_t)g.total_bins + 1);
+    launch_pdl(k_place_bucket, dim3((unsigned)((kBucketSplit * n + kSortThreads - 1) / kSortThreads)),
+               dim3(kSortThreads), smem, s, g, pos, n, b);
+    note_launches(2);
+    return;
   }
   const bool own_scan = b.build_done != nullptr && g.total_bins <= kPrepBinScanMax;
   k_prep<<<(unsigned)((n + kPrepThreads - 1) / kPrepThreads), kPrepThreads, 0, s>>>(

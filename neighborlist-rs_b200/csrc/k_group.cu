@@ -381,6 +381,7 @@ __device__ void finish_list(const GridBuffers& b, const GroupSearch& o, int32_t 
       r[1] = M;
       r[2] = err;
       r[3] = records;
+      r[4] = b.max_bin ? *b.max_bin : 0;
       __threadfence_system();
       r[0] = 1;
     }
@@ -475,6 +476,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
       const float2 cx2 = make_float2(cx, cx), cy2 = make_float2(cy, cy),
                    cz2 = make_float2(cz, cz);
       float closest = INFINITY;  // smallest |t|
+#pragma unroll 2
       for (int q = 0; q < n_quads; ++q) {
         unsigned m[4];
 #pragma unroll
@@ -488,7 +490,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
           m[2 * h + 1] = __ballot_sync(0xffffffffu, d2.y < 0.f && __float_as_int(zi.w) < jj);
           closest = fminf(fminf(closest, fabsf(d2.x)), fabsf(d2.y));
         }
-        if (lane == 0) w_sm.mask[q] = make_uint4(m[0], m[1], m[2], m[3]);
+        w_sm.mask[q] = make_uint4(m[0], m[1], m[2], m[3]);
       }
       if (__any_sync(0xffffffffu, closest <= band.width) || near_lo == -INFINITY) {
         // Some pair lies within the guard band: the reference's FP64 test.

@@ -42,6 +42,7 @@ struct FastKey {
   int32_t need_rank;
   int32_t prof;
   int32_t split;  // segments per group (0: pair tasks)
+  int32_t bucket;
 };
 
 struct FastState {
@@ -52,6 +53,7 @@ struct FastState {
   int64_t last_m = 0;
   int64_t last_mask_words = 0;
   int64_t last_records = 0;  // records the last group search asked for
+  int64_t bin_n = 0, bin_nb = 0, bin_max = 0;  // largest bin of the last bucket build
 };
 
 thread_local FastState tl_states[16];
@@ -116,7 +118,7 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   // Zeroed block, so that a single memset at the start clears everything and
   // the kernels follow each other directly: bin histogram, scatter cursors, 2
   // task counters, 64-bit mask cursor (8-byte aligned: 2 nb + 2 is even),
-  // build completion count, emit task counter, loose flag and padding, then
+  // build completion count, emit task counter, loose flag, largest bin, then
   // (8-byte aligned) the offsets scan's state, or the group search's ticket,
   // error word, total, completion count, record cursor, block sums and segment
   // counts and the bin scan's state.
@@ -135,6 +137,7 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   b.build_done = zeroed + 2 * nb + 4;
   b.emit_queue = reinterpret_cast<uint32_t*>(zeroed + 2 * nb + 5);
   b.loose = zeroed + 2 * nb + 6;
+  b.max_bin = zeroed + 2 * nb + 7;
   int64_t* state = reinterpret_cast<int64_t*>(zeroed + 2 * nb + 8);
   sp.scan_state = state;
   b.bin_scan = bin_scan ? reinterpret_cast<uint64_t*>(state + group_words) : nullptr;
@@ -184,8 +187,9 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   b.bin_start = slot<int64_t>(c, kSlotBinStart, nb + 1);
   b.key = slot<uint64_t>(c, kSlotKey, n);
   b.rank = slot<int32_t>(c, kSlotRank, n);
-  b.skey = slot<uint64_t>(c, kSlotSkey, n);
-  b.sidx = slot<int32_t>(c, kSlotSidx, n);
+  const int64_t entries = b.bucket > 0 ? nb * b.bucket : n;
+  b.skey = slot<uint64_t>(c, kSlotSkey, entries);
+  b.sidx = slot<int32_t>(c, kSlotSidx, entries);
   b.skey2 = slot<uint64_t>(c, kSlotSkey2, n);
   b.sidx2 = slot<int32_t>(c, kSlotSidx2, n);
   b.px = slot<double>(c, kSlotPx, n);
@@ -322,6 +326,17 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   sp.grouped = single_pipeline_mode() == 0 && sp.n < ((int64_t)1 << 26);
   sp.search.split = sp.grouped ? group_split(sp.n, sp.grid.total_bins, cells) : 0;
   tl_last_pipeline = sp.grouped ? 0 : 1;
+  sp.gb.bucket = 0;
+  if (sp.grouped && bucket_build(sp.n, sp.grid.total_bins)) {
+    // Room for four times the mean bin, and for the largest of the last
+    // system of this size; within 64 MB.
+    int64_t most = 4 * sp.n / sp.grid.total_bins;
+    if (fs.bin_n == sp.n && fs.bin_nb == sp.grid.total_bins)
+      most = std::max(most, fs.bin_max + fs.bin_max / 4);
+    int64_t bucket = 32;
+    while (bucket < most) bucket *= 2;
+    if (bucket * sp.grid.total_bins * 12 <= (int64_t)64 << 20) sp.gb.bucket = (int32_t)bucket;
+  }
   const double rc = std::sqrt(sp.rc_sq[0]);
   int64_t capacity = std::max<int64_t>(
       {4096, (int64_t)(1.25 * (double)fs.last_m), (int64_t)(1.5 * (double)estimate_edges(sp, rc))});
@@ -362,6 +377,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   key.need_rank = sp.rank_cached ? 0 : 1;
   key.prof = c.prof ? 1 : 0;
   key.split = sp.search.split;
+  key.bucket = sp.gb.bucket;
 
   const bool report = !c.prof;
   if (report) c.h_report[0] = 0;
@@ -422,6 +438,11 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
     const int64_t m = r[1];
     if (r[2] != 0) return fail(NLB_ERR_CUDA, "prefix scan gave up waiting for a tile");
     if (sp.grouped) fs.last_records = r[3];
+    if (sp.gb.bucket > 0) {
+      fs.bin_n = sp.n;
+      fs.bin_nb = sp.grid.total_bins;
+      fs.bin_max = r[4];
+    }
     if (m <= capacity && (!sp.grouped || r[3] <= sp.search.chunk_cap)) {
       if (c.stream == c.own_stream) {
         if (!stream_ordered) {

@@ -107,7 +107,21 @@ struct GridBuffers {
   // (bin_scan_words(total_bins), zeroed by the caller before the build; used
   // when group_start is set); [1] is its error word.
   uint64_t* bin_scan;
+  // Bucket build (bucket > 0; see bucket_build): k_prep puts every atom
+  // straight into its bin's bucket (skey, sidx: total_bins x bucket entries),
+  // and the placement scans the histogram itself.  max_bin receives the
+  // largest bin's count.
+  int32_t bucket;
+  int32_t* max_bin;
 };
+
+// Systems that take the bucket build: small ones, where the launches saved
+// count for more than reading the bins' buckets in the atoms' order (each CTA
+// of the placement scans the whole histogram, and a bin above its bucket
+// compares with every atom of the system).
+inline bool bucket_build(int64_t n, int64_t total_bins) {
+  return n <= 32768 && total_bins <= 3072;
+}
 
 // Grids with at least this many atoms per bin on average get chunk boxes.
 constexpr double kChunkPruneMinPerBin = 64.0;
