@@ -262,6 +262,12 @@ int nlb_build_ex(const double* positions, int64_t n_atoms, double cutoff, const 
                  const uint8_t* pbc, int flags, nlb_result_ex* out);
 int nlb_build_device_ex(const double* d_positions, int64_t n_atoms, double cutoff,
                         const double* cell, const uint8_t* pbc, int flags, nlb_result_ex* out);
+/* As nlb_build_device_ex, but hands the arrays over: device blocks that the
+ * caller returns with nlb_device_free, complete in the order of the active
+ * stream (nlb_set_stream); NULL when there are no edges. */
+int nlb_build_device_ex_owned(const double* d_positions, int64_t n_atoms, double cutoff,
+                              const double* cell, const uint8_t* pbc, int flags,
+                              nlb_result_ex* out);
 void nlb_result_ex_free(nlb_result_ex* r);
 
 /* ---- Verlet (skin) list manager for MD (asked for by the reference's

@@ -152,14 +152,62 @@ __device__ __forceinline__ void g_place_cell(const GridParams& g, const int32_t 
   }
 }
 
+// Writes edge e (atoms i, j, shift s): sources and destinations in ei, shifts
+// in sh.  EX: the output options too -- the directed list's reverse edge (j,
+// i, -s) at M + e, the displacement d = (r_j - r_i) + H s (-d for the reverse)
+// and its length -- with the expressions of k_extras.cu.  d_ei: entries
+// between the sources and the destinations.
+template <bool EX>
+__device__ __forceinline__ void write_edge(const GroupOut& o, int64_t d_ei, int64_t M, int64_t e,
+                                           int32_t i, int32_t j, int32_t s0, int32_t s1,
+                                           int32_t s2) {
+  o.ei[e] = (int64_t)i;
+  o.ei[d_ei + e] = (int64_t)j;
+  int32_t* sp = o.sh + 3 * e;
+  sp[0] = s0;
+  sp[1] = s1;
+  sp[2] = s2;
+  if (!EX) return;
+  if (o.directed) {
+    o.ei[M + e] = (int64_t)j;
+    o.ei[d_ei + M + e] = (int64_t)i;
+    sp += 3 * M;
+    sp[0] = -s0;
+    sp[1] = -s1;
+    sp[2] = -s2;
+  }
+  if (!o.vec && !o.dist) return;
+  double d[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    d[k] = dsub(__ldg(&o.pos[3 * (int64_t)j + k]), __ldg(&o.pos[3 * (int64_t)i + k]));
+    if (o.cell.has_cell)
+      d[k] = dadd(d[k], dadd(dadd(dmul(o.cell.h[3 * k], (double)s0),
+                                  dmul(o.cell.h[3 * k + 1], (double)s1)),
+                             dmul(o.cell.h[3 * k + 2], (double)s2)));
+  }
+  if (o.vec) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      o.vec[3 * e + k] = d[k];
+      if (o.directed) o.vec[3 * (M + e) + k] = -d[k];
+    }
+  }
+  if (o.dist) {
+    const double r = __dsqrt_rn(norm2(d[0], d[1], d[2]));
+    o.dist[e] = r;
+    if (o.directed) o.dist[M + e] = r;
+  }
+}
+
 // Irregular atom p (its home stencil is not its stored bin): one warp walks
 // its own stencil in FP64 exactly like pair_irregular in k_search2.cu.
 // Returns its edge count; EMIT: its edges go to slots [e0, ...) in canonical
 // order.
-template <bool EMIT>
+template <bool EMIT, bool EX>
 __device__ uint32_t g_irregular(const GridParams& g, const GridBuffers& b, int32_t n_cells,
-                                double rc_sq, int32_t p, int64_t e0, int64_t* src, int64_t* dst,
-                                int32_t* shifts) {
+                                double rc_sq, int32_t p, int64_t e0, const GroupOut* out,
+                                int64_t d_ei, int64_t M) {
   const int lane = threadIdx.x & 31;
   const double xi = b.px[p], yi = b.py[p], zi = b.pz[p];
   const SlotMeta mi = b.meta[p];
@@ -193,12 +241,9 @@ __device__ uint32_t g_irregular(const GridParams& g, const GridBuffers& b, int32
       const unsigned m = __ballot_sync(0xffffffffu, hit);
       if (EMIT && hit) {
         const int64_t e = e0 + count + __popc(m & lanemask_lt());
-        src[e] = (int64_t)mi.orig;
-        dst[e] = (int64_t)mj.orig;
-        int32_t* sp = shifts + 3 * e;
-        sp[0] = (mj.sx - mi.sx) + unpack_shift(csh, 0);
-        sp[1] = (mj.sy - mi.sy) + unpack_shift(csh, 1);
-        sp[2] = (mj.sz - mi.sz) + unpack_shift(csh, 2);
+        write_edge<EX>(*out, d_ei, M, e, mi.orig, mj.orig, (mj.sx - mi.sx) + unpack_shift(csh, 0),
+                       (mj.sy - mi.sy) + unpack_shift(csh, 1),
+                       (mj.sz - mi.sz) + unpack_shift(csh, 2));
       }
       count += __popc(m);
     }
@@ -305,8 +350,8 @@ __device__ __forceinline__ void finish_group(const GridParams& g, const GridBuff
   }
   for (unsigned m = irr_mask; m; m &= m - 1) {
     const int l = __ffs(m) - 1;
-    const uint32_t v = g_irregular<false>(g, b, n_cells, band.rc_sq, grp.first + l, 0, nullptr,
-                                          nullptr, nullptr);
+    const uint32_t v = g_irregular<false, false>(g, b, n_cells, band.rc_sq, grp.first + l, 0,
+                                                 nullptr, 0, 0);
     if (lane == l) run = v;
   }
   int64_t x = run;
@@ -654,17 +699,18 @@ __device__ __forceinline__ void copy16(void* smem, const void* global) {
 // Emit pass (the file comment).  Writes nothing when a wait gave up, the list
 // does not fit, or the records did not (the host then grows the arrays and
 // runs what is missing again).
+template <bool EX>
 __global__ void __launch_bounds__(kGThreads, 28)
     k_group_emit(const __grid_constant__ GridParams g, const __grid_constant__ GridBuffers b,
                  int32_t n_cells, double rc_sq, const __grid_constant__ GroupSearch o,
-                 int64_t* __restrict__ src, int32_t* __restrict__ sh, int64_t capacity) {
+                 const __grid_constant__ GroupOut out) {
   extern __shared__ __align__(16) unsigned char gsm[];
   const int lane = threadIdx.x;
   GEmitWarp& w_sm = *reinterpret_cast<GEmitWarp*>(gsm);
   pdl_wait();
   const int64_t M = *o.total;
-  if (o.state[1] != 0 || M > capacity || *o.records > o.chunk_cap) return;
-  int64_t* __restrict__ dst = src + M;
+  if (o.state[1] != 0 || M > out.capacity || *o.records > o.chunk_cap) return;
+  const int64_t d_ei = EX && out.directed ? 2 * M : M;
   const int32_t split = o.split;
   const int64_t n_items = (int64_t)b.counters[0] * split;
   const int64_t item = blockIdx.x;
@@ -758,12 +804,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
         s1 = mj.sy + unpack_shift(csh, 1);
         s2 = mj.sz + unpack_shift(csh, 2);
       }
-      src[e] = (int64_t)ml.orig;
-      dst[e] = (int64_t)cj.y;
-      int32_t* sp = sh + 3 * e;
-      sp[0] = s0 - ml.sx;
-      sp[1] = s1 - ml.sy;
-      sp[2] = s2 - ml.sz;
+      write_edge<EX>(out, d_ei, M, e, ml.orig, cj.y, s0 - ml.sx, s1 - ml.sy, s2 - ml.sz);
     }
     __syncwarp();
     r0 += n_win;
@@ -772,7 +813,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
     const int l = __ffs(im) - 1;
     const int64_t e0 =
         o.block_base[t / kGroupBlock] + base + o.atom_base[(int64_t)t * 32 + l];
-    g_irregular<true>(g, b, n_cells, rc_sq, grp.first + l, e0, src, dst, sh);
+    g_irregular<true, EX>(g, b, n_cells, rc_sq, grp.first + l, e0, &out, d_ei, M);
   }
 }
 
@@ -800,12 +841,11 @@ void launch_group_count(const GridParams& g, const GridBuffers& b, int32_t n_cel
 }
 
 void launch_group_emit(const GridParams& g, const GridBuffers& b, int32_t n_cells,
-                       const GroupBand& band, const GroupSearch& o, int64_t* src, int32_t* sh,
-                       int64_t capacity, cudaStream_t s) {
-  const size_t smem = sizeof(GEmitWarp);
-  ensure_smem_attr((const void*)k_group_emit, (int)smem);
-  launch_pdl(k_group_emit, dim3((unsigned)(o.max_groups * o.split)), dim3(kGThreads), smem, s, g, b, n_cells,
-             band.rc_sq, o, src, sh, capacity);
+                       const GroupBand& band, const GroupSearch& o, const GroupOut& out,
+                       cudaStream_t s) {
+  const auto k = out.directed || out.vec || out.dist ? &k_group_emit<true> : &k_group_emit<false>;
+  launch_pdl(k, dim3((unsigned)(o.max_groups * o.split)), dim3(kGThreads), sizeof(GEmitWarp), s, g,
+             b, n_cells, band.rc_sq, o, out);
   note_launches(1);
 }
 

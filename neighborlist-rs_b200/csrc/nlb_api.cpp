@@ -351,6 +351,20 @@ void take_result_arrays(Ctx& c, int64_t** ei, int32_t** sh) {
   *bs[1] = Ctx::Buf{};
 }
 
+void* take_slot(Ctx& c, void* p) {
+  if (!p) return nullptr;
+  ResultPool& rp = result_pool();
+  std::lock_guard<std::mutex> lk(rp.mu);
+  for (Ctx::Buf& b : c.bufs) {
+    if (b.p != p) continue;
+    rp.owned[p] = {c.device, b.cap};
+    ++rp.handed;
+    b = Ctx::Buf{};
+    return p;
+  }
+  return nullptr;
+}
+
 void warm_result_pool(int device, size_t bytes, cudaStream_t s) {
   cudaMemPool_t pool = result_pool_for(device);
   void* p = nullptr;
@@ -939,7 +953,7 @@ Status run_single(const double* pos, int64_t n, const double* cell9, const uint8
 // without it the bounds come from the device positions.
 Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int64_t n,
                         const double* cell9, const uint8_t* pbc, double cutoff, int64_t** ei,
-                        int32_t** sh, int64_t* m) {
+                        int32_t** sh, int64_t* m, int flags, nlb_result_ex* ex) {
   double bounds[6];
   const double* bptr = nullptr;
   if (!cell9 && !pos_host) {
@@ -958,10 +972,25 @@ Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int
   Status st = plan_system(pos_host, n, cell9, pb, cs, false, false, sp, bptr);
   if (!st.ok()) return st;
   if (fast_eligible(sp)) {
+    const bool direct = ex && flags && takes_group_search(sp);
+    if (direct) {
+      sp.ex_flags = flags;
+      if (cell9) {
+        std::memcpy(sp.ex_cell.h, cell9, sizeof(sp.ex_cell.h));
+        sp.ex_cell.has_cell = 1;
+      }
+    }
     st = run_fast(c, sp, d_pos, m);
     if (!st.ok()) return st;
     *ei = sp.out_src;
     *sh = sp.out_sh;
+    if (direct) {
+      ex->n_edges = flags & NLB_DIRECTED ? 2 * *m : *m;
+      ex->edge_index = sp.out_src;
+      ex->shift = sp.out_sh;
+      ex->vectors = sp.out_vec;
+      ex->distances = sp.out_dist;
+    }
     return Status{NLB_OK};
   }
   st = count_system(c, sp, d_pos);
@@ -1020,9 +1049,12 @@ bool extras_flags_valid(int flags) {
 }
 
 // nlb_build_ex / nlb_build_device_ex: d_pos_in == nullptr means host
-// positions (uploaded here) and pinned host results.
+// positions (uploaded here) and pinned host results.  owned (device results):
+// the arrays are handed over to the caller, complete in the order of the
+// active stream.
 Status run_single_ex(const double* pos, const double* d_pos_in, int64_t n, const double* cell9,
-                     const uint8_t* pbc, double cutoff, int flags, nlb_result_ex* out) {
+                     const uint8_t* pbc, double cutoff, int flags, nlb_result_ex* out,
+                     bool owned = false) {
   std::memset(out, 0, sizeof(*out));
   if (!extras_flags_valid(flags)) return fail(NLB_ERR_VALUE, "unknown output option flags");
   if (!cutoffs_valid(&cutoff, 1)) return fail(NLB_ERR_VALUE, "Cutoff must be positive and finite");
@@ -1036,6 +1068,8 @@ Status run_single_ex(const double* pos, const double* d_pos_in, int64_t n, const
   int32_t* sh = nullptr;
   int64_t m = 0;
   const double* d_pos = d_pos_in;
+  nlb_result_ex dev;
+  std::memset(&dev, 0, sizeof(dev));
   if (n > 0) {
     if (host) {
       double* up = nullptr;
@@ -1043,17 +1077,27 @@ Status run_single_ex(const double* pos, const double* d_pos_in, int64_t n, const
       if (!st.ok()) return st;
       d_pos = up;
     }
-    st = half_list_device(*c, host ? pos : nullptr, d_pos, n, cell9, pbc, cutoff, &ei, &sh, &m);
+    st = half_list_device(*c, host ? pos : nullptr, d_pos, n, cell9, pbc, cutoff, &ei, &sh, &m,
+                          flags, &dev);
     if (!st.ok()) return st;
   }
-  nlb_result_ex dev;
-  st = apply_extras(*c, d_pos, cell9, flags, ei, sh, m, &dev);
+  // (the group search's emit pass has written them already)
+  const bool written = dev.edge_index != nullptr;
+  if (!written) st = apply_extras(*c, d_pos, cell9, flags, ei, sh, m, &dev);
   if (!st.ok()) return st;
   if (!host) {
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "edge extras");
+    if (!(owned && written)) {
+      cudaError_t e = cudaStreamSynchronize(c->stream);
+      if (e != cudaSuccess) return cuda_fail(e, "edge extras");
+    }
     if (c->prof) c->harvest();
     *out = dev;
+    if (!owned) return Status{NLB_OK};
+    const bool any = dev.n_edges > 0;
+    out->edge_index = any ? static_cast<int64_t*>(take_slot(*c, dev.edge_index)) : nullptr;
+    out->shift = any ? static_cast<int32_t*>(take_slot(*c, dev.shift)) : nullptr;
+    out->vectors = any ? static_cast<double*>(take_slot(*c, dev.vectors)) : nullptr;
+    out->distances = any ? static_cast<double*>(take_slot(*c, dev.distances)) : nullptr;
     return Status{NLB_OK};
   }
   // Pinned host results.
@@ -1244,6 +1288,20 @@ int nlb_build_device_ex(const double* d_positions, int64_t n_atoms, double cutof
   static const double kNone = 0.0;
   return run_single_ex(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell, pbc, cutoff,
                        flags, out)
+      .code;
+}
+
+int nlb_build_device_ex_owned(const double* d_positions, int64_t n_atoms, double cutoff,
+                              const double* cell, const uint8_t* pbc, int flags,
+                              nlb_result_ex* out) {
+  if (!out) return fail(NLB_ERR_VALUE, "out is NULL").code;
+  if (!d_positions && n_atoms > 0) {
+    std::memset(out, 0, sizeof(*out));
+    return fail(NLB_ERR_VALUE, "positions is NULL").code;
+  }
+  static const double kNone = 0.0;
+  return run_single_ex(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell, pbc, cutoff,
+                       flags, out, true)
       .code;
 }
 

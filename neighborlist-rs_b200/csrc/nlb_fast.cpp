@@ -43,6 +43,7 @@ struct FastKey {
   int32_t prof;
   int32_t split;  // segments per group (0: pair tasks)
   int32_t bucket;
+  int32_t ex_flags;
 };
 
 struct FastState {
@@ -99,6 +100,17 @@ void release_fast_states() {
     if (fs.exec) cudaGraphExecDestroy(fs.exec);
     fs = FastState();
   }
+}
+
+// The result arrays for `capacity` half edges.
+bool out_arrays(Ctx& c, SystemPlan& sp, int64_t capacity) {
+  const size_t edges = (size_t)capacity * (sp.ex_flags & NLB_DIRECTED ? 2 : 1);
+  sp.out_src = slot<int64_t>(c, kSlotOutEi, 2 * edges);
+  sp.out_sh = slot<int32_t>(c, kSlotOutSh, 3 * edges);
+  const bool vec = sp.ex_flags & NLB_VECTORS, dist = sp.ex_flags & NLB_DISTANCES;
+  sp.out_vec = vec ? slot<double>(c, kSlotOutVec, 3 * edges) : nullptr;
+  sp.out_dist = dist ? slot<double>(c, kSlotOutDist, edges) : nullptr;
+  return sp.out_src && sp.out_sh && (!vec || sp.out_vec) && (!dist || sp.out_dist);
 }
 
 // Sizes every workspace buffer of the fast pipeline (may allocate; never
@@ -204,12 +216,12 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   b.scan_tmp = slot<int64_t>(c, kSlotScanTmp, scan_tmp_elems(sp.grouped ? nb : std::max<int64_t>(row, nb)));
   sp.counts = slot<uint32_t>(c, kSlotCounts, sp.grouped ? 1 : row);
   sp.offs = slot<int64_t>(c, kSlotOffs, sp.grouped ? 1 : row + 1);
-  sp.out_src = slot<int64_t>(c, kSlotOutEi, 2 * (size_t)capacity);
-  sp.out_sh = slot<int32_t>(c, kSlotOutSh, 3 * (size_t)capacity);
+  if (!out_arrays(c, sp, capacity))
+    return fail(NLB_ERR_NOMEM, "device allocation for the edge lists failed");
   if (!b.rank_of_bin || !b.bin_start || !b.key || !b.rank || !b.skey || !b.sidx || !b.skey2 ||
       !b.sidx2 || !b.px || !b.py || !b.pz || !b.meta || !b.p32 || !b.sbin || !b.groups ||
-      !b.irr_list || !b.irr || !b.scan_tmp || !sp.counts || !sp.offs || !sp.out_src ||
-      !sp.out_sh || !b.task_hdr || (chunk_boxes && !b.cbox) || !b.fill)
+      !b.irr_list || !b.irr || !b.scan_tmp || !sp.counts || !sp.offs ||
+      !b.task_hdr || (chunk_boxes && !b.cbox) || !b.fill)
     return fail(NLB_ERR_NOMEM, "device allocation failed");
   return Status{NLB_OK};
 }
@@ -230,7 +242,7 @@ int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
 }
 
 // The group search's two launches.
-void issue_search(Ctx& c, SystemPlan& sp, int64_t capacity, bool count) {
+void issue_search(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t capacity, bool count) {
   const GroupBand band = group_band(sp.band);
   const int32_t cells = (int32_t)stencil_cells_of(sp.grid);
   if (count) {
@@ -245,8 +257,17 @@ void issue_search(Ctx& c, SystemPlan& sp, int64_t capacity, bool count) {
     c.mark(3);
     c.mark(4);
   }
-  launch_group_emit(sp.grid, sp.gb, cells, band, sp.search, sp.out_src, sp.out_sh, capacity,
-                    c.stream);
+  GroupOut out;
+  std::memset(&out, 0, sizeof(out));
+  out.ei = sp.out_src;
+  out.sh = sp.out_sh;
+  out.vec = sp.out_vec;
+  out.dist = sp.out_dist;
+  out.pos = d_pos;
+  out.cell = sp.ex_cell;
+  out.capacity = capacity;
+  out.directed = sp.ex_flags & NLB_DIRECTED ? 1 : 0;
+  launch_group_emit(sp.grid, sp.gb, cells, band, sp.search, out, c.stream);
 }
 
 EmitTargets fast_targets(const SystemPlan& sp, int64_t capacity, int64_t* report = nullptr) {
@@ -274,7 +295,7 @@ void issue_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t capacity) {
   c.mark(1);
   if (sp.grouped) {
     // (Phases: the offsets are part of the count pass.)
-    issue_search(c, sp, capacity, true);
+    issue_search(c, sp, d_pos, capacity, true);
     c.mark(5);
     return;
   }
@@ -312,6 +333,12 @@ Status wait_report(Ctx& c) {
 // Runs the fast pipeline for a planned single-cutoff cell-list system and
 // leaves M edges in sp.out_src ([src | dst]) / sp.out_sh.
 //
+// (The group search counts a row of candidates -- at most 32 images of all
+// atoms -- in 32 bits.)
+bool takes_group_search(const SystemPlan& sp) {
+  return fast_eligible(sp) && single_pipeline_mode() == 0 && sp.n < ((int64_t)1 << 26);
+}
+
 // M reaches the host through host-mapped memory as soon as it is known: when
 // the count pass ends (mode 1: when its emit pass starts).  On a caller's
 // stream the call then returns at once: the emit is queued on that stream
@@ -321,9 +348,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
                 bool stream_ordered) {
   FastState& fs = state_for(c);
   const int64_t cells = stencil_cells_of(sp.grid);
-  // (the group search counts a row of candidates -- at most 32 images of all
-  // atoms -- in 32 bits)
-  sp.grouped = single_pipeline_mode() == 0 && sp.n < ((int64_t)1 << 26);
+  sp.grouped = takes_group_search(sp);
   sp.search.split = sp.grouped ? group_split(sp.n, sp.grid.total_bins, cells) : 0;
   tl_last_pipeline = sp.grouped ? 0 : 1;
   sp.gb.bucket = 0;
@@ -341,9 +366,13 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   int64_t capacity = std::max<int64_t>(
       {4096, (int64_t)(1.25 * (double)fs.last_m), (int64_t)(1.5 * (double)estimate_edges(sp, rc))});
   // Keep the arena's current size if it is already large enough.
-  const size_t have = c.bufs[kSlotOutSh].cap / (3 * sizeof(int32_t));
-  if ((int64_t)have > capacity && c.bufs[kSlotOutEi].cap / (2 * sizeof(int64_t)) >= have)
-    capacity = (int64_t)have;
+  const size_t per = sp.ex_flags & NLB_DIRECTED ? 2 : 1;
+  size_t have = std::min(c.bufs[kSlotOutSh].cap / (3 * sizeof(int32_t)),
+                         c.bufs[kSlotOutEi].cap / (2 * sizeof(int64_t)));
+  if (sp.ex_flags & NLB_VECTORS)
+    have = std::min(have, c.bufs[kSlotOutVec].cap / (3 * sizeof(double)));
+  if (sp.ex_flags & NLB_DISTANCES) have = std::min(have, c.bufs[kSlotOutDist].cap / sizeof(double));
+  if ((int64_t)(have / per) > capacity) capacity = (int64_t)(have / per);
   // Hit-mask arena: the last run's need x 1.25, at least 64 words per atom;
   // the group search's records (32 words each): one per 32 candidates of a
   // segment, with the groups and candidates of a uniform density.
@@ -378,6 +407,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   key.prof = c.prof ? 1 : 0;
   key.split = sp.search.split;
   key.bucket = sp.gb.bucket;
+  key.ex_flags = sp.ex_flags;
 
   const bool report = !c.prof;
   if (report) c.h_report[0] = 0;
@@ -497,9 +527,8 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
     // Too little room: grow it (outside any capture) and run what is missing
     // again.  The records: the count pass once more, its state cleared first.
     const int64_t cap2 = m > capacity ? m + m / 8 + 1024 : capacity;
-    sp.out_src = slot<int64_t>(c, kSlotOutEi, 2 * (size_t)cap2);
-    sp.out_sh = slot<int32_t>(c, kSlotOutSh, 3 * (size_t)cap2);
-    if (!sp.out_src || !sp.out_sh) return fail(NLB_ERR_NOMEM, "device allocation for the edge lists failed");
+    if (!out_arrays(c, sp, cap2))
+      return fail(NLB_ERR_NOMEM, "device allocation for the edge lists failed");
     if (recount) {
       GroupSearch& o = sp.search;
       o.masks = slot<uint32_t>(c, kSlotMasks, 32 * (size_t)records);
@@ -510,7 +539,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
       cudaMemsetAsync(o.state, 0, sizeof(uint64_t) * (size_t)group_state_words(o.max_groups), c.stream);
     }
     if (sp.grouped)
-      issue_search(c, sp, cap2, recount);
+      issue_search(c, sp, d_pos, cap2, recount);
     else
       launch_pair_emit(sp.grid, sp.gb, sp.n, sp.band, sp.offs, fast_targets(sp, cap2), c.stream);
     c.h_small[1] = 0;

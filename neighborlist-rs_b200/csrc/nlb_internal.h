@@ -61,6 +61,8 @@ enum Slot : int {
   kSlotAtomBase,
   kSlotSegCnt,
   kSlotSegRec,
+  kSlotOutVec,
+  kSlotOutDist,
   kSlotFill,
   kSlotBatch0,  // first slot owned by the batched path
   kSlotCount = kSlotBatch0 + 32,
@@ -135,6 +137,8 @@ Status get_ctx(Ctx** out);
 // the context forgets them and its next build allocates fresh ones from the
 // pool.  The caller returns each with nlb_device_free.
 void take_result_arrays(Ctx& c, int64_t** ei, int32_t** sh);
+// The same for the workspace slot that holds p (nullptr: nothing).
+void* take_slot(Ctx& c, void* p);
 // Frees the calling thread's contexts and fast-path graphs (threads that end
 // before the process does, e.g. server workers).
 void release_thread_ctx();
@@ -198,6 +202,12 @@ struct SystemPlan {
   int32_t* out_sh = nullptr;    // fast path: shift arena
   bool grouped = false;         // fast path: two-launch group search (k_group.cu)
   GroupSearch search{};         // its buffers
+  // Output options (NLB_* flags; group search only): the emit pass writes the
+  // final arrays (out_src, out_sh, out_vec, out_dist).
+  int ex_flags = 0;
+  EdgeExtrasCell ex_cell{};
+  double* out_vec = nullptr;
+  double* out_dist = nullptr;
   CutoffSet pass(int32_t g0) const;
 };
 
@@ -226,6 +236,8 @@ Status emit_system(Ctx& c, SystemPlan& sp, const double* d_pos, const DevLists& 
 // stream.
 Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
                 bool stream_ordered = false);
+// Whether run_fast takes the group search for this system.
+bool takes_group_search(const SystemPlan& sp);
 // Single-system pipeline choice: 0 = the two-launch group search, 1 = the
 // three-launch pair-task pipeline.
 int32_t single_pipeline_mode();

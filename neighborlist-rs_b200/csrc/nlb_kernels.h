@@ -204,6 +204,12 @@ struct PairBands {
 };
 // Stencils above this many cells use the per-atom FP64 kernels.
 constexpr int64_t kPairMaxCells = 1024;
+// Cell of the displacement vectors d = (r_j - r_i) + H.S.
+struct EdgeExtrasCell {
+  double h[9];       // row-major H (columns = lattice vectors)
+  int32_t has_cell;  // 0: no H term (vectors are r_j - r_i)
+};
+
 // ---- k_group.cu : single-cutoff search in two launches (count with hit
 // masks, emit), a segment of a 32-atom group's stencil cells per warp.  Needs
 // the groups in canonical order (GridBuffers::group_start set for the build)
@@ -249,11 +255,23 @@ inline int64_t group_blocks(int64_t max_groups) {
 constexpr int32_t kGroupSpinLimit = 1 << 22;
 void launch_group_count(const GridParams& g, const GridBuffers& b, int32_t n_cells,
                         const GroupBand& band, const GroupSearch& o, cudaStream_t s);
-// The list [src | dst] with dst = src + M, and its shifts; nothing when M is
-// above the capacity or the records did not fit.
+// Destinations of the group search: the list [src | dst] and its shifts, with
+// the output options of launch_edge_extras (vec, dist null: not wanted).
+// Nothing is written when M is above the capacity (edges of the half list) or
+// the records did not fit.
+struct GroupOut {
+  int64_t* ei;
+  int32_t* sh;
+  double* vec;
+  double* dist;
+  const double* pos;
+  EdgeExtrasCell cell;
+  int64_t capacity;
+  int32_t directed;
+};
 void launch_group_emit(const GridParams& g, const GridBuffers& b, int32_t n_cells,
-                       const GroupBand& band, const GroupSearch& o, int64_t* src, int32_t* sh,
-                       int64_t capacity, cudaStream_t s);
+                       const GroupBand& band, const GroupSearch& o, const GroupOut& out,
+                       cudaStream_t s);
 
 // Returns false when the FP32 test cannot be made safe for this grid (the
 // band would be too wide); callers then use the FP64 kernels.
@@ -385,10 +403,6 @@ void launch_bounds(const double* pos, int64_t n, double* out, cudaStream_t s);
 // Output options on a device half list ([src | dst] ei, shifts sh, m edges):
 // directed list, displacement vectors, distances (k_extras.cu).  Outputs
 // that are not wanted are NULL; with directed == 0 ei_out/sh_out may be NULL.
-struct EdgeExtrasCell {
-  double h[9];       // row-major H (columns = lattice vectors)
-  int32_t has_cell;  // 0: no H term (vectors are r_j - r_i)
-};
 void launch_edge_extras(const double* pos, const EdgeExtrasCell& cell, const int64_t* ei,
                         const int32_t* sh, int64_t m, int directed, int64_t* ei_out,
                         int32_t* sh_out, double* vec, double* dist, cudaStream_t s);

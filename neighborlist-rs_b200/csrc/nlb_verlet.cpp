@@ -35,7 +35,7 @@ constexpr int32_t kVerletSpinLimit = 1 << 22;
 // Search pieces shared with nlb_api.cpp.
 Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int64_t n,
                         const double* cell9, const uint8_t* pbc, double cutoff, int64_t** ei,
-                        int32_t** sh, int64_t* m);
+                        int32_t** sh, int64_t* m, int flags = 0, nlb_result_ex* ex = nullptr);
 
 namespace {
 

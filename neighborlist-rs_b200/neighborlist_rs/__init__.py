@@ -640,8 +640,7 @@ def build_neighborlists_torch(cell, positions, cutoff, directed=False, vectors=F
     so a consumer on another stream keeps them alive until its work there is
     done, as with torch's own record_stream rule).  directed / vectors /
     distances as in build_neighborlists_ex (adds "vectors" float64 (M, 3) and
-    "distances" float64 (M,); those results are copied out of the library's
-    workspace)."""
+    "distances" float64 (M,))."""
     if directed or vectors or distances:
         return _torch_ex(cell, positions, cutoff, directed, vectors, distances)
     import torch
@@ -699,6 +698,7 @@ _lib.nlb_build_ex.argtypes = [_dp, ctypes.c_int64, ctypes.c_double, _dp, _u8p, c
                               ctypes.POINTER(_ResultEx)]
 _lib.nlb_build_device_ex.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_double, _dp,
                                      _u8p, ctypes.c_int, ctypes.POINTER(_ResultEx)]
+_lib.nlb_build_device_ex_owned.argtypes = _lib.nlb_build_device_ex.argtypes
 _lib.nlb_result_ex_free.argtypes = [ctypes.POINTER(_ResultEx)]
 
 
@@ -758,24 +758,23 @@ def _torch_ex(cell, positions, cutoff, directed, vectors, distances):
         set_stream(stream.cuda_stream)
         try:
             r = _ResultEx()
-            _check(_lib.nlb_build_device_ex(ctypes.c_void_p(pos.data_ptr() if n else 0), n, c, h,
-                                            pb, _ex_flags(directed, vectors, distances),
-                                            ctypes.byref(r)))
-            m = int(r.n_edges)
-            out = {"edge_index": torch.empty((2, m), dtype=torch.int64, device=dev),
-                   "shift": torch.empty((m, 3), dtype=torch.int32, device=dev)}
-            if vectors:
-                out["vectors"] = torch.empty((m, 3), dtype=torch.float64, device=dev)
-            if distances:
-                out["distances"] = torch.empty((m,), dtype=torch.float64, device=dev)
-            if m:
-                s = stream.cuda_stream
-                _cudart_copy(out["edge_index"].data_ptr(), r.edge_index, 16 * m, s)
-                _cudart_copy(out["shift"].data_ptr(), r.shift, 12 * m, s)
-                if vectors:
-                    _cudart_copy(out["vectors"].data_ptr(), r.vectors, 24 * m, s)
-                if distances:
-                    _cudart_copy(out["distances"].data_ptr(), r.distances, 8 * m, s)
+            _check(_lib.nlb_build_device_ex_owned(
+                ctypes.c_void_p(pos.data_ptr() if n else 0), n, c, h, pb,
+                _ex_flags(directed, vectors, distances), ctypes.byref(r)))
         finally:
             set_stream(None)
+        m = int(r.n_edges)
+
+        def block(ptr, shape, dtype, typestr):
+            if m == 0:
+                return torch.zeros(shape, dtype=dtype, device=dev)
+            return torch.as_tensor(_DeviceBlock(ptr, shape, typestr, stream.cuda_stream),
+                                   device=dev)
+
+        out = {"edge_index": block(r.edge_index, (2, m), torch.int64, "<i8"),
+               "shift": block(r.shift, (m, 3), torch.int32, "<i4")}
+        if vectors:
+            out["vectors"] = block(r.vectors, (m, 3), torch.float64, "<f8")
+        if distances:
+            out["distances"] = block(r.distances, (m,), torch.float64, "<f8")
     return out
