@@ -309,9 +309,6 @@ void issue_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t capacity) {
   c.mark(5);
 }
 
-// Waits until the launch just issued has filled the host-mapped report
-// (c.h_report[0] = 1), polling the stream now and then: a stream that failed,
-// or ended without a report, ends the wait with an error.
 Status wait_report(Ctx& c) {
   volatile int64_t* r = c.h_report;
   for (uint32_t k = 1; r[0] == 0; ++k) {

@@ -236,6 +236,10 @@ Status emit_system(Ctx& c, SystemPlan& sp, const double* d_pos, const DevLists& 
 // stream.
 Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
                 bool stream_ordered = false);
+// Waits until the launch just issued on c.stream has filled the host-mapped
+// report (c.h_report[0] = 1), polling the stream now and then: a stream that
+// failed, or ended without a report, ends the wait with an error.
+Status wait_report(Ctx& c);
 // Whether run_fast takes the group search for this system.
 bool takes_group_search(const SystemPlan& sp);
 // Single-system pipeline choice: 0 = the two-launch group search, 1 = the

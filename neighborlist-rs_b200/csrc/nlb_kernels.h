@@ -412,14 +412,27 @@ void launch_edge_extras(const double* pos, const EdgeExtrasCell& cell, const int
 // edges kept at rc, compacted in stored order.
 void launch_max_disp(const double* pos, const double* ref, int64_t n, unsigned long long* out,
                      cudaStream_t s);
-// The kept edges in one pass (k_verlet_compact): out_ei [src | dst] of M
-// edges and out_sh; dst_tmp has room for m destinations; state has
-// verlet_compact_state_words(m) words (cleared here): [1] the look-back's
-// error word, [3] M.
+// The manager's stored edges: atoms, packed shifts, and the plain shifts that
+// are read instead when *wide is set (some shift does not fit 10 bits).
+struct VerletEdges {
+  const int2* ij;
+  const uint32_t* packed;
+  const int32_t* plain;
+  const int32_t* wide;
+  int64_t m;
+};
+void launch_verlet_pack(const int64_t* ei, const int32_t* sh, int64_t m, int2* ij,
+                        uint32_t* packed, int32_t* plain, int32_t* wide, cudaStream_t s);
+// One update (k_verlet_compact): the kept edges, out_ei [src | dst] of M edges
+// and out_sh; dst_tmp has room for list.m destinations; state has
+// verlet_compact_state_words(list.m) words, zero on entry and zero again
+// afterwards.  report (host-mapped): [1] M, [2] the look-back's error word,
+// [3] the bits of the largest squared displacement, then [0] = 1 when all is
+// written.
 int64_t verlet_compact_state_words(int64_t m);
-void launch_verlet_compact(const double* pos, const EdgeExtrasCell& cell, const int64_t* ei,
-                           const int32_t* sh, int64_t m, double rc_sq, int64_t* out_ei,
-                           int32_t* out_sh, int64_t* dst_tmp, uint64_t* state,
-                           int32_t spin_limit, cudaStream_t s);
+void launch_verlet_compact(const double* pos, const double* ref, int64_t n,
+                           const EdgeExtrasCell& cell, const VerletEdges& list, double rc_sq,
+                           int64_t* out_ei, int32_t* out_sh, int32_t* dst_tmp, uint64_t* state,
+                           int32_t spin_limit, int64_t* report, cudaStream_t s);
 
 }  // namespace nlb

@@ -4,14 +4,13 @@
 // r_list = r_cut + r_skin, reference positions, rebuild when
 // max_i |r_i - r_i,ref| > r_skin / 2, update / needs_rebuild / get); the
 // reference does not implement it.  Each update:
-//   1. if a list exists for the same atom count, cell and pbc, one kernel
-//      takes the largest displacement since the last rebuild (one sync);
+//   1. if a list exists for the same atom count, cell and pbc, one launch
+//      takes the largest displacement since the last rebuild and filters the
+//      stored list with the current positions at rc, in stored order;
 //   2. if there is no list, the system changed, or that displacement is
 //      above skin / 2: rebuild -- the exact half list at rc + skin (the same
-//      search as nlb_build), kept in the manager's device buffers, and the
-//      current positions become the reference;
-//   3. filter the stored list with the current positions at rc (keep flags,
-//      one scan, compaction in stored order; one sync for the total).
+//      search as nlb_build), kept packed in the manager's device buffers, and
+//      the current positions become the reference -- and filter it.
 // As long as no atom moved more than skin / 2, every pair now closer than rc
 // was closer than rc + skin at the rebuild, so the filtered list holds
 // exactly the pairs (i, j, S) with |(r_j - r_i) + H.S| < rc -- the set a
@@ -95,23 +94,11 @@ class Verlet {
     ++updates_;
     bool rebuild = !same_system(n, cell9, pbc);
     if (!rebuild && n > 0) {
-      // The displacement check and the filter of the stored list go out
-      // together (the filter only reads the positions and the list) and one
-      // synchronisation reads both; a rebuild, when due, discards the filter.
-      auto* d = static_cast<unsigned long long*>(disp_.get(sizeof(unsigned long long)));
-      if (!d) return fail(NLB_ERR_NOMEM, "device allocation failed");
-      launch_max_disp(d_pos, static_cast<const double*>(ref_.p), n, d, s);
-      cudaError_t e = cudaMemcpyAsync(c->h_small + 2, d, sizeof(unsigned long long),
-                                      cudaMemcpyDeviceToHost, s);
-      if (e != cudaSuccess) return cuda_fail(e, "displacement check");
-      st = filter(*c, d_pos, m_out, ei_out, sh_out, owned);
-      if (!st.ok()) return st;
-      if (m_list_ == 0) {  // (the filter had nothing to do and did not synchronise)
-        e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return cuda_fail(e, "displacement check");
-      }
+      // (one launch takes the displacement and filters the stored list; a
+      // rebuild, when due, discards the filter)
       double d2 = 0.0;
-      std::memcpy(&d2, c->h_small + 2, sizeof(double));
+      st = filter(*c, d_pos, m_out, ei_out, sh_out, owned, &d2);
+      if (!st.ok()) return st;
       last_disp_ = std::sqrt(d2);
       rebuild = last_disp_ > 0.5 * skin_;
       if (!rebuild) return Status{NLB_OK};
@@ -214,16 +201,15 @@ class Verlet {
       Status st = half_list_device(c, pos_host, d_pos, n, cell9, pbc, rc_ + skin_, &ei, &sh, &m);
       if (!st.ok()) return st;
     }
-    int64_t* vei = static_cast<int64_t*>(list_ei_.get(16 * (size_t)m));
-    int32_t* vsh = static_cast<int32_t*>(list_sh_.get(12 * (size_t)m));
+    int2* ij = static_cast<int2*>(list_ij_.get(8 * (size_t)m));
+    uint32_t* packed = static_cast<uint32_t*>(list_packed_.get(4 * (size_t)m));
+    int32_t* plain = static_cast<int32_t*>(list_plain_.get(12 * (size_t)m));
+    int32_t* wide = static_cast<int32_t*>(list_wide_.get(sizeof(int32_t)));
     double* ref = static_cast<double*>(ref_.get(24 * (size_t)n));
-    if (!vei || !vsh || !ref) return fail(NLB_ERR_NOMEM, "device allocation failed");
-    cudaError_t e = cudaSuccess;
-    if (m > 0) {
-      e = cudaMemcpyAsync(vei, ei, 16 * (size_t)m, cudaMemcpyDeviceToDevice, c.stream);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(vsh, sh, 12 * (size_t)m, cudaMemcpyDeviceToDevice, c.stream);
-    }
+    if (!ij || !packed || !plain || !wide || !ref)
+      return fail(NLB_ERR_NOMEM, "device allocation failed");
+    launch_verlet_pack(ei, sh, m, ij, packed, plain, wide, c.stream);
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && n > 0)
       e = cudaMemcpyAsync(ref, d_pos, 24 * (size_t)n, cudaMemcpyDeviceToDevice, c.stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync (Verlet list)");
@@ -241,7 +227,7 @@ class Verlet {
   // owned: the kept edges go to blocks of the result pool sized for the
   // whole stored list, handed to the caller (released again on failure).
   Status filter(Ctx& c, const double* d_pos, int64_t* m_out, int64_t** ei_out,
-                int32_t** sh_out, bool owned = false) {
+                int32_t** sh_out, bool owned = false, double* disp_sq = nullptr) {
     const int64_t m = m_list_;
     int64_t* out_ei = nullptr;
     int32_t* out_sh = nullptr;
@@ -260,9 +246,10 @@ class Verlet {
       out_sh = static_cast<int32_t*>(out_sh_.get(12 * (size_t)m));
       if (!out_ei || !out_sh) return fail(NLB_ERR_NOMEM, "device allocation failed");
     }
-    int64_t* dst_tmp = static_cast<int64_t*>(dst_tmp_.get(8 * (size_t)m));
-    uint64_t* state =
-        static_cast<uint64_t*>(state_.get(8 * (size_t)verlet_compact_state_words(m)));
+    int32_t* dst_tmp = static_cast<int32_t*>(dst_tmp_.get(4 * (size_t)m));
+    const size_t state_bytes = 8 * (size_t)verlet_compact_state_words(m);
+    const size_t state_cap = state_.cap;
+    uint64_t* state = static_cast<uint64_t*>(state_.get(state_bytes));
     if (!dst_tmp || !state) {
       if (owned) {
         release_owned_device(out_ei, c.stream);
@@ -272,7 +259,7 @@ class Verlet {
     }
     *ei_out = out_ei;
     *sh_out = out_sh;
-    if (m == 0) {
+    if (m == 0 && !disp_sq) {
       m_last_ = 0;
       return Status{NLB_OK};
     }
@@ -281,28 +268,38 @@ class Verlet {
       std::memcpy(cell.h, h_, sizeof(h_));
       cell.has_cell = 1;
     }
-    const int64_t* vei = static_cast<const int64_t*>(list_ei_.p);
-    const int32_t* vsh = static_cast<const int32_t*>(list_sh_.p);
-    launch_verlet_compact(d_pos, cell, vei, vsh, m, rc_ * rc_, out_ei, out_sh, dst_tmp, state,
-                          kVerletSpinLimit, c.stream);
-    // M and the look-back's bounded-wait error word
-    cudaError_t e = cudaMemcpyAsync(c.h_small, state + 3, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                    c.stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(c.h_small + 1, state + 1, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                          c.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
-    if (e != cudaSuccess || c.h_small[1] != 0) {
+    VerletEdges list;
+    list.ij = static_cast<const int2*>(list_ij_.p);
+    list.packed = static_cast<const uint32_t*>(list_packed_.p);
+    list.plain = static_cast<const int32_t*>(list_plain_.p);
+    list.wide = static_cast<const int32_t*>(list_wide_.p);
+    list.m = m;
+    // (the launch leaves the state cleared; a new or a failed one is not)
+    if (!state_clean_ || state_.cap != state_cap)
+      cudaMemsetAsync(state, 0, state_.cap, c.stream);
+    state_clean_ = false;
+    c.h_report[0] = 0;
+    launch_verlet_compact(d_pos, static_cast<const double*>(ref_.p), n_, cell, list, rc_ * rc_,
+                          out_ei, out_sh, dst_tmp, state, kVerletSpinLimit, c.d_report, c.stream);
+    // (reported when everything is written: no other synchronisation)
+    Status st = wait_report(c);
+    const volatile int64_t* r = c.h_report;
+    if (!st.ok() || r[2] != 0) {
       if (owned) {
         release_owned_device(out_ei, c.stream);
         release_owned_device(out_sh, c.stream);
         *ei_out = nullptr;
         *sh_out = nullptr;
       }
-      if (e != cudaSuccess) return cuda_fail(e, "Verlet filter");
+      if (!st.ok()) return st;
       return fail(NLB_ERR_CUDA, "prefix scan gave up waiting for a tile");
     }
-    m_last_ = c.h_small[0];
+    state_clean_ = true;
+    if (disp_sq) {
+      const int64_t bits = r[3];
+      std::memcpy(disp_sq, &bits, sizeof(double));
+    }
+    m_last_ = r[1];
     *m_out = m_last_;
     return Status{NLB_OK};
   }
@@ -317,7 +314,9 @@ class Verlet {
   int64_t m_list_ = 0, m_last_ = 0;
   int64_t updates_ = 0, rebuilds_ = 0;
   double last_disp_ = 0.0;
-  DevBuf pos_up_, ref_, disp_, list_ei_, list_sh_, out_ei_, out_sh_, dst_tmp_, state_;
+  bool state_clean_ = false;
+  DevBuf pos_up_, ref_, disp_, list_ij_, list_packed_, list_plain_, list_wide_, out_ei_, out_sh_,
+      dst_tmp_, state_;
 };
 
 }  // namespace nlb
