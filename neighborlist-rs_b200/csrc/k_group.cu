@@ -297,17 +297,17 @@ struct GCountWarp {
 static_assert(sizeof(GCountWarp) % 16 == 0, "vector accesses");
 
 // Takes room for the records of `candidates` candidates (at most one per 32)
-// from a region; *fits: there was room.
+// from a region.
+// Lane 0 gets the first record, or -1 without room; the others 0 (so that
+// nothing waits for the atomic before the first record is stored).
 __device__ __forceinline__ int64_t take_records(const GroupSearch& o, int region,
-                                                int64_t candidates, bool& fits) {
+                                                int64_t candidates) {
   const int64_t room = (candidates + 31) >> 5;
-  int64_t at = 0;
-  if ((threadIdx.x & 31) == 0 && room > 0)
-    at = (int64_t)atomicAdd(&o.chunk_top[16 * region], (unsigned long long)room);
-  at = __shfl_sync(0xffffffffu, at, 0);
+  if (threadIdx.x != 0) return 0;
   const int64_t cap = o.chunk_cap / kGroupRegions;
-  fits = at + room <= cap;
-  return region * cap + at;
+  const int64_t at =
+      room > 0 ? (int64_t)atomicAdd(&o.chunk_top[16 * region], (unsigned long long)room) : 0;
+  return at + room <= cap ? region * cap + at : -1;
 }
 
 // Candidates of the cells [c0, c0 + nc) of a group (segments of more than 32
@@ -341,11 +341,15 @@ __device__ __forceinline__ void finish_group(const GridParams& g, const GridBuff
   if (o.split > 1) {
     run = 0;
     uint32_t* row = o.seg_cnt + (int64_t)t * o.split * 32 + lane;
-#pragma unroll 4
-    for (int s = 0; s < o.split; ++s) {
-      const uint32_t v = __ldcg(&row[32 * s]);
-      row[32 * s] = run;
-      run += v;
+    for (int s0 = 0; s0 < o.split; s0 += 16) {  // (16 loads in flight)
+      uint32_t v[16];
+#pragma unroll
+      for (int s = 0; s < 16; ++s) v[s] = s0 + s < o.split ? __ldcg(&row[32 * (s0 + s)]) : 0u;
+#pragma unroll
+      for (int s = 0; s < 16; ++s) {
+        if (s0 + s < o.split) row[32 * (s0 + s)] = run;
+        run += v[s];
+      }
     }
   }
   for (unsigned m = irr_mask; m; m &= m - 1) {
@@ -458,20 +462,20 @@ __global__ void __launch_bounds__(kGThreads, 28)
   }
   __syncwarp();
   pdl_wait();
-  const int32_t n_groups = b.counters[0];
+  const int32_t split = o.split;
+  const int64_t item = blockIdx.x;
+  const int32_t t = (int32_t)((uint32_t)item / (uint32_t)split);
+  const int32_t seg = (int32_t)(item - (int64_t)t * split);
+  const int32_t c0 = n_cells * seg / split;
+  const int32_t nc = n_cells * (seg + 1) / split - c0;
+  // (loaded together; the record of a group past the last is not used)
+  const int32_t n_groups = b.counters[0], loose = *b.loose;
+  const GroupRec grp = b.groups[t];
+  const int64_t n_items = (int64_t)n_groups * split;
   // (an atom outside its stored bin by more than rounding: certain hits are
   // rechecked too, since the reference may prune their cell)
-  const float near_lo = *b.loose != 0 ? -INFINITY : -band.width;
-  const int32_t split = o.split;
-  const int64_t n_items = (int64_t)n_groups * split;
-
-  const int64_t item = blockIdx.x;
+  const float near_lo = loose != 0 ? -INFINITY : -band.width;
   if (item < n_items) {
-    const int32_t t = (int32_t)((uint32_t)item / (uint32_t)split);
-    const int32_t seg = (int32_t)(item - (int64_t)t * split);
-    const int32_t c0 = n_cells * seg / split;
-    const int32_t nc = n_cells * (seg + 1) / split - c0;
-    const GroupRec grp = b.groups[t];
     const int32_t len = grp.end - grp.first < 32 ? grp.end - grp.first : 32;
     const int32_t p = grp.first + (lane < len ? lane : 0);
     const float4 a = b.p32[p];
@@ -503,12 +507,10 @@ __global__ void __launch_bounds__(kGThreads, 28)
     // kGroupRegions regions (a single cursor would hand out one place every
     // 2 ns).
     const int region = (int)(item % kGroupRegions);
-    int64_t base = 0;  // next free record
-    bool keep_records = true;
+    int64_t taken = 0;  // lane 0: the segment's first record (-1: no room)
 
     uint32_t cnt = 0;  // lane: this atom's hits in the segment
     int32_t fill = 0, head = 0, n_rec = 0;
-    int64_t first_rec = 0;
     const int n_quads = (len + 3) >> 2;
 
     // 3. the oldest v candidates of the ring against the group's atoms
@@ -559,7 +561,8 @@ __global__ void __launch_bounds__(kGThreads, 28)
       const uint32_t h = lane < 4 * n_quads ? mbuf[lane] : 0u;
       if (__any_sync(0xffffffffu, h != 0)) {
         cnt += __popc(h);
-        if (keep_records) {
+        const int64_t base = __shfl_sync(0xffffffffu, taken, 0);
+        if (base >= 0) {
           const int2 id = valid ? ring.id[k] : make_int2(0, 0);
           const uint32_t sh = (uint32_t)id.y;
           const bool shifted = __any_sync(0xffffffffu, sh != 0);
@@ -605,9 +608,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
         start = 0x7fffffff;
       }
       if (cb == 0) {
-        base = take_records(o, region, nc > 32 ? row_candidates(g, b, grp, n_cells, c0, nc) : tot,
-                            keep_records);
-        first_rec = base;
+        taken = take_records(o, region, nc > 32 ? row_candidates(g, b, grp, n_cells, c0, nc) : tot);
       }
       __syncwarp();
 
@@ -657,7 +658,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
       __syncwarp();  // (the cells' records are free again)
     }
 
-    if (lane == 0) o.seg_rec[item] = make_longlong2(first_rec, n_rec);
+    if (lane == 0) o.seg_rec[item] = make_longlong2(taken, n_rec);
     int32_t before = split - 1;
     if (split > 1) {
       // The last segment of the group to be counted finishes it.
@@ -708,17 +709,18 @@ __global__ void __launch_bounds__(kGThreads, 28)
   const int lane = threadIdx.x;
   GEmitWarp& w_sm = *reinterpret_cast<GEmitWarp*>(gsm);
   pdl_wait();
-  const int64_t M = *o.total;
-  if (o.state[1] != 0 || M > out.capacity || *o.records > o.chunk_cap) return;
-  const int64_t d_ei = EX && out.directed ? 2 * M : M;
   const int32_t split = o.split;
-  const int64_t n_items = (int64_t)b.counters[0] * split;
   const int64_t item = blockIdx.x;
-  if (item >= n_items) return;
   const int32_t t = (int32_t)((uint32_t)item / (uint32_t)split);
-  const longlong2 rec = o.seg_rec[item];
   const int32_t seg = (int32_t)(item - (int64_t)t * split);
+  // (loaded together; what belongs to a group past the last is not used)
+  const int64_t M = *o.total, records = *o.records;
+  const uint64_t err = o.state[1];
+  const int32_t n_groups = b.counters[0];
+  const longlong2 rec = o.seg_rec[item];
   const GroupRec grp = b.groups[t];
+  int64_t slot = o.block_base[t / kGroupBlock] + o.atom_base[(int64_t)t * 32 + lane];
+  if (split > 1) slot += o.seg_cnt[item * 32 + lane];  // (the atom's hits in earlier segments)
   // The group's first slot: its block's and the block's groups before it.
   int64_t base = 0;
 #pragma unroll
@@ -726,8 +728,8 @@ __global__ void __launch_bounds__(kGThreads, 28)
     const int32_t u = t / kGroupBlock * kGroupBlock + 32 * k + lane;
     if (u < t) base += o.group_total[u];
   }
-  int64_t slot = o.block_base[t / kGroupBlock] + o.atom_base[(int64_t)t * 32 + lane];
-  if (split > 1) slot += o.seg_cnt[item * 32 + lane];  // (the atom's hits in earlier segments)
+  if (err != 0 || M > out.capacity || records > o.chunk_cap || t >= n_groups) return;
+  const int64_t d_ei = EX && out.directed ? 2 * M : M;
   const int64_t first_rec = rec.x;
   const int n_rec = (int)rec.y;
   const int32_t len = grp.end - grp.first < 32 ? grp.end - grp.first : 32;
