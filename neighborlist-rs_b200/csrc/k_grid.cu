@@ -717,19 +717,10 @@ __global__ void k_chunk_box(const GroupRec* __restrict__ groups,
 
 constexpr int kBoundsThreads = 1024;
 
-__global__ void __launch_bounds__(kBoundsThreads)
-    k_bounds(const double* __restrict__ pos, int64_t n, double* __restrict__ out) {
+// Minima and maxima of the CTA's values (lo, hi per thread) into out[0..5] by
+// the first three threads.
+__device__ __forceinline__ void cta_bounds(double lo[3], double hi[3], double* out) {
   __shared__ double red[6][kBoundsThreads / 32];
-  double lo[3] = {INFINITY, INFINITY, INFINITY};
-  double hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double v = pos[3 * i + a];
-      if (v < lo[a]) lo[a] = v;
-      if (v > hi[a]) hi[a] = v;
-    }
-  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -754,6 +745,72 @@ __global__ void __launch_bounds__(kBoundsThreads)
     out[threadIdx.x] = l;
     out[3 + threadIdx.x] = h;
   }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void share_bounds(const double* __restrict__ pos, int64_t n,
+                                             double lo[3], double hi[3]) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = INFINITY;
+    hi[a] = -INFINITY;
+  }
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double v = pos[3 * i + a];
+      if (v < lo[a]) lo[a] = v;
+      if (v > hi[a]) hi[a] = v;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kBoundsThreads)
+    k_bounds(const double* __restrict__ pos, int64_t n, double* __restrict__ out) {
+  double lo[3], hi[3];
+  share_bounds(pos, n, lo, hi);
+  cta_bounds(lo, hi, out);
+}
+
+// Bounds by several CTAs: each leaves its own in part[blockIdx], the last one
+// to end reduces them and reports.  One CTA alone reads about 100 GB/s (240
+// us for a million atoms).
+constexpr int kBoundsCtas = 256;
+struct BoundsTmp {
+  double part[kBoundsCtas][6];
+  int32_t done;
+};
+__global__ void __launch_bounds__(kBoundsThreads)
+    k_bounds_report(const double* __restrict__ pos, int64_t n, BoundsTmp* tmp, int64_t* report) {
+  __shared__ int32_t s_last;
+  __shared__ double s_out[6];
+  double lo[3], hi[3];
+  share_bounds(pos, n, lo, hi);
+  cta_bounds(lo, hi, gridDim.x == 1 ? s_out : tmp->part[blockIdx.x]);
+  if (gridDim.x > 1) {
+    if (threadIdx.x == 0) {
+      __threadfence();
+      s_last = atomicAdd(&tmp->done, 1) == (int32_t)gridDim.x - 1;
+      __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const bool on = threadIdx.x < gridDim.x;
+      lo[a] = on ? __ldcg(&tmp->part[threadIdx.x][a]) : INFINITY;
+      hi[a] = on ? __ldcg(&tmp->part[threadIdx.x][3 + a]) : -INFINITY;
+    }
+    cta_bounds(lo, hi, s_out);
+    if (threadIdx.x == 0) tmp->done = 0;
+  }
+  if (threadIdx.x == 0) {
+    volatile int64_t* r = report;
+    for (int a = 0; a < 6; ++a) r[1 + a] = __double_as_longlong(s_out[a]);
+    __threadfence_system();
+    r[0] = 1;
+  }
 }
 
 // Atoms from which the placement takes one thread per atom (a million atoms:
@@ -768,6 +825,16 @@ int64_t bin_scan_words(int64_t total_bins) { return 2 + (total_bins + kBinTile -
 
 void launch_bounds(const double* pos, int64_t n, double* out, cudaStream_t s) {
   k_bounds<<<1, kBoundsThreads, 0, s>>>(pos, n, out);
+  note_launches(1);
+}
+
+size_t bounds_tmp_bytes() { return sizeof(BoundsTmp); }
+
+void launch_bounds_report(const double* pos, int64_t n, void* tmp, int64_t* report,
+                          cudaStream_t s) {
+  const int64_t want = (n + 4 * kBoundsThreads - 1) / (4 * kBoundsThreads);
+  const unsigned grid = (unsigned)(want < 1 ? 1 : (want < kBoundsCtas ? want : kBoundsCtas));
+  k_bounds_report<<<grid, kBoundsThreads, 0, s>>>(pos, n, static_cast<BoundsTmp*>(tmp), report);
   note_launches(1);
 }
 

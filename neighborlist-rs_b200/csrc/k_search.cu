@@ -202,6 +202,133 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   visit_brute_atom(bp, pos, n, i, cs.max_sq, sink);
 }
 
+// ---- brute force of one small system, one cutoff, in two launches
+//
+// Count: a warp per atom tests j > i in index order, 32 at a time, and keeps
+// each step's hits as one mask word (lane w keeps step w: at most 32 steps);
+// the last CTA turns the atoms' counts into offsets, and M goes to the host.
+// Emit: a warp per atom expands its words; only the hits' shifts are computed
+// again.  Bound by latency at these sizes: 500 atoms, minimum image, took 80
+// us with count, scan, copies and a synchronisation for M, and an emit pass
+// that tested every pair again (12 + 5 + 17 us of kernels).
+
+// Squared distance and minimum-image shift of the pair (src/search.rs:1187-1405).
+__device__ __forceinline__ double brute_pair(const BruteParams& bp, double xi, double yi,
+                                             double zi, double xj, double yj, double zj,
+                                             int32_t s[3]) {
+  if (bp.mode == kBruteRaw) {
+    s[0] = s[1] = s[2] = 0;
+    return norm2(dsub(xj, xi), dsub(yj, yi), dsub(zj, zi));
+  }
+  double df[3], sf[3], hv[3];
+  matvec(bp.hinv, dsub(xj, xi), dsub(yj, yi), dsub(zj, zi), df);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    sf[a] = bp.pbc[a] ? -round(df[a]) : 0.0;
+    s[a] = sat_i32(sf[a]);
+  }
+  matvec(bp.h, sf[0], sf[1], sf[2], hv);
+  return norm2(dsub(dadd(xj, hv[0]), xi), dsub(dadd(yj, hv[1]), yi), dsub(dadd(zj, hv[2]), zi));
+}
+
+constexpr int kBruteWarps = 4;
+
+__global__ void __launch_bounds__(kBruteWarps * 32)
+    k_brute_masks(const __grid_constant__ BruteParams bp, const double* __restrict__ pos,
+                  int32_t n, double rc_sq, BruteRows rows, int64_t* report) {
+  __shared__ int64_t warp_sum[kBruteWarps];
+  __shared__ int32_t s_last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int32_t i = (int32_t)blockIdx.x * kBruteWarps + warp;
+  if (i < n) {
+    const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
+    uint32_t word = 0;
+    for (int32_t jb = i + 1, w = 0; jb < n; jb += 32, ++w) {
+      const int32_t j = jb + lane;
+      bool hit = false;
+      if (j < n) {
+        int32_t s[3];
+        hit = brute_pair(bp, xi, yi, zi, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], s) < rc_sq;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (lane == w) word = m;
+    }
+    rows.masks[32 * i + lane] = word;
+    const int cnt = __reduce_add_sync(0xffffffffu, __popc(word));
+    if (lane == 0) rows.counts[i] = cnt;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(rows.done, 1) == (int32_t)gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  const int32_t per = (n + kBruteWarps * 32 - 1) / (kBruteWarps * 32);
+  const int32_t a0 = min(tid * per, n), a1 = min(a0 + per, n);
+  int64_t sum = 0;
+#pragma unroll 4
+  for (int32_t k = a0; k < a1; ++k) sum += __ldcg(&rows.counts[k]);
+  int64_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sum[warp] = x;
+  __syncthreads();
+  int64_t run = x - sum, M = 0;
+  for (int w = 0; w < kBruteWarps; ++w) {
+    run += w < warp ? warp_sum[w] : 0;
+    M += warp_sum[w];
+  }
+  for (int32_t k = a0; k < a1; ++k) {
+    rows.offs[k] = run;
+    run += __ldcg(&rows.counts[k]);
+  }
+  if (tid == 0) {
+    rows.offs[n] = M;
+    *rows.done = 0;  // (for the next launch)
+    volatile int64_t* r = report;
+    r[1] = M;
+    r[2] = 0;
+    __threadfence_system();
+    r[0] = 1;
+  }
+}
+
+__global__ void __launch_bounds__(kBruteWarps * 32)
+    k_brute_write(const __grid_constant__ BruteParams bp, const double* __restrict__ pos,
+                  int32_t n, BruteRows rows, int64_t* __restrict__ src, int32_t* __restrict__ sh,
+                  int64_t capacity) {
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int32_t i = (int32_t)blockIdx.x * kBruteWarps + (threadIdx.x >> 5);
+  if (i >= n) return;
+  const int64_t M = rows.offs[n];
+  int64_t e0 = rows.offs[i];
+  const uint32_t word = rows.masks[32 * i + lane];
+  if (M > capacity) return;  // the caller grows the arrays and writes again
+  const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
+  for (unsigned some = __ballot_sync(0xffffffffu, word != 0); some; some &= some - 1) {
+    const int w = __ffs(some) - 1;
+    const unsigned m = __shfl_sync(0xffffffffu, word, w);
+    if ((m >> lane) & 1u) {
+      const int32_t j = i + 1 + 32 * w + lane;
+      int32_t s[3];
+      brute_pair(bp, xi, yi, zi, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], s);
+      const int64_t e = e0 + __popc(m & lanemask_lt());
+      src[e] = i;
+      src[M + e] = j;
+      sh[3 * e] = s[0];
+      sh[3 * e + 1] = s[1];
+      sh[3 * e + 2] = s[2];
+    }
+    e0 += __popc(m);
+  }
+}
+
 inline unsigned blocks_for(int64_t n) {
   return (unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock);
 }
@@ -229,6 +356,20 @@ void launch_brute_count(const BruteParams& bp, const double* pos, int64_t n, con
 void launch_brute_emit(const BruteParams& bp, const double* pos, int64_t n, const CutoffSet& cs,
                        const int64_t* offs, const EmitTargets& t, cudaStream_t s) {
   k_brute_emit<<<blocks_for(n), kWarpsPerBlock * 32, 0, s>>>(bp, pos, n, cs, offs, t);
+  note_launches(1);
+}
+
+void launch_brute_masks(const BruteParams& bp, const double* pos, int32_t n, double rc_sq,
+                        const BruteRows& rows, int64_t* report, cudaStream_t s) {
+  k_brute_masks<<<(unsigned)((n + kBruteWarps - 1) / kBruteWarps), kBruteWarps * 32, 0, s>>>(
+      bp, pos, n, rc_sq, rows, report);
+  note_launches(1);
+}
+
+void launch_brute_write(const BruteParams& bp, const double* pos, int32_t n, const BruteRows& rows,
+                        int64_t* src, int32_t* sh, int64_t capacity, cudaStream_t s) {
+  launch_pdl(k_brute_write, dim3((unsigned)((n + kBruteWarps - 1) / kBruteWarps)),
+             dim3(kBruteWarps * 32), 0, s, bp, pos, n, rows, src, sh, capacity);
   note_launches(1);
 }
 

@@ -919,11 +919,12 @@ Status run_single(const double* pos, int64_t n, const double* cell9, const uint8
   double* d_pos = nullptr;
   st = upload_positions(*c, pos, n, &d_pos);
   if (!st.ok()) return st;
-  if (fast_eligible(sp)) {
+  if (fast_eligible(sp) || brute_rows_eligible(sp)) {
     int64_t m = 0;
     // (the copies follow the search on the stream, so the call goes on as
     // soon as M is known)
-    st = run_fast(*c, sp, d_pos, &m, true);
+    st = fast_eligible(sp) ? run_fast(*c, sp, d_pos, &m, true)
+                           : run_brute_rows(*c, sp, d_pos, &m, true);
     if (!st.ok()) return st;
     DevLists L;
     L.src.assign(1, sp.out_src);
@@ -957,12 +958,8 @@ Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int
   double bounds[6];
   const double* bptr = nullptr;
   if (!cell9 && !pos_host) {
-    double* d_b = static_cast<double*>(c.raw(kSlotBatch0 + 31, sizeof(double) * 6));
-    if (!d_b) return fail(NLB_ERR_NOMEM, "device allocation failed");
-    launch_bounds(d_pos, n, d_b, c.stream);
-    cudaError_t e = cudaMemcpyAsync(bounds, d_b, sizeof(bounds), cudaMemcpyDeviceToHost, c.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
-    if (e != cudaSuccess) return cuda_fail(e, "bounds");
+    Status bs = device_bounds(c, d_pos, n, bounds);
+    if (!bs.ok()) return bs;
     bptr = bounds;
   }
   const bool pb[3] = {pbc ? pbc[0] != 0 : true, pbc ? pbc[1] != 0 : true,
@@ -991,6 +988,13 @@ Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int
       ex->vectors = sp.out_vec;
       ex->distances = sp.out_dist;
     }
+    return Status{NLB_OK};
+  }
+  if (brute_rows_eligible(sp)) {
+    st = run_brute_rows(c, sp, d_pos, m);
+    if (!st.ok()) return st;
+    *ei = sp.out_src;
+    *sh = sp.out_sh;
     return Status{NLB_OK};
   }
   st = count_system(c, sp, d_pos);
@@ -1152,12 +1156,8 @@ Status run_single_device(const double* d_pos, int64_t n, const double* cell9, co
   double bounds[6];
   const double* bptr = nullptr;
   if (!cell9) {
-    double* d_b = static_cast<double*>(c->raw(kSlotBatch0 + 31, sizeof(double) * 6));
-    if (!d_b) return fail(NLB_ERR_NOMEM, "device allocation failed");
-    launch_bounds(d_pos, n, d_b, c->stream);
-    cudaError_t e = cudaMemcpyAsync(bounds, d_b, sizeof(bounds), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "bounds");
+    st = device_bounds(*c, d_pos, n, bounds);
+    if (!st.ok()) return st;
     bptr = bounds;
   }
   const bool pb[3] = {pbc ? pbc[0] != 0 : true, pbc ? pbc[1] != 0 : true,
@@ -1166,9 +1166,9 @@ Status run_single_device(const double* d_pos, int64_t n, const double* cell9, co
   std::vector<double> cs(1, cutoff);
   st = plan_system(nullptr, n, cell9, pb, cs, false, false, sp, bptr);
   if (!st.ok()) return st;
-  if (fast_eligible(sp)) {
+  if (fast_eligible(sp) || brute_rows_eligible(sp)) {
     int64_t m = 0;
-    st = run_fast(*c, sp, d_pos, &m);
+    st = fast_eligible(sp) ? run_fast(*c, sp, d_pos, &m) : run_brute_rows(*c, sp, d_pos, &m);
     if (!st.ok()) return st;
     out->n_edges = m;
     out->edge_index = sp.out_src;

@@ -558,4 +558,79 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   return Status{NLB_OK};
 }
 
+Status run_brute_rows(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
+                      bool stream_ordered) {
+  FastState& fs = state_for(c);
+  const int64_t n = sp.n;
+  int32_t tile = 0, spins = 0;
+  take_scan_stall(&tile, &spins);  // (no launch here waits for another)
+  int64_t capacity = std::max<int64_t>(
+      {4096, (int64_t)(1.25 * (double)fs.last_m),
+       (int64_t)(1.5 * (double)estimate_edges(sp, std::sqrt(sp.rc_sq[0])))});
+  capacity = std::min(capacity, n * (n - 1) / 2 + 1);
+  BruteRows rows;
+  rows.masks = slot<uint32_t>(c, kSlotBruteMasks, 32 * (size_t)kBruteRowAtoms);
+  // (offsets, counts and the completion count, which every launch leaves at
+  // zero)
+  const bool fresh = c.bufs[kSlotBruteRows].p == nullptr;
+  rows.offs = slot<int64_t>(c, kSlotBruteRows, 2 * (size_t)kBruteRowAtoms + 2);
+  if (!rows.masks || !rows.offs || !out_arrays(c, sp, capacity))
+    return fail(NLB_ERR_NOMEM, "device allocation failed");
+  rows.counts = reinterpret_cast<int32_t*>(rows.offs + kBruteRowAtoms + 1);
+  rows.done = rows.counts + kBruteRowAtoms;
+  if (fresh) cudaMemsetAsync(rows.done, 0, sizeof(int32_t), c.stream);
+  c.h_report[0] = 0;
+  c.mark(0);
+  c.mark(1);
+  launch_brute_masks(sp.brute, d_pos, (int32_t)n, sp.rc_sq[0], rows, c.d_report, c.stream);
+  c.mark(2);
+  c.mark(3);
+  c.mark(4);
+  launch_brute_write(sp.brute, d_pos, (int32_t)n, rows, sp.out_src, sp.out_sh, capacity, c.stream);
+  c.mark(5);
+  Status st = wait_report(c);
+  if (!st.ok()) return st;
+  const int64_t m = const_cast<volatile int64_t*>(c.h_report)[1];
+  fs.have_key = false;  // (the result arrays are not the ones of the last search)
+  if (m > capacity) {
+    if (!out_arrays(c, sp, m))
+      return fail(NLB_ERR_NOMEM, "device allocation for the edge lists failed");
+    launch_brute_write(sp.brute, d_pos, (int32_t)n, rows, sp.out_src, sp.out_sh, m, c.stream);
+  }
+  if (c.stream == c.own_stream || c.prof) {
+    if (!stream_ordered || c.prof) {
+      const cudaError_t e = cudaStreamSynchronize(c.stream);
+      if (e != cudaSuccess) return cuda_fail(e, "brute force");
+    }
+  } else {
+    const cudaError_t e = cudaEventRecord(c.early_ev, c.stream);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
+    c.early_stream = c.stream;
+  }
+  if (c.prof) {
+    c.prof_pending_count = true;
+    c.prof_pending_emit = true;
+    c.harvest();
+  }
+  fs.last_m = m;
+  *m_out = m;
+  return Status{NLB_OK};
+}
+
+Status device_bounds(Ctx& c, const double* d_pos, int64_t n, double bounds6[6]) {
+  const bool fresh = c.bufs[kSlotBounds].p == nullptr;
+  void* tmp = c.raw(kSlotBounds, bounds_tmp_bytes());
+  if (!tmp) return fail(NLB_ERR_NOMEM, "device allocation failed");
+  if (fresh) cudaMemsetAsync(tmp, 0, bounds_tmp_bytes(), c.stream);
+  c.h_report[0] = 0;
+  launch_bounds_report(d_pos, n, tmp, c.d_report, c.stream);
+  Status st = wait_report(c);
+  if (!st.ok()) return st;
+  for (int a = 0; a < 6; ++a) {
+    const int64_t bits = const_cast<volatile int64_t*>(c.h_report)[1 + a];
+    std::memcpy(&bounds6[a], &bits, sizeof(double));
+  }
+  return Status{NLB_OK};
+}
+
 }  // namespace nlb

@@ -61,6 +61,9 @@ enum Slot : int {
   kSlotAtomBase,
   kSlotSegCnt,
   kSlotSegRec,
+  kSlotBruteMasks,
+  kSlotBruteRows,
+  kSlotBounds,
   kSlotOutVec,
   kSlotOutDist,
   kSlotFill,
@@ -236,6 +239,16 @@ Status emit_system(Ctx& c, SystemPlan& sp, const double* d_pos, const DevLists& 
 // stream.
 Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
                 bool stream_ordered = false);
+// Brute-force systems of at most kBruteRowAtoms atoms, one cutoff: the list
+// in sp.out_src ([src | dst]) and sp.out_sh, returning like run_fast.
+Status run_brute_rows(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
+                      bool stream_ordered = false);
+inline bool brute_rows_eligible(const SystemPlan& sp) {
+  return sp.method != Method::kCellList && sp.rc_sq.size() == 1 && sp.n <= kBruteRowAtoms;
+}
+// Per-axis minima and maxima of device positions, read back through the
+// host-mapped report.
+Status device_bounds(Ctx& c, const double* d_pos, int64_t n, double bounds6[6]);
 // Waits until the launch just issued on c.stream has filled the host-mapped
 // report (c.h_report[0] = 1), polling the stream now and then: a stream that
 // failed, or ended without a report, ends the wait with an error.

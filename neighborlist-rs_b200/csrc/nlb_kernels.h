@@ -307,6 +307,21 @@ void launch_brute_count(const BruteParams& bp, const double* pos, int64_t n, con
 void launch_brute_emit(const BruteParams& bp, const double* pos, int64_t n, const CutoffSet& cs,
                        const int64_t* offs, const EmitTargets& t, cudaStream_t s);
 
+// Brute force of one system of at most kBruteRowAtoms atoms, one cutoff.
+constexpr int64_t kBruteRowAtoms = 1024;  // 32 mask words an atom
+struct BruteRows {
+  uint32_t* masks;  // [32 n] hits of atom i among i + 1 + 32 w + lane
+  int32_t* counts;  // [n]
+  int64_t* offs;    // [n + 1] first slot of each atom; M
+  int32_t* done;    // zero on entry, and again afterwards
+};
+// report (host-mapped): [1] M, [2] 0, then [0] = 1.
+void launch_brute_masks(const BruteParams& bp, const double* pos, int32_t n, double rc_sq,
+                        const BruteRows& rows, int64_t* report, cudaStream_t s);
+// The list [src | dst] with dst = src + M; nothing when M > capacity.
+void launch_brute_write(const BruteParams& bp, const double* pos, int32_t n, const BruteRows& rows,
+                        int64_t* src, int32_t* sh, int64_t capacity, cudaStream_t s);
+
 // ---- k_batch.cu : many small systems per launch (one CTA per system)
 constexpr int kBatchMaxAtoms = 2048;  // larger systems take the single-system pipeline
 
@@ -399,6 +414,12 @@ void note_launches(int n);
 // out[0..2] = min, out[3..5] = max (NaN coordinates are ignored, like the
 // reference's `<` / `>` scan starting from +/-inf).
 void launch_bounds(const double* pos, int64_t n, double* out, cudaStream_t s);
+// The same over several CTAs (tmp: bounds_tmp_bytes(), zero before the first
+// launch, left zero where it has to be), to the host-mapped report: [1..6] the
+// six values, then [0] = 1.
+size_t bounds_tmp_bytes();
+void launch_bounds_report(const double* pos, int64_t n, void* tmp, int64_t* report,
+                          cudaStream_t s);
 
 // Output options on a device half list ([src | dst] ei, shifts sh, m edges):
 // directed list, displacement vectors, distances (k_extras.cu).  Outputs
