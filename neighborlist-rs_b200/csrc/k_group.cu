@@ -3,9 +3,10 @@
 // writes the list from them.
 //
 // A group is a run of at most 32 atoms of one bin (canonical order: bins in
-// rank order, runs in slot order); its stencil cells, in order, are split
-// into segments of consecutive cells.  A segment is one warp's work in both
-// passes; warps share nothing, so the slowest segment holds up nobody.
+// rank order, runs in slot order); the row of its candidates -- its stencil
+// cells' atoms, cell after cell -- is split into segments (slices of the row,
+// or runs of cells when there are more than 32).  A segment is one warp's work
+// in both passes; warps share nothing, so the slowest segment holds up nobody.
 //
 // k_group_count, per segment:
 //   1. one lane per stencil cell describes it (candidates, image shift, FP32
@@ -466,8 +467,10 @@ __global__ void __launch_bounds__(kGThreads, 28)
   const int64_t item = blockIdx.x;
   const int32_t t = (int32_t)((uint32_t)item / (uint32_t)split);
   const int32_t seg = (int32_t)(item - (int64_t)t * split);
-  const int32_t c0 = n_cells * seg / split;
-  const int32_t nc = n_cells * (seg + 1) / split - c0;
+  // (up to 32 cells: a segment is a slice of the row of all their candidates)
+  const bool slices = n_cells <= 32;
+  const int32_t c0 = slices ? 0 : n_cells * seg / split;
+  const int32_t nc = slices ? n_cells : n_cells * (seg + 1) / split - c0;
   // (loaded together; the record of a group past the last is not used)
   const int32_t n_groups = b.counters[0], loose = *b.loose;
   const GroupRec grp = b.groups[t];
@@ -596,8 +599,14 @@ __global__ void __launch_bounds__(kGThreads, 28)
         const int32_t y = __shfl_up_sync(0xffffffffu, start, s);
         if (lane >= s) start += y;
       }
-      const int32_t tot = __shfl_sync(0xffffffffu, start, 31);
+      int32_t tot = __shfl_sync(0xffffffffu, start, 31);
       start -= k;
+      int32_t f_begin = 0;
+      if (slices && split > 1) {  // (about equal slices; the last one to the end)
+        const int32_t per = tot / split, more = tot - per * split;
+        f_begin = per * seg + min(seg, more);
+        tot = f_begin + per + (seg < more ? 1 : 0);
+      }
       const unsigned some = __ballot_sync(0xffffffffu, k > 0);
       if (k > 0) {
         const int at = __popc(some & lanemask_lt());
@@ -608,14 +617,17 @@ __global__ void __launch_bounds__(kGThreads, 28)
         start = 0x7fffffff;
       }
       if (cb == 0) {
-        taken = take_records(o, region, nc > 32 ? row_candidates(g, b, grp, n_cells, c0, nc) : tot);
+        taken = take_records(
+            o, region, nc > 32 ? row_candidates(g, b, grp, n_cells, c0, nc) : tot - f_begin);
       }
       __syncwarp();
 
       // 2. the row's candidates, 32 at a time, through the ring (the next 32
       // are loaded before these are tested)
       float4 q = make_float4(0.f, 0.f, 0.f, 0.f), tc = q;
-      int32_t j = 0, before = -1;
+      int32_t j = 0;
+      // (cells that start before the slice)
+      int32_t before = __popc(__ballot_sync(0xffffffffu, start < f_begin)) - 1;
       uint32_t csh = 0;
       auto fetch = [&](int32_t f0) {
         // cells that start in this window, at their place in it
@@ -630,9 +642,9 @@ __global__ void __launch_bounds__(kGThreads, 28)
           q = b.p32[j];
         }
       };
-      if (tot > 0) fetch(0);
+      if (f_begin < tot) fetch(f_begin);
       const bool last = cb + 32 >= nc;
-      for (int32_t f0 = 0;; f0 += 32) {
+      for (int32_t f0 = f_begin;; f0 += 32) {
         const float cx = q.x + tc.x, cy = q.y + tc.y, cz = q.z + tc.z;
         const int32_t jo = __float_as_int(q.w) + (csh != 0 ? 1 : 0);
         const int2 id = make_int2(j, (int32_t)csh);
@@ -686,9 +698,9 @@ struct GEmitWarp {
   int2 cand[32 * kGWindow];      // and candidates {wrap + image shift (packed), original index}
   SlotMeta meta[32];             // the group's atoms
   int64_t slot[32];              // atom's next output slot minus its place in the stage
-  uint16_t hits[kGStage];        // atom << 9 | candidate of the window, in output order
+  uint16_t hits[kGStage];        // atom << 10 | candidate of the window, in output order
 };
-static_assert(sizeof(GEmitWarp) % 16 == 0 && 32 * kGWindow <= 512, "vector accesses, 9-bit entries");
+static_assert(sizeof(GEmitWarp) % 16 == 0 && 32 * kGWindow <= 1024, "vector accesses, 10-bit entries");
 
 __device__ __forceinline__ void copy16(void* smem, const void* global) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
@@ -783,7 +795,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
     slot += mine;
     for (int c = 0; c < n_win; ++c) {
       uint32_t h = w_sm.mask[32 * c + lane];
-      const uint32_t entry = (uint32_t)lane << 9 | (uint32_t)c << 5;
+      const uint32_t entry = (uint32_t)lane << 10 | (uint32_t)c << 5;
       while (h) {
         w_sm.hits[pre++] = (uint16_t)(entry | (uint32_t)(__ffs(h) - 1));
         h &= h - 1;
@@ -793,14 +805,14 @@ __global__ void __launch_bounds__(kGThreads, 28)
 #pragma unroll 2
     for (int k = lane; k < total; k += 32) {
       const uint32_t v = w_sm.hits[k];
-      const int2 cj = w_sm.cand[v & 511u];
-      const SlotMeta ml = w_sm.meta[v >> 9];
-      const int64_t e = w_sm.slot[v >> 9] + k;
+      const int2 cj = w_sm.cand[v & 1023u];
+      const SlotMeta ml = w_sm.meta[v >> 10];
+      const int64_t e = w_sm.slot[v >> 10] + k;
       int32_t s0 = unpack_shift((uint32_t)cj.x, 0), s1 = unpack_shift((uint32_t)cj.x, 1),
               s2 = unpack_shift((uint32_t)cj.x, 2);
       if (wide) {
-        const uint32_t w = o.cand[at + (v & 511u)];
-        const uint32_t csh = w >> 31 ? o.cshift[at + (v & 511u)] : 0u;
+        const uint32_t w = o.cand[at + (v & 1023u)];
+        const uint32_t csh = w >> 31 ? o.cshift[at + (v & 1023u)] : 0u;
         const SlotMeta mj = b.meta[w & 0x7fffffffu];
         s0 = mj.sx + unpack_shift(csh, 0);
         s1 = mj.sy + unpack_shift(csh, 1);

@@ -226,18 +226,29 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   return Status{NLB_OK};
 }
 
-// Segments per group.  Grids with large bins (every group tests hundreds of
-// atoms in most cells, none in others): one per stencil cell.  Others: as many
-// as give the chip one round of warps (28 per SM): fewer leave warps idle
-// (10,008 atoms at rc 6: 90 us with two per group, 82 with six to nine), more
-// pay for describing cells twice (88 us with twelve).
+// Segments per group: slices of the row of its candidates (stencils of up to
+// 32 cells), or runs of stencil cells.
+//   * As many as give the chip one round of warps (28 per SM): fewer leave
+//     warps idle (10,008 atoms at rc 6: 90 us with two per group, 75 with six
+//     to nine), more describe the cells again (81 us with twelve); slices of
+//     at least 24 candidates (1000 isolated atoms: 70 us with 16 to 24, 78
+//     with 64; a cell of 60 atoms: 58 with 16, 57 with 24 to 32).
+//   * Large bins (above kSplitDense atoms): slices of about 192 candidates, up
+//     to 18,000 segments.  A slice near the group is all hits, and a warp with
+//     a whole cell of them was the last to end by far (10,008 atoms at rc 14:
+//     198 us with one segment per cell, 190 with slices of 192, 202 with 96;
+//     30,000 atoms at rc 14: 508 us per cell, 450 with slices of 192, 426 with
+//     384).
 constexpr double kSplitDense = 64.0;
-constexpr int64_t kSplitTarget = 5000;
+constexpr int64_t kSplitTarget = 5000, kSplitDenseTarget = 18000;
+constexpr int64_t kSplitLeast = 24, kSplitSlice = 192;
 int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
   const int64_t groups = n / 32 + std::min<int64_t>(n, nb) + 1;  // (at most)
-  const int64_t want = (double)n > kSplitDense * (double)nb
-                           ? std::min<int64_t>(cells, ((int64_t)1 << 30) / groups)
-                           : std::min<int64_t>(kSplitTarget / groups, cells);
+  const int64_t row = (int64_t)((double)cells * (double)n / (double)nb);  // candidates of a group
+  int64_t want = kSplitTarget / groups;
+  if ((double)n > kSplitDense * (double)nb)
+    want = std::max(want, std::min(row / kSplitSlice, kSplitDenseTarget / groups));
+  want = std::min({want, cells <= 32 ? row / kSplitLeast : cells, ((int64_t)1 << 30) / groups});
   return (int32_t)std::max<int64_t>(want, 1);
 }
 

@@ -243,7 +243,7 @@ struct GroupSearch {
   uint32_t* seg_cnt;    // [32 max_groups split] hits of each atom in the segments before
   longlong2* seg_rec;   // [max_groups split] {first record, records}
   int64_t max_groups;
-  int32_t split;        // segments per group (at most the stencil cells)
+  int32_t split;        // segments per group
   int32_t spin_limit;   // polls of one wait for a block's groups before it gives up
   int32_t withhold;     // failure-detection hook: this group never joins its block (-1: none)
 };
