@@ -433,7 +433,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
     } else {
       cudaGetLastError();
     }
-  } else if (same && c.stream != nullptr && !c.prof) {
+  } else if (same && c.stream != nullptr && c.stream != cudaStreamLegacy && !c.prof) {
     // (Profiling runs stay outside graphs: its per-phase events are timed on
     // directly launched kernels.)
     // Second identical call: capture the sequence once and replay it.

@@ -545,7 +545,8 @@ class Server {
     if (!st.ok()) return st;
     if (fast_eligible(sp)) {
       int64_t m = 0;
-      st = run_fast(*c, sp, d_pos, &m);
+      // (the result copies follow on the stream; one synchronisation after them)
+      st = run_fast(*c, sp, d_pos, &m, true);
       if (!st.ok()) return st;
       st = deliver(*c, r, sp.out_src, sp.out_sh, m);
     } else {

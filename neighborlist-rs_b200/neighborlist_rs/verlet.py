@@ -21,7 +21,7 @@ from __future__ import annotations
 import ctypes
 
 from . import (_DeviceBlock, _DevResult, _Result, _cell_args, _check, _check_cutoff, _dp, _lib,
-               _positions, _to_dict, _u8p)
+               _on_stream_of, _positions, _to_dict, _u8p)
 
 _lib.nlb_verlet_create.argtypes = [ctypes.c_double, ctypes.c_double]
 _lib.nlb_verlet_create.restype = ctypes.c_void_p
@@ -79,33 +79,26 @@ class VerletList:
         if _is_cuda_tensor(positions):
             import torch
 
-            from . import set_stream
-
             if positions.dtype != torch.float64 or positions.dim() != 2:
                 raise TypeError("positions must be a CUDA float64 tensor of shape (N, 3)")
             if positions.shape[1] != 3:
                 raise ValueError("Positions must be (N, 3)")
             pos = positions.contiguous()
             dev = pos.device
-            with torch.cuda.device(dev):
-                stream = torch.cuda.current_stream(dev)
-                set_stream(stream.cuda_stream)
-                try:
-                    r = _DevResult()
-                    _check(_lib.nlb_verlet_update_device_owned(
-                        self._handle(), ctypes.c_void_p(pos.data_ptr()), pos.shape[0], h, pb,
-                        ctypes.byref(flag), ctypes.byref(r)))
-                finally:
-                    set_stream(None)
+            with _on_stream_of(pos) as stream:
+                r = _DevResult()
+                _check(_lib.nlb_verlet_update_device_owned(
+                    self._handle(), pos.data_ptr(), pos.shape[0], h, pb, ctypes.byref(flag),
+                    ctypes.byref(r)))
                 m = int(r.n_edges)
                 if m == 0:
                     ei = torch.zeros((2, 0), dtype=torch.int64, device=dev)
                     sh = torch.zeros((0, 3), dtype=torch.int32, device=dev)
                 else:
-                    ei = torch.as_tensor(_DeviceBlock(r.edge_index, (2, m), "<i8",
-                                                      stream.cuda_stream), device=dev)
-                    sh = torch.as_tensor(_DeviceBlock(r.shift, (m, 3), "<i4",
-                                                      stream.cuda_stream), device=dev)
+                    ei = torch.as_tensor(_DeviceBlock(r.edge_index, (2, m), "<i8", stream),
+                                         device=dev)
+                    sh = torch.as_tensor(_DeviceBlock(r.shift, (m, 3), "<i4", stream),
+                                         device=dev)
             self.rebuilt = bool(flag.value)
             return {"edge_index": ei, "shift": sh}
         pos = _positions(positions)
