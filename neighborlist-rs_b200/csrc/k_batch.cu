@@ -534,10 +534,12 @@ __device__ __forceinline__ void system_cutoff(const CutoffSet& cs, const SysPlan
   out.disjoint = 0;
 }
 
-// Record sink of the single-cutoff count pass: besides the count, every
-// candidate step of the atom with at least one hit becomes a record {hit
-// mask, first candidate, the cell's image shift in three signed 10-bit
-// fields}.  Lane l buffers the atom's l-th pending record; 32 pending
+// Record sink of the count pass: besides the counts, every candidate step of
+// the atom with at least one hit becomes a record {hit mask, first candidate,
+// the cell's image shift in three signed 10-bit fields}; with several cutoffs
+// (MULTI) one record per list with a hit, the list in the shift's top two
+// bits, and the header is followed by the atom's edges of each list in
+// earlier segments.  Lane l buffers the atom's l-th pending record; 32 pending
 // records (and the atom's last ones) are flushed as one segment whose header
 // holds the atom's run slot, its edges in earlier segments, the record count
 // and the system.  Each atom's first segment was reserved with its warp's
@@ -546,10 +548,12 @@ __device__ __forceinline__ void system_cutoff(const CutoffSet& cs, const SysPlan
 // when empty, and further segments (atoms with more than 32 records) are
 // taken one by one.  A segment or a shift that does not fit sets the
 // overflow flag: the emit pass then recomputes instead of expanding.
+template <bool MULTI>
 struct RecSink {
   const CutoffSet* cs;
   BatchRecords rb;
-  uint32_t cnt = 0;  // lane 0: the atom's edge count
+  uint32_t cnt = 0;   // lane q: the atom's edge count of list q
+  uint32_t done = 0;  // MULTI, lane q: of these, the ones in flushed segments
   uint32_t r_mask = 0, r_j = 0, r_sh = 0;  // lane l: pending record l
   int n_rec = 0, e_done = 0, e_buf = 0;  // warp-uniform
   int32_t p_abs = 0, sys = 0;
@@ -581,34 +585,61 @@ struct RecSink {
         r[1] = r_j;
         r[2] = r_sh;
       }
-      if (lane == 0) rb.seg_hdr[sg] = make_int4(p_abs, e_done, n_rec, sys);
+      if (MULTI) {
+        int4* hdr = rb.seg_hdr + 2 * (size_t)sg;
+        if (lane == 0) hdr[0] = make_int4(p_abs, 0, n_rec, sys);
+        if (lane < kBatchRecordLists) reinterpret_cast<uint32_t*>(hdr + 1)[lane] = done;
+      } else if (lane == 0) {
+        rb.seg_hdr[sg] = make_int4(p_abs, e_done, n_rec, sys);
+      }
     } else if (lane == 0) {
       *rb.overflow = 1;
     }
+    done = cnt;
     e_done += e_buf;
     e_buf = 0;
     n_rec = 0;
   }
-  __device__ __forceinline__ void operator()(bool hit, double d2, int32_t, int32_t,
-                                             const int32_t*) {
-    const int lane = threadIdx.x & 31;
-    const bool h = hit && d2 < cs->rc_sq[0] && !(cs->disjoint && d2 < cs->lower_sq);
-    const unsigned m = __ballot_sync(0xffffffffu, h);
-    if (!m) return;
-    if (lane == 0) cnt += __popc(m);
-    if (!sh_ok && lane == 0) *rb.overflow = 1;
-    if (lane == n_rec) {
+  __device__ __forceinline__ void push(unsigned m, uint32_t sh) {
+    if ((threadIdx.x & 31) == n_rec) {
       r_mask = m;
       r_j = cur_j;
-      r_sh = cur_sh;
+      r_sh = sh;
     }
     ++n_rec;
     e_buf += __popc(m);
     if (n_rec == 32) flush(false);
   }
+  __device__ __forceinline__ void operator()(bool hit, double d2, int32_t, int32_t,
+                                             const int32_t*) {
+    const int lane = threadIdx.x & 31;
+    if (MULTI) {
+      if (!__any_sync(0xffffffffu, hit)) return;
+      if (!sh_ok && lane == 0) *rb.overflow = 1;
+      const int k = cs->k;
+      double prev = cs->lower_sq;
+      for (int q = 0; q < k; ++q) {
+        const double rq = cs->rc_sq[q];
+        const bool h = hit && d2 < rq && !(cs->disjoint && d2 < prev);
+        const unsigned m = __ballot_sync(0xffffffffu, h);
+        prev = rq;
+        if (!m) continue;
+        if (lane == q) cnt += __popc(m);
+        push(m, (cur_sh & 0x3fffffffu) | ((uint32_t)q << 30));
+      }
+      return;
+    }
+    const bool h = hit && d2 < cs->rc_sq[0] && !(cs->disjoint && d2 < cs->lower_sq);
+    const unsigned m = __ballot_sync(0xffffffffu, h);
+    if (!m) return;
+    if (lane == 0) cnt += __popc(m);
+    if (!sh_ok && lane == 0) *rb.overflow = 1;
+    push(m, cur_sh);
+  }
 };
 
-template <int THREADS, bool REC>
+// REC: no records (0), of one list (1), of up to four (2).
+template <int THREADS, int REC>
 // 80 registers per thread for 64 / 128 / 256-thread CTAs.  The 512-thread count
 // spills at the 64-register budget of two CTAs per SM; one CTA per SM with
 // room for ~106 registers measured 7-8 % faster.
@@ -654,7 +685,7 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 512 ? 1 : 768 / THREADS)
     }
     for (int p = item.y + warp, q = 0; p < p_end; p += kWarps, ++q) {
       if (REC) {
-        RecSink sink{csp, rb};
+        RecSink<REC == 2> sink{csp, rb};
         sink.p_abs = P.slot + p;
         sink.sys = item.x;
         sink.first_sg = seg_base + q;
@@ -663,7 +694,7 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 512 ? 1 : 768 / THREADS)
         else
           visit_smem_brute_atom(P, v, p, csp->max_sq, sink);
         sink.flush(true);
-        if (lane == 0) counts[P.slot + p] = sink.cnt;
+        if (lane < (REC == 2 ? csp->k : 1)) counts[(int64_t)lane * row + P.slot + p] = sink.cnt;
       } else {
         CountSink sink{csp, 0u};
         if (P.method == 2)
@@ -771,19 +802,27 @@ __device__ __forceinline__ int select_bit(uint32_t m, int k) {
   return pos;
 }
 
-// Expansion of the count pass's records into the single-cutoff list: one
-// warp per segment; each record's hit lanes write (i, j, shift) at the
+// Expansion of the count pass's records into the lists (MULTI: one list after
+// the other, so that each list's stores stay contiguous): one warp per
+// segment; each record's hit lanes write (i, j, shift) at the
 // atom's next slots, in record order -- the order the recomputing emit pass
 // writes.  Shifts: (s_j - s_i) + the cell's image shift (cell list; zero
 // wrap shifts and image for raw brute force); the minimum-image systems
 // recompute the pair's shift from the raw positions exactly as the count
 // pass did.
+//
+// Two shells of 333 systems (8 to 256 atoms, 0.9 M edges): the recomputing
+// pass took 152 us, this one 49 (the records cost the count pass 1).
+template <bool MULTI>
 __global__ void __launch_bounds__(256, 4)
     k_batch_expand(BatchRecords rb, const SysPlan* __restrict__ plans,
                    const double* __restrict__ pos, const int64_t* __restrict__ offs, int64_t row,
-                   EmitTargets t) {
+                   int n_lists, EmitTargets t) {
   if (t.scan_error && *t.scan_error != 0) return;
-  if (t.capacity > 0 && offs[row] - offs[0] > t.capacity) return;
+  if (t.capacity > 0) {
+    for (int q = 0; q < (MULTI ? n_lists : 1); ++q)
+      if (offs[(int64_t)(q + 1) * row] - offs[(int64_t)q * row] > t.capacity) return;
+  }
   if (*rb.overflow) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *rb.need_recompute = 1;
     return;
@@ -794,17 +833,19 @@ __global__ void __launch_bounds__(256, 4)
   // (the next segment's header and records are loaded while this one is
   // written)
   int sg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int4 hdr_next = make_int4(0, 0, 0, 0);
+  constexpr int kHdr = MULTI ? 2 : 1;
+  int4 hdr_next = make_int4(0, 0, 0, 0), done_next = hdr_next;
   uint32_t rec_next[3] = {0u, 0u, 0u};
   if (sg < n_seg) {
-    hdr_next = rb.seg_hdr[sg];
+    hdr_next = rb.seg_hdr[(size_t)kHdr * sg];
+    if (MULTI) done_next = rb.seg_hdr[(size_t)kHdr * sg + 1];
     const uint32_t* r = rb.rec + ((size_t)sg * 32 + lane) * 3;
     rec_next[0] = r[0];
     rec_next[1] = r[1];
     rec_next[2] = r[2];
   }
   for (; sg < n_seg; sg += warps) {
-    const int4 hdr = hdr_next;
+    const int4 hdr = hdr_next, done = done_next;
     uint32_t my_mask = 0, my_j = 0, my_sh = 0;
     if (lane < hdr.z) {
       my_mask = rec_next[0];
@@ -812,7 +853,8 @@ __global__ void __launch_bounds__(256, 4)
       my_sh = rec_next[2];
     }
     if (sg + warps < n_seg) {
-      hdr_next = rb.seg_hdr[sg + warps];
+      hdr_next = rb.seg_hdr[(size_t)kHdr * (sg + warps)];
+      if (MULTI) done_next = rb.seg_hdr[(size_t)kHdr * (sg + warps) + 1];
       const uint32_t* r = rb.rec + ((size_t)(sg + warps) * 32 + lane) * 3;
       rec_next[0] = r[0];
       rec_next[1] = r[1];
@@ -823,17 +865,7 @@ __global__ void __launch_bounds__(256, 4)
     const int64_t start = P->start;
     const int32_t slot = P->slot;
     const SlotMeta mi = rb.meta[hdr.x];
-    const int64_t cur = t.base[0] + (offs[hdr.x] - offs[0]) + hdr.y;
     const int64_t idx_off = t.local_indices ? t.index_offset : start + t.index_offset;
-    int64_t* src = t.src[0];
-    int64_t* dst = t.dst[0];
-    if (t.system_blocks) {
-      // This system's list is one [src | dst] block at src[0] + 2 b0.
-      const int64_t b0 = offs[slot] - offs[0];
-      const int64_t m_sys = offs[slot + P->n] - offs[slot];
-      src = t.src[0] + b0;
-      dst = t.src[0] + b0 + m_sys;
-    }
     double xi = 0.0, yi = 0.0, zi = 0.0;
     if (method == 1) {
       const double* pi = pos + 3 * (start + mi.orig);
@@ -841,55 +873,70 @@ __global__ void __launch_bounds__(256, 4)
       yi = pi[1];
       zi = pi[2];
     }
-    // The segment's hits are consecutive in the list: hit h (records in
-    // order, bits in order) goes to slot cur + h.  Each lane takes hits h =
-    // lane, lane + 32, ...: its record by a binary search over the records'
-    // inclusive hit counts, its candidate as that record's (h - first)-th
-    // set bit; the warp's stores are contiguous.
-    const int c = __popc(my_mask);
-    int incl = c;
+    for (int q = 0; q < (MULTI ? n_lists : 1); ++q) {
+      // The segment's hits are consecutive in the list: hit h (records in
+      // order, bits in order) goes to slot cur + h.  Each lane takes hits h =
+      // lane, lane + 32, ...: its record by a binary search over the records'
+      // inclusive hit counts, its candidate as that record's (h - first)-th
+      // set bit; the warp's stores are contiguous.
+      const int c = !MULTI || (int)(my_sh >> 30) == q ? __popc(my_mask) : 0;
+      int incl = c;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    const int excl = incl - c;
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-#pragma unroll 2
-    for (int h0 = 0; h0 < total; h0 += 32) {
-      const int h = h0 + lane;
-      int r = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, incl, r + step - 1);
-        if (v <= h) r += step;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
       }
-      const uint32_t mask = __shfl_sync(0xffffffffu, my_mask, r);
-      const int32_t j0 = (int32_t)__shfl_sync(0xffffffffu, my_j, r);
-      const uint32_t psh = __shfl_sync(0xffffffffu, my_sh, r);
-      const int first = __shfl_sync(0xffffffffu, excl, r);
-      if (h < total) {
-        const int jj = select_bit(mask, h - first);
-        const SlotMeta mj = rb.meta[slot + j0 + jj];
-        int32_t s[3];
-        if (method == 1) {
-          const double* pj = pos + 3 * (start + mj.orig);
-          double df[3];
-          matvec(P->g.hinv, dsub(pj[0], xi), dsub(pj[1], yi), dsub(pj[2], zi), df);
+      const int excl = incl - c;
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      if (MULTI && total == 0) continue;
+      const int64_t* of = offs + (int64_t)q * row;
+      const int before = !MULTI ? hdr.y : q == 0 ? done.x : q == 1 ? done.y : q == 2 ? done.z : done.w;
+      const int64_t cur = t.base[q] + (of[hdr.x] - of[0]) + before;
+      int64_t* src = t.src[q];
+      int64_t* dst = t.dst[q];
+      if (!MULTI && t.system_blocks) {
+        // This system's list is one [src | dst] block at src[0] + 2 b0.
+        const int64_t b0 = offs[slot] - offs[0];
+        const int64_t m_sys = offs[slot + P->n] - offs[slot];
+        src = t.src[0] + b0;
+        dst = t.src[0] + b0 + m_sys;
+      }
+#pragma unroll 2
+      for (int h0 = 0; h0 < total; h0 += 32) {
+        const int h = h0 + lane;
+        int r = 0;
 #pragma unroll
-          for (int a = 0; a < 3; ++a) s[a] = sat_i32(P->pbc[a] ? -round(df[a]) : 0.0);
-        } else {
-          s[0] = (mj.sx - mi.sx) + ((int32_t)(psh << 22) >> 22);
-          s[1] = (mj.sy - mi.sy) + ((int32_t)(psh << 12) >> 22);
-          s[2] = (mj.sz - mi.sz) + ((int32_t)(psh << 2) >> 22);
+        for (int step = 16; step > 0; step >>= 1) {
+          const int v = __shfl_sync(0xffffffffu, incl, r + step - 1);
+          if (v <= h) r += step;
         }
-        const int64_t e = cur + h;
-        src[e] = (int64_t)mi.orig + idx_off;
-        dst[e] = (int64_t)mj.orig + idx_off;
-        int32_t* sp = t.sh[0] + 3 * e;
-        sp[0] = s[0];
-        sp[1] = s[1];
-        sp[2] = s[2];
+        const uint32_t mask = __shfl_sync(0xffffffffu, my_mask, r);
+        const int32_t j0 = (int32_t)__shfl_sync(0xffffffffu, my_j, r);
+        const uint32_t psh = __shfl_sync(0xffffffffu, my_sh, r);
+        const int first = __shfl_sync(0xffffffffu, excl, r);
+        if (h < total) {
+          const int jj = select_bit(mask, h - first);
+          const SlotMeta mj = rb.meta[slot + j0 + jj];
+          int32_t s[3];
+          if (method == 1) {
+            const double* pj = pos + 3 * (start + mj.orig);
+            double df[3];
+            matvec(P->g.hinv, dsub(pj[0], xi), dsub(pj[1], yi), dsub(pj[2], zi), df);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) s[a] = sat_i32(P->pbc[a] ? -round(df[a]) : 0.0);
+          } else {
+            s[0] = (mj.sx - mi.sx) + ((int32_t)(psh << 22) >> 22);
+            s[1] = (mj.sy - mi.sy) + ((int32_t)(psh << 12) >> 22);
+            s[2] = (mj.sz - mi.sz) + ((int32_t)(psh << 2) >> 22);
+          }
+          const int64_t e = cur + h;
+          src[e] = (int64_t)mi.orig + idx_off;
+          dst[e] = (int64_t)mj.orig + idx_off;
+          int32_t* sp = t.sh[q] + 3 * e;
+          sp[0] = s[0];
+          sp[1] = s[1];
+          sp[2] = s[2];
+        }
       }
     }
   }
@@ -942,19 +989,21 @@ const BatchShape kBatchShapeTable[kBatchShapes] = {
 
 namespace {
 
-using CountFn = decltype(&k_batch_count<256, false>);
+using CountFn = decltype(&k_batch_count<256, 0>);
 using EmitFn = decltype(&k_batch_emit<256>);
 
-CountFn count_fn(int threads, bool rec = false) {
-  if (rec)
-    return threads <= 64    ? &k_batch_count<64, true>
-           : threads <= 128 ? &k_batch_count<128, true>
-           : threads <= 256 ? &k_batch_count<256, true>
-                            : &k_batch_count<512, true>;
-  return threads <= 64    ? &k_batch_count<64, false>
-         : threads <= 128 ? &k_batch_count<128, false>
-         : threads <= 256 ? &k_batch_count<256, false>
-                          : &k_batch_count<512, false>;
+template <int REC>
+CountFn count_fn_of(int threads) {
+  return threads <= 64    ? &k_batch_count<64, REC>
+         : threads <= 128 ? &k_batch_count<128, REC>
+         : threads <= 256 ? &k_batch_count<256, REC>
+                          : &k_batch_count<512, REC>;
+}
+// rec: the kernel's REC
+CountFn count_fn(int threads, int rec) {
+  return rec == 2   ? count_fn_of<2>(threads)
+         : rec == 1 ? count_fn_of<1>(threads)
+                    : count_fn_of<0>(threads);
 }
 EmitFn emit_fn(int threads) {
   return threads <= 64    ? &k_batch_emit<64>
@@ -970,8 +1019,7 @@ void preload_batch_kernels() {
   // asks for its attributes first (lazy loading): do it for every variant.
   cudaFuncAttributes a;
   for (int threads : {64, 128, 256, 512}) {
-    cudaFuncGetAttributes(&a, (const void*)count_fn(threads));
-    cudaFuncGetAttributes(&a, (const void*)count_fn(threads, true));
+    for (int rec : {0, 1, 2}) cudaFuncGetAttributes(&a, (const void*)count_fn(threads, rec));
     cudaFuncGetAttributes(&a, (const void*)emit_fn(threads));
   }
   cudaGetLastError();
@@ -984,9 +1032,10 @@ void launch_batch_count(const SysPlan* plans, const BatchItems& w, const double*
   BatchRecords rb;
   std::memset(&rb, 0, sizeof(rb));
   if (rec) rb = *rec;
+  const int kind = !rec ? 0 : cs.k > 1 ? 2 : 1;
   if (w.n_large > 0) {
     const size_t smem = batch_smem_bytes(w.cap_large);
-    const CountFn k = count_fn(sh.large_threads, rec != nullptr);
+    const CountFn k = count_fn(sh.large_threads, kind);
     ensure_smem_attr((const void*)k, (int)smem);
     const int grid = std::min(grid_for((const void*)k, sh.large_threads, smem), w.n_large);
     k<<<grid, sh.large_threads, smem, s>>>(plans, w.items, w.n_large, sh.chunk, pos,
@@ -995,7 +1044,7 @@ void launch_batch_count(const SysPlan* plans, const BatchItems& w, const double*
   }
   if (w.n_small > 0) {
     const size_t smem = batch_smem_bytes(w.cap_small);
-    const CountFn k = count_fn(sh.small_threads, rec != nullptr);
+    const CountFn k = count_fn(sh.small_threads, kind);
     ensure_smem_attr((const void*)k, (int)smem);
     const int grid = std::min(grid_for((const void*)k, sh.small_threads, smem), w.n_small);
     k<<<grid, sh.small_threads, smem, s>>>(plans, w.items + w.n_large, w.n_small, 1 << 30, pos,
@@ -1005,9 +1054,11 @@ void launch_batch_count(const SysPlan* plans, const BatchItems& w, const double*
 }
 
 void launch_batch_expand(const BatchRecords& rb, const SysPlan* plans, const double* pos,
-                         const int64_t* offs, int64_t row, const EmitTargets& t, cudaStream_t s) {
-  const int grid = grid_for((const void*)k_batch_expand, 256, 0);
-  k_batch_expand<<<grid, 256, 0, s>>>(rb, plans, pos, offs, row, t);
+                         const int64_t* offs, int64_t row, int n_lists, const EmitTargets& t,
+                         cudaStream_t s) {
+  const auto k = n_lists > 1 ? &k_batch_expand<true> : &k_batch_expand<false>;
+  const int grid = grid_for((const void*)k, 256, 0);
+  k<<<grid, 256, 0, s>>>(rb, plans, pos, offs, row, n_lists, t);
   note_launches(1);
 }
 

@@ -254,7 +254,7 @@ struct FastBatchArgs {
   int64_t* d_bounds;  // nullptr: no per-system offsets
   BatchItems bw;
   int64_t cap;
-  bool use_rec;          // single cutoff: count pass records hits, expansion writes the list
+  bool use_rec;          // up to four lists: count pass records hits, expansion writes the lists
   BatchRecords rec;
   int32_t* rec_flags;    // rec.seg_top / overflow / need_recompute (zeroed per batch)
 };
@@ -265,12 +265,14 @@ void issue_emit_fast(Ctx& c, const FastBatchArgs& a, const std::vector<double>& 
   if (a.use_rec && !recompute) {
     EmitTargets t;
     std::memset(&t, 0, sizeof(t));
-    t.src[0] = static_cast<int64_t*>(c.batch_out[0].p);
-    t.dst[0] = static_cast<int64_t*>(c.batch_out[1].p);
-    t.sh[0] = static_cast<int32_t*>(c.batch_out[2].p);
+    for (int32_t q = 0; q < k; ++q) {
+      t.src[q] = static_cast<int64_t*>(c.batch_out[3 * q].p);
+      t.dst[q] = static_cast<int64_t*>(c.batch_out[3 * q + 1].p);
+      t.sh[q] = static_cast<int32_t*>(c.batch_out[3 * q + 2].p);
+    }
     t.capacity = a.cap;
     t.scan_error = a.scan_tmp + 1;
-    launch_batch_expand(a.rec, a.plans, a.d_pos, a.offs, a.row, t, s);
+    launch_batch_expand(a.rec, a.plans, a.d_pos, a.offs, a.row, k, t, s);
     return;
   }
   for (int32_t g0 = 0; g0 < k; g0 += kMaxCutoffsPerPass) {
@@ -393,25 +395,22 @@ Status run_small_fast(Ctx& c, const double* d_pos, const std::vector<int64_t>& s
   // The arenas' actual capacity (so that repeated calls see the same value
   // once the arenas stop growing).
   a.cap = arena_capacity(c, k);
-  // Hit records (single cutoff): at most one segment per atom plus one per
-  // 32 records, and a record holds at least one of the <= cap edges.
-  a.use_rec = k == 1;
+  // Hit records: at most one segment per atom plus one per 32 records, and a
+  // record holds at least one of a list's <= cap edges.  Without the memory
+  // for them the emit pass recomputes.
+  const int64_t segs = run_atoms + k * (cap / 32 + 1) + 1024;
+  a.use_rec = k <= kBatchRecordLists && segs <= INT32_MAX / 2;
   if (a.use_rec) {
-    const int64_t segs = run_atoms + cap / 32 + 1024;
-    if (segs > INT32_MAX / 2) {
-      a.use_rec = false;
-    } else {
-      a.rec.seg_cap = (int)segs;
-      a.rec.seg_hdr = slot<int4>(c, kSlotBatch0 + 13, (size_t)segs);
-      a.rec.rec = slot<uint32_t>(c, kSlotBatch0 + 14, (size_t)segs * 96);
-      a.rec.meta = slot<SlotMeta>(c, kSlotBatch0 + 15, (size_t)run_atoms);
-      a.rec_flags = slot<int32_t>(c, kSlotBatch0 + 12, 3);
-      if (!a.rec.seg_hdr || !a.rec.rec || !a.rec.meta || !a.rec_flags)
-        return fail(NLB_ERR_NOMEM, "device allocation failed");
-      a.rec.seg_top = a.rec_flags;
-      a.rec.overflow = a.rec_flags + 1;
-      a.rec.need_recompute = a.rec_flags + 2;
-    }
+    a.rec.seg_cap = (int)segs;
+    a.rec.seg_hdr = slot<int4>(c, kSlotBatch0 + 13, (size_t)segs * (k > 1 ? 2 : 1));
+    a.rec.rec = slot<uint32_t>(c, kSlotBatch0 + 14, (size_t)segs * 96);
+    a.rec.meta = slot<SlotMeta>(c, kSlotBatch0 + 15, (size_t)run_atoms);
+    a.rec_flags = slot<int32_t>(c, kSlotBatch0 + 12, 3);
+    a.rec.seg_top = a.rec_flags;
+    a.rec.overflow = a.rec_flags + 1;
+    a.rec.need_recompute = a.rec_flags + 2;
+    a.use_rec = a.rec.seg_hdr && a.rec.rec && a.rec.meta && a.rec_flags;
+    if (!a.use_rec) std::memset(&a.rec, 0, sizeof(a.rec));
   }
 
   // Everything the issued work depends on.

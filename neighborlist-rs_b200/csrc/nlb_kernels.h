@@ -377,12 +377,16 @@ struct BatchItems {
 // Host: builds the item list (upload it and set w.items before launching).
 void plan_batch_items(const int64_t* sizes, int n_sys, const BatchShape& shape,
                       std::vector<int2>& items, BatchItems& w);
-// Hit records of a single-cutoff batched count pass, expanded into the list
-// by launch_batch_expand instead of a recomputing emit pass.  seg_top,
+// Hit records of a batched count pass of up to kBatchRecordLists lists,
+// expanded into the lists by launch_batch_expand instead of a recomputing emit pass.  seg_top,
 // overflow and need_recompute must be zero on entry; capacity: seg_cap
 // segments of 32 records (3 words each), meta: one per run slot.
+constexpr int kBatchRecordLists = 4;  // (a record has two bits for its list)
 struct BatchRecords {
-  int4* seg_hdr;         // {run slot of the atom, its edges in earlier segments, records, system}
+  // {run slot of the atom, its edges in earlier segments, records, system}; with
+  // several lists followed by the edges of each list in earlier segments
+  // (two int4 per segment)
+  int4* seg_hdr;
   uint32_t* rec;         // [seg_cap * 32 * 3]
   SlotMeta* meta;        // sorted meta per run slot (orig: index within the system)
   int* seg_top;          // segments used
@@ -392,14 +396,16 @@ struct BatchRecords {
 };
 
 // counts[q * row + slot + p]; work2[0..1] must be zero on entry.  With rec
-// (single-cutoff passes only) the pass also writes hit records.
+// (at most kBatchRecordLists cutoffs) the pass also writes hit records.
 void launch_batch_count(const SysPlan* plans, const BatchItems& w, const double* pos,
                         const CutoffSet& cs, uint32_t* counts, int64_t row, int* work2,
                         cudaStream_t s, const BatchRecords* rec = nullptr);
-// Writes the single-cutoff list from the records (t: src/dst/sh[0], base[0],
-// index options, capacity and scan_error as for launch_batch_emit).
+// Writes the lists from the records (t: src/dst/sh, base, index options,
+// capacity and scan_error as for launch_batch_emit; system_blocks with one
+// list only).
 void launch_batch_expand(const BatchRecords& rb, const SysPlan* plans, const double* pos,
-                         const int64_t* offs, int64_t row, const EmitTargets& t, cudaStream_t s);
+                         const int64_t* offs, int64_t row, int n_lists, const EmitTargets& t,
+                         cudaStream_t s);
 void launch_batch_emit(const SysPlan* plans, const BatchItems& w, const double* pos,
                        const CutoffSet& cs, const int64_t* offs, int64_t row,
                        const EmitTargets& t, int* work2, cudaStream_t s);

@@ -758,7 +758,7 @@ class Server {
     t.local_indices = 1;
     t.system_blocks = 1;  // request i: [src | dst] at src + 2 hb[i]
     if (use_rec && (diag[2] & 0xffffffff) == 0) {
-      launch_batch_expand(rb, plans, d_pos, offs, row, t, s);
+      launch_batch_expand(rb, plans, d_pos, offs, row, 1, t, s);
     } else {
       cudaMemsetAsync(flags + 1, 0, sizeof(int32_t) * 2, s);
       launch_batch_emit(plans, trials.pick(*c), d_pos, cs, offs, row, t, flags + 1, s);
