@@ -211,37 +211,88 @@ __device__ __forceinline__ bool triple_less(uint64_t a0, uint64_t a1, int32_t a2
   return a2 < b2;
 }
 
+// One aligned run of 32 triples per warp: a bitonic network on shuffles
+// (lane l holds element l; padding lanes hold the largest triple).
+__device__ __forceinline__ void sort_run32(uint64_t& k0, uint64_t& k1, int32_t& k2) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      const uint64_t o0 = __shfl_xor_sync(0xffffffffu, k0, stride);
+      const uint64_t o1 = __shfl_xor_sync(0xffffffffu, k1, stride);
+      const int32_t o2 = __shfl_xor_sync(0xffffffffu, k2, stride);
+      const bool keep_min = ((lane & size) == 0) == ((lane & stride) == 0);
+      if (triple_less(o0, o1, o2, k0, k1, k2) == keep_min) {
+        k0 = o0;
+        k1 = o1;
+        k2 = o2;
+      }
+    }
+}
+
+// Sorts the triples (bcode, key, idx), all different by idx, in place:
+// runs of 32 in registers, then merges in which every element finds its
+// place by a binary search in the sibling run, between the triples and the
+// position / meta arrays (not yet filled).  A bitonic sort in shared memory
+// has log2(n)(log2(n) + 1) / 2 steps with a barrier each; this has
+// log2(n / 32) + 1.
+// Measured on the count pass: one system of 1,900 atoms 254 -> 211 us, 64 of
+// 1,000 416 -> 375, 4,096 of 8 to 256 unchanged (471, 466).
 __device__ void sort_triples(const SmemView& v, int n) {
-  int p = 1;
-  while (p < n) p <<= 1;
-  for (int i = n + threadIdx.x; i < p; i += blockDim.x) {
-    v.bcode[i] = ~0ull;
-    v.key[i] = ~0ull;
-    v.idx[i] = 0x7fffffff;
+  uint64_t *a0 = v.bcode, *a1 = v.key;
+  int32_t* a2 = v.idx;
+  uint64_t* b0 = reinterpret_cast<uint64_t*>(v.px);
+  uint64_t* b1 = reinterpret_cast<uint64_t*>(v.py);
+  int32_t* b2 = reinterpret_cast<int32_t*>(v.meta);
+  int levels = 0;
+  while ((32 << levels) < n) ++levels;
+  const bool swap = levels & 1;  // (an odd number of merges starts in the other arrays)
+  for (int q = 32 * (threadIdx.x >> 5); q < n; q += blockDim.x) {
+    const int p = q + (threadIdx.x & 31);
+    uint64_t k0 = ~0ull, k1 = ~0ull;
+    int32_t k2 = 0x7fffffff;
+    if (p < n) {
+      k0 = a0[p];
+      k1 = a1[p];
+      k2 = a2[p];
+    }
+    sort_run32(k0, k1, k2);
+    if (p < n) {
+      (swap ? b0 : a0)[p] = k0;
+      (swap ? b1 : a1)[p] = k1;
+      (swap ? b2 : a2)[p] = k2;
+    }
   }
   __syncthreads();
-  for (int size = 2; size <= p; size <<= 1)
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < p; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & size) == 0;
-          const bool gt = triple_less(v.bcode[j], v.key[j], v.idx[j], v.bcode[i], v.key[i], v.idx[i]);
-          if (gt == up) {
-            uint64_t t0 = v.bcode[i];
-            v.bcode[i] = v.bcode[j];
-            v.bcode[j] = t0;
-            uint64_t t1 = v.key[i];
-            v.key[i] = v.key[j];
-            v.key[j] = t1;
-            int32_t t2 = v.idx[i];
-            v.idx[i] = v.idx[j];
-            v.idx[j] = t2;
-          }
-        }
+  for (int l = 0; l < levels; ++l) {
+    const bool from_b = ((l & 1) != 0) != swap;
+    const uint64_t *s0 = from_b ? b0 : a0, *s1 = from_b ? b1 : a1;
+    const int32_t* s2 = from_b ? b2 : a2;
+    uint64_t *d0 = from_b ? a0 : b0, *d1 = from_b ? a1 : b1;
+    int32_t* d2 = from_b ? a2 : b2;
+    const int len = 32 << l;
+    for (int p = threadIdx.x; p < n; p += blockDim.x) {
+      const uint64_t k0 = s0[p], k1 = s1[p];
+      const int32_t k2 = s2[p];
+      const int off = p & (len - 1), base = p & ~(2 * len - 1);
+      const int sib = (p ^ len) & ~(len - 1);
+      int lo = min(sib, n), hi = min(sib + len, n);
+      const int first = lo;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (triple_less(s0[mid], s1[mid], s2[mid], k0, k1, k2))
+          lo = mid + 1;
+        else
+          hi = mid;
       }
-      __syncthreads();
+      const int to = base + off + (lo - first);
+      d0[to] = k0;
+      d1[to] = k1;
+      d2[to] = k2;
     }
+    __syncthreads();
+  }
 }
 
 __device__ __forceinline__ uint64_t bin_code(int32_t bx, int32_t by, int32_t bz) {
