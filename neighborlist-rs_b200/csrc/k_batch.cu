@@ -1147,9 +1147,15 @@ void plan_batch_items(const int64_t* sizes, int n_sys, const BatchShape& shape,
   w = BatchItems{};
   w.shape = shape;
   int64_t max_large = 0, max_small = 0;
+  // (whole systems are items like the others when both kinds run in CTAs of
+  // one size: one launch instead of two, one after the other)
+  const int64_t split =
+      shape.small_threads == shape.large_threads && shape.chunk >= shape.large_atoms
+          ? 0
+          : shape.large_atoms;
   for (int32_t i : order) {
     const int64_t n = sizes[i];
-    if (n > shape.large_atoms) {
+    if (n > split) {
       for (int64_t a = 0; a < n; a += shape.chunk) items.push_back(make_int2(i, (int)a));
       max_large = std::max(max_large, n);
     }
@@ -1157,7 +1163,7 @@ void plan_batch_items(const int64_t* sizes, int n_sys, const BatchShape& shape,
   w.n_large = (int)items.size();
   for (int32_t i : order) {
     const int64_t n = sizes[i];
-    if (n <= shape.large_atoms) {
+    if (n <= split) {
       items.push_back(make_int2(i, 0));
       max_small = std::max(max_small, n);
     }

@@ -18,7 +18,8 @@
 //     process -- its emit pass, which walks the same pairs, and every later
 //     batch of the kind use it.
 //
-// A new kind therefore costs a few extra count passes once, and a batch of a
+// A batch too small to fill the GPU is cut finer than any of these shapes, by a
+// rule (fine_shape) and without trials.  A new kind therefore costs a few extra count passes once, and a batch of a
 // known kind nothing.  Every kernel variant is loaded before the first timed
 // launch, so no candidate pays for loading a module.  NLB_BATCH_SHAPE=i in
 // the environment, or nlb_batch_shape(i), pins shape i for every batch.
@@ -112,15 +113,44 @@ TuneKey make_tune_key(int32_t device, int32_t k, const int64_t* sizes, int32_t n
   return key;
 }
 
+// A batch that leaves the GPU mostly idle (at most kFineAtoms atoms per SM, and
+// not many more systems than SMs) is cut finer than any shape of the table,
+// down to one atom per warp, and needs no trials: such a batch is as slow as
+// its slowest work item, and an atom takes a warp some 5 us.  The pieces are
+// the smallest with which the items still run nearly at once, one CTA of 512
+// threads per SM (each item sorts its whole system again).  Count pass, best
+// shape of the table against this one, us: one system of 200 atoms 35 / 13, of
+// 1,000 111 / 40, of 1,900 131 / 59; six of 300 to 1,600 242 / 66; 64 of 64
+// 39 / 28; 9 of 2,000 134 / 134.  Many tiny systems are better off in the
+// table's small CTAs (300 of 16: 35 / 45), and so are larger batches (64 of
+// 1,000: 375 / 870).
+constexpr int64_t kFineAtoms = 128;
+int sm_count(int device) {
+  int n = 0;
+  return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess ? n : 0;
+}
+BatchShape fine_shape(int64_t atoms, int32_t n_sys, int sms) {
+  int chunk = 16;
+  while (chunk < 128 && (atoms + chunk - 1) / chunk + n_sys / 2 > sms + sms / 4) chunk <<= 1;
+  return BatchShape{512, 512, chunk, chunk};
+}
+
 Status ShapeTrials::prepare(Ctx& c, const TuneKey& k, const int64_t* sizes, int32_t n_sys,
                            int items_slot) {
   key = k;
   shapes.clear();
   timed = false;
+  int64_t atoms = 0;
+  for (int32_t i = 0; i < n_sys; ++i) atoms += sizes[i];
+  const int sms = sm_count(c.device);
+  BatchShape fine{};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     if (g_pinned >= 0) {
       shapes.push_back(g_pinned);
+    } else if (atoms <= kFineAtoms * sms && n_sys <= sms + sms / 4) {
+      shapes.push_back(0);
+      fine = fine_shape(atoms, n_sys, sms);
     } else {
       auto it = g_tune.find(key);
       if (it == g_tune.end()) {
@@ -156,7 +186,7 @@ Status ShapeTrials::prepare(Ctx& c, const TuneKey& k, const int64_t* sizes, int3
   std::vector<int2> all, one;
   std::vector<size_t> off(shapes.size());
   for (size_t i = 0; i < shapes.size(); ++i) {
-    plan_batch_items(sizes, n_sys, kBatchShapeTable[shapes[i]], one, w[i]);
+    plan_batch_items(sizes, n_sys, fine.chunk ? fine : kBatchShapeTable[shapes[i]], one, w[i]);
     off[i] = all.size();
     all.insert(all.end(), one.begin(), one.end());
   }
