@@ -7,20 +7,20 @@
 //   k_max_disp      max_i |r_i - r_i,ref|^2 over the atoms (FP64, exact
 //                   squares and sums; the max of non-negative doubles is
 //                   taken on their bit patterns, which order the same way)
-//   k_verlet_compact  one launch per update: that maximum, and one pass over
-//                   the stored edges (i, j, S): kept when |(r_j - r_i) +
-//                   H.S|^2 < rc^2 with the current positions (the
-//                   displacement expression of k_extras.cu), compacted in
-//                   stored order by a decoupled look-back over tiles ([src |
-//                   dst], shifts); M and the maximum go to the host through
-//                   host-mapped memory
-// A streaming kernel: 12 B + two position gathers per stored edge, 28 B (+ 8
-// for the destinations' move, int32 in between) per kept edge.  With 28-byte
-// stored edges, read again for the kept ones, int64 destinations in between,
-// a launch of its own for the maximum and copies and a synchronisation for
-// the results, an update of the 10,008-atom liquid (rc 6, skin 1) took 74 us.
+//   k_verlet_count  that maximum, and one pass over the stored edges (i, j, S):
+//                   kept when |(r_j - r_i) + H.S|^2 < rc^2 with the current
+//                   positions (the displacement expression of k_extras.cu), as
+//                   a bit per edge and counts; M and the maximum go to the
+//                   host through host-mapped memory as soon as they are known
+//   k_verlet_write  the kept edges in stored order ([src | dst], shifts), while
+//                   the caller goes on
+// Streaming kernels: 12 B + two position gathers per stored edge, 12 + 28 B per
+// kept edge.  An update of the 10,008-atom liquid (rc 6, skin 1, 0.7 M stored
+// edges) has a floor of 5 us and is a chain of latencies: 16 us for the count,
+// 7.6 for the write; the call took 74 us in three launches with copies and a
+// synchronisation, 45 in one launch that found the slots by a look-back and
+// moved the destinations behind the sources at its end, and takes 32.
 #include <algorithm>
-#include <atomic>
 
 #include "nlb_kernels.h"
 
@@ -81,12 +81,9 @@ __global__ void k_max_disp(const double* __restrict__ pos, const double* __restr
 }
 
 constexpr int kVcThreads = 256;
-constexpr int kVcPer = 8;                          // stored edges per thread
-constexpr int kVcTile = kVcThreads * kVcPer;       // stored edges per tile
-constexpr uint64_t kVcShift = 62;
-constexpr uint64_t kVcAggregate = 1ull << kVcShift;
-constexpr uint64_t kVcInclusive = 2ull << kVcShift;
-constexpr uint64_t kVcValue = (1ull << kVcShift) - 1;
+constexpr int kVcPer = 8;                     // stored edges per thread
+constexpr int kVcTile = kVcThreads * kVcPer;  // stored edges per CTA
+constexpr int kVcWords = kVcTile / 32;        // its mask words
 
 __global__ void k_verlet_pack(const int64_t* __restrict__ ei, const int32_t* __restrict__ sh,
                               int64_t m, int2* __restrict__ ij, uint32_t* __restrict__ packed,
@@ -106,198 +103,163 @@ __global__ void k_verlet_pack(const int64_t* __restrict__ ei, const int32_t* __r
   if (far) atomicExch(wide, 1);
 }
 
-// CTAs first take their share of the largest displacement, then tiles of
-// kVcTile stored edges in order (tickets): tested at rc with the current
-// positions (each warp a run of 256 edges, lane-striped so that loads are
-// coalesced), the tile's first output slot found by a decoupled look-back over
-// the tiles before it (bounded polls; a wait that runs out sets state[1] and
-// the tile writes nothing), the kept edges written in stored order: sources
-// and shifts in place, destinations to dst_tmp.  Once every tile is written
-// (all tickets are held by running CTAs, so the wait ends; bounded all the
-// same), the CTAs move the destinations behind the M sources.  The last CTA
-// to end clears the state for the next launch and reports {M, error word,
-// displacement bits}.  state (zero on entry): [0] ticket, [1] error, [2] tiles
-// done, [3] M, [4] CTAs done, [5] displacement, [6 + t] tile t's look-back
-// word.
+// An update's first launch: the CTA's share of the largest displacement, and
+// one tile of kVcTile stored edges tested at rc with the current positions
+// (each warp a run of 256 edges, lane-striped so that loads are coalesced): a
+// mask word per 32 edges and the tile's count. The last CTA to end turns the
+// counts into the tiles' first slots, reports {M, displacement bits} and
+// leaves done and disp zero for the next launch.
 __global__ void __launch_bounds__(kVcThreads)
-    k_verlet_compact(const double* __restrict__ pos, const double* __restrict__ ref, int64_t n,
-                     EdgeExtrasCell cell, VerletEdges list, double rc_sq,
-                     int64_t* __restrict__ out_ei, int32_t* __restrict__ out_sh,
-                     int32_t* __restrict__ dst_tmp, uint64_t* __restrict__ state,
-                     int32_t spin_limit, int64_t* report) {
-  __shared__ int64_t s_tile, s_base;
-  __shared__ int32_t warp_cnt[kVcThreads / 32];
-  __shared__ int32_t s_skip;
+    k_verlet_count(const double* __restrict__ pos, const double* __restrict__ ref, int64_t n,
+                   const __grid_constant__ EdgeExtrasCell cell,
+                   const __grid_constant__ VerletEdges list, double rc_sq,
+                   const __grid_constant__ VerletWork work, int64_t* report) {
+  __shared__ int64_t warp_sum[kVcThreads / 32];
+  __shared__ double warp_far[kVcThreads / 32];
+  __shared__ bool s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t m = list.m;
   const int64_t n_tiles = (m + kVcTile - 1) / kVcTile;
-  uint64_t* const tiles = state + 6;
+  pdl_wait();
+  const int64_t t = blockIdx.x;
+  const int64_t wbase = t * kVcTile + (int64_t)warp * 32 * kVcPer;
   const bool wide = *list.wide != 0;
-  if ((int64_t)blockIdx.x * kVcThreads < n) {
+  int2 ij[kVcPer];
+  uint32_t psh[kVcPer];
+#pragma unroll
+  for (int k = 0; k < kVcPer; ++k) {
+    const int64_t e = wbase + 32 * k + lane;
+    ij[k] = e < m ? list.ij[e] : make_int2(0, 0);
+    psh[k] = e < m ? list.packed[e] : 0u;
+  }
+  const bool moved = t * kVcThreads < n;
+  if (moved) {
     const double far = max_disp_share(pos, ref, n);
-    if (lane == 0)
-      atomicMax(reinterpret_cast<unsigned long long*>(&state[5]),
-                (unsigned long long)__double_as_longlong(far));
+    if (lane == 0) warp_far[warp] = far;
   }
-  for (;;) {
-    if (tid == 0) s_tile = (int64_t)atomicAdd(reinterpret_cast<unsigned long long*>(state), 1ull);
-    __syncthreads();
-    const int64_t t = s_tile;
-    if (t >= n_tiles) break;
-    const int64_t wbase = t * kVcTile + (int64_t)warp * 32 * kVcPer;
-    int2 ij[kVcPer];
-    uint32_t psh[kVcPer], kmask[kVcPer];
-    int32_t wtot = 0;
+  uint32_t word = 0;  // lane k: the run's mask word k
+  int32_t kept = 0;
 #pragma unroll
-    for (int k = 0; k < kVcPer; ++k) {
-      const int64_t e = wbase + 32 * k + lane;
-      ij[k] = e < m ? list.ij[e] : make_int2(0, 0);
-      psh[k] = e < m ? list.packed[e] : 0u;
+  for (int k = 0; k < kVcPer; ++k) {
+    const int64_t e = wbase + 32 * k + lane;
+    bool keep = false;
+    if (e < m) {
+      int32_t s[3];
+      edge_shift(list, wide, e, psh[k], s);
+      double d[3];
+      edge_disp(pos, cell, ij[k].x, ij[k].y, s[0], s[1], s[2], d);
+      keep = norm2(d[0], d[1], d[2]) < rc_sq;
     }
-#pragma unroll
-    for (int k = 0; k < kVcPer; ++k) {
-      const int64_t e = wbase + 32 * k + lane;
-      bool keep = false;
-      if (e < m) {
-        int32_t s[3];
-        edge_shift(list, wide, e, psh[k], s);
-        double d[3];
-        edge_disp(pos, cell, ij[k].x, ij[k].y, s[0], s[1], s[2], d);
-        keep = norm2(d[0], d[1], d[2]) < rc_sq;
-      }
-      kmask[k] = __ballot_sync(0xffffffffu, keep);
-      wtot += __popc(kmask[k]);
-    }
-    if (lane == 0) warp_cnt[warp] = wtot;
-    __syncthreads();
-    int32_t woff = 0, tile_tot = 0;
-#pragma unroll
+    const uint32_t mask = __ballot_sync(0xffffffffu, keep);
+    if (lane == k) word = mask;
+    kept += __popc(mask);
+  }
+  if (t < n_tiles && lane < kVcPer) work.masks[t * kVcWords + warp * kVcPer + lane] = word;
+  if (lane == 0) warp_sum[warp] = kept;
+  __syncthreads();
+  if (tid == 0) {
+    int64_t sum = 0;
+    double far = 0.0;
     for (int w = 0; w < kVcThreads / 32; ++w) {
-      const int32_t v = warp_cnt[w];
-      woff += w < warp ? v : 0;
-      tile_tot += v;
+      sum += warp_sum[w];
+      if (moved && warp_far[w] > far) far = warp_far[w];
     }
-    if (warp == 0) {
-      // Publish the tile's count at once, then walk back over the tiles
-      // before it (32 at a time) to its first output slot.
-      if (lane == 0) {
-        __threadfence();
-        *reinterpret_cast<volatile uint64_t*>(&tiles[t]) =
-            (t == 0 ? kVcInclusive : kVcAggregate) | (uint64_t)tile_tot;
-      }
-      int64_t prefix = 0;
-      bool failed_any = false;
-      if (t > 0) {
-        int64_t tt = t - 1;
-        for (;;) {
-          const int64_t pred = tt - lane;
-          uint64_t v = kVcInclusive;
-          bool failed = false;
-          if (pred >= 0) {
-            int spins = 0;
-            v = *reinterpret_cast<const volatile uint64_t*>(&tiles[pred]);
-            while ((v >> kVcShift) == 0 && spins < spin_limit) {
-              __nanosleep(32);
-              v = *reinterpret_cast<const volatile uint64_t*>(&tiles[pred]);
-              ++spins;
-            }
-            failed = (v >> kVcShift) == 0;
-          }
-          if (__any_sync(0xffffffffu, failed)) {
-            if (lane == 0) atomicExch(reinterpret_cast<unsigned long long*>(&state[1]), 1ull);
-            failed_any = true;
-            break;
-          }
-          const unsigned inc = __ballot_sync(0xffffffffu, (v >> kVcShift) == 2);
-          const int stop = __ffs(inc) - 1;
-          int64_t val = (pred >= 0 && lane <= (stop < 0 ? 31 : stop)) ? (int64_t)(v & kVcValue) : 0;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
-          prefix += val;
-          if (stop >= 0) break;
-          tt -= 32;
-        }
-        if (lane == 0 && !failed_any) {
-          __threadfence();
-          *reinterpret_cast<volatile uint64_t*>(&tiles[t]) =
-              kVcInclusive | (uint64_t)(prefix + tile_tot);
-        }
-      }
-      if (lane == 0) {
-        s_base = prefix;
-        s_skip = failed_any ? 1 : 0;
-        if (t == n_tiles - 1) state[3] = failed_any ? 0 : (uint64_t)(prefix + tile_tot);
-      }
-    }
-    __syncthreads();
-    if (!s_skip) {
-      const int64_t g = s_base + woff;
-      int32_t acc = 0;
-#pragma unroll
-      for (int k = 0; k < kVcPer; ++k) {
-        if ((kmask[k] >> lane) & 1u) {
-          const int64_t o = g + acc + __popc(kmask[k] & ((1u << lane) - 1u));
-          int32_t s[3];
-          edge_shift(list, wide, wbase + 32 * k + lane, psh[k], s);
-          out_ei[o] = (int64_t)ij[k].x;
-          dst_tmp[o] = ij[k].y;
-          out_sh[3 * o] = s[0];
-          out_sh[3 * o + 1] = s[1];
-          out_sh[3 * o + 2] = s[2];
-        }
-        acc += __popc(kmask[k]);
-      }
-    }
-    // One thread releases the tile's writes (ordered before it by the
-    // barrier) with the completion count.
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      atomicAdd(reinterpret_cast<unsigned long long*>(&state[2]), 1ull);
-    }
-  }
-  if (tid == 0) {
-    int spins = 0;
-    unsigned long long d = *reinterpret_cast<volatile unsigned long long*>(&state[2]);
-    while (d < (unsigned long long)n_tiles && spins < spin_limit) {
-      __nanosleep(64);
-      d = *reinterpret_cast<volatile unsigned long long*>(&state[2]);
-      ++spins;
-    }
-    s_skip = d >= (unsigned long long)n_tiles ? 0 : 1;
-    if (s_skip) atomicExch(reinterpret_cast<unsigned long long*>(&state[1]), 1ull);
+    if (moved)
+      atomicMax(reinterpret_cast<unsigned long long*>(work.disp),
+                (unsigned long long)__double_as_longlong(far));
+    if (t < n_tiles) work.base[t] = sum;
+    // (the CTA's writes, ordered before this by the barrier, are released
+    // with it)
     __threadfence();
-  }
-  __syncthreads();
-  if (!s_skip) {
-    const int64_t total = (int64_t)*reinterpret_cast<volatile uint64_t*>(&state[3]);
-    for (int64_t k = (int64_t)blockIdx.x * kVcThreads + tid; k < total;
-         k += (int64_t)gridDim.x * kVcThreads)
-      out_ei[total + k] = (int64_t)__ldcg(&dst_tmp[k]);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_skip = atomicAdd(reinterpret_cast<unsigned long long*>(&state[4]), 1ull) ==
+    s_last = atomicAdd(reinterpret_cast<unsigned long long*>(work.done), 1ull) ==
              (unsigned long long)gridDim.x - 1ull;
     __threadfence();
   }
   __syncthreads();
-  if (!s_skip) return;
-  // The last CTA: every other one has ended.
-  volatile uint64_t* st = state;
-  const uint64_t kept = st[3], err = st[1], far = st[5];
+  if (!s_last) return;
+  // Thread k takes the k-th run of tiles: its sum, the sums before it, and the
+  // tiles' first slots.
+  const int64_t per = (n_tiles + kVcThreads - 1) / kVcThreads;
+  const int64_t b0 = tid * per < n_tiles ? tid * per : n_tiles;
+  const int64_t b1 = b0 + per < n_tiles ? b0 + per : n_tiles;
+  int64_t mine = 0;
+#pragma unroll 4
+  for (int64_t k = b0; k < b1; ++k) mine += __ldcg(&work.base[k]);
+  int64_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
-  for (int64_t k = tid; k < 6 + n_tiles; k += kVcThreads) state[k] = 0;
-  __syncthreads();
+  int64_t slot = incl - mine, total = 0;
+#pragma unroll
+  for (int w = 0; w < kVcThreads / 32; ++w) {
+    slot += w < warp ? warp_sum[w] : 0;
+    total += warp_sum[w];
+  }
+#pragma unroll 4
+  for (int64_t k = b0; k < b1; ++k) {
+    const int64_t c = __ldcg(&work.base[k]);
+    work.base[k] = slot;
+    slot += c;
+  }
   if (tid == 0) {
-    __threadfence();
+    *work.total = total;
     volatile int64_t* r = report;
-    r[1] = (int64_t)kept;
-    r[2] = (int64_t)err;
-    r[3] = (int64_t)far;
+    r[1] = total;
+    r[2] = 0;
+    r[3] = (int64_t) * reinterpret_cast<volatile uint64_t*>(work.disp);
+    *work.done = 0;
+    *work.disp = 0;
     __threadfence_system();
     r[0] = 1;
+  }
+}
+
+// Its second launch: the kept edges, in stored order, a CTA per tile.
+__global__ void __launch_bounds__(kVcThreads)
+    k_verlet_write(const __grid_constant__ VerletEdges list,
+                   const __grid_constant__ VerletWork work, int64_t* __restrict__ out_ei,
+                   int32_t* __restrict__ out_sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_wait();
+  const int64_t t = blockIdx.x;
+  const bool wide = *list.wide != 0;
+  const int64_t M = *work.total;
+  int64_t o0 = work.base[t];
+  // the run's mask words, and the kept edges of the runs before it
+  static_assert(kVcWords == 64, "two words a lane");
+  const uint32_t w0 = work.masks[t * kVcWords + lane], w1 = work.masks[t * kVcWords + 32 + lane];
+  const int first = warp * kVcPer;
+  o0 += __reduce_add_sync(0xffffffffu, (lane < first ? __popc(w0) : 0) +
+                                           (lane + 32 < first ? __popc(w1) : 0));
+  const int64_t wbase = t * kVcTile + (int64_t)first * 32;
+  uint32_t mask[kVcPer];
+  int2 ij[kVcPer];
+  uint32_t psh[kVcPer];
+#pragma unroll
+  for (int k = 0; k < kVcPer; ++k) {
+    mask[k] = __shfl_sync(0xffffffffu, first < 32 ? w0 : w1, (first + k) & 31);
+    if ((mask[k] >> lane) & 1u) {
+      ij[k] = list.ij[wbase + 32 * k + lane];
+      psh[k] = list.packed[wbase + 32 * k + lane];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kVcPer; ++k) {
+    if ((mask[k] >> lane) & 1u) {
+      const int64_t o = o0 + __popc(mask[k] & ((1u << lane) - 1u));
+      int32_t s[3];
+      edge_shift(list, wide, wbase + 32 * k + lane, psh[k], s);
+      out_ei[o] = (int64_t)ij[k].x;
+      out_ei[M + o] = (int64_t)ij[k].y;
+      out_sh[3 * o] = s[0];
+      out_sh[3 * o + 1] = s[1];
+      out_sh[3 * o + 2] = s[2];
+    }
+    o0 += __popc(mask[k]);
   }
 }
 
@@ -328,33 +290,23 @@ void launch_verlet_pack(const int64_t* ei, const int32_t* sh, int64_t m, int2* i
   note_launches(1);
 }
 
-int64_t verlet_compact_state_words(int64_t m) { return 6 + (m + kVcTile - 1) / kVcTile; }
+int64_t verlet_tiles(int64_t m) { return (m + kVcTile - 1) / kVcTile; }
+int64_t verlet_mask_words(int64_t m) { return verlet_tiles(m) * kVcWords; }
 
-void launch_verlet_compact(const double* pos, const double* ref, int64_t n,
-                           const EdgeExtrasCell& cell, const VerletEdges& list, double rc_sq,
-                           int64_t* out_ei, int32_t* out_sh, int32_t* dst_tmp, uint64_t* state,
-                           int32_t spin_limit, int64_t* report, cudaStream_t s) {
-  // (SMs and resident CTAs per SM of each device, looked up once)
-  static std::atomic<int> cached[64][2];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const bool known = dev >= 0 && dev < 64;
-  int sms = known ? cached[dev][0].load() : 0, per_sm = known ? cached[dev][1].load() : 0;
-  if (sms <= 0 || per_sm <= 0) {
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_verlet_compact, kVcThreads, 0);
-    sms = std::max(sms, 1);
-    per_sm = std::max(per_sm, 1);
-    if (known) {
-      cached[dev][0].store(sms);
-      cached[dev][1].store(per_sm);
-    }
-  }
-  const int64_t n_tiles = (list.m + kVcTile - 1) / kVcTile;
-  const int64_t grid = std::min<int64_t>((int64_t)sms * per_sm, std::max<int64_t>(n_tiles, sms));
-  k_verlet_compact<<<(unsigned)grid, kVcThreads, 0, s>>>(pos, ref, n, cell, list, rc_sq, out_ei,
-                                                         out_sh, dst_tmp, state, spin_limit,
-                                                         report);
+void launch_verlet_update(const double* pos, const double* ref, int64_t n,
+                          const EdgeExtrasCell& cell, const VerletEdges& list, double rc_sq,
+                          const VerletWork& work, int64_t* out_ei, int32_t* out_sh,
+                          int64_t* report, cudaStream_t s) {
+  const int64_t n_tiles = verlet_tiles(list.m);
+  // (with few stored edges, a CTA per SM at most for the displacements)
+  const int64_t moves = std::min<int64_t>((n + kVcThreads - 1) / kVcThreads, 148);
+  const int64_t grid = std::max<int64_t>({n_tiles, moves, 1});
+  launch_pdl(k_verlet_count, dim3((unsigned)grid), dim3(kVcThreads), 0, s, pos, ref, n, cell, list,
+             rc_sq, work, report);
+  note_launches(1);
+  if (n_tiles == 0) return;
+  launch_pdl(k_verlet_write, dim3((unsigned)n_tiles), dim3(kVcThreads), 0, s, list, work, out_ei,
+             out_sh);
   note_launches(1);
 }
 

@@ -450,16 +450,26 @@ struct VerletEdges {
 };
 void launch_verlet_pack(const int64_t* ei, const int32_t* sh, int64_t m, int2* ij,
                         uint32_t* packed, int32_t* plain, int32_t* wide, cudaStream_t s);
-// One update (k_verlet_compact): the kept edges, out_ei [src | dst] of M edges
-// and out_sh; dst_tmp has room for list.m destinations; state has
-// verlet_compact_state_words(list.m) words, zero on entry and zero again
-// afterwards.  report (host-mapped): [1] M, [2] the look-back's error word,
-// [3] the bits of the largest squared displacement, then [0] = 1 when all is
-// written.
-int64_t verlet_compact_state_words(int64_t m);
-void launch_verlet_compact(const double* pos, const double* ref, int64_t n,
-                           const EdgeExtrasCell& cell, const VerletEdges& list, double rc_sq,
-                           int64_t* out_ei, int32_t* out_sh, int32_t* dst_tmp, uint64_t* state,
-                           int32_t spin_limit, int64_t* report, cudaStream_t s);
+// Work arrays of an update (done and disp zero before the first one, left
+// zero): CTAs done, bits of the largest squared displacement, M, each tile's
+// kept edges and then first slot [verlet_tiles], and a bit per stored edge
+// [verlet_mask_words].
+struct VerletWork {
+  uint64_t* done;
+  uint64_t* disp;
+  int64_t* total;
+  int64_t* base;
+  uint32_t* masks;
+};
+int64_t verlet_tiles(int64_t m);
+int64_t verlet_mask_words(int64_t m);
+// One update: the kept edges, out_ei [src | dst] of M edges and out_sh.
+// report (host-mapped): [1] M, [2] 0, [3] the bits of the largest squared
+// displacement, then [0] = 1, when they are known (the edges follow on the
+// stream; they read list and work, not pos).
+void launch_verlet_update(const double* pos, const double* ref, int64_t n,
+                          const EdgeExtrasCell& cell, const VerletEdges& list, double rc_sq,
+                          const VerletWork& work, int64_t* out_ei, int32_t* out_sh,
+                          int64_t* report, cudaStream_t s);
 
 }  // namespace nlb

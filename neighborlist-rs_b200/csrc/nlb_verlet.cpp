@@ -28,9 +28,6 @@
 
 namespace nlb {
 
-// Polls of one look-back wait in the Verlet compaction before it gives up.
-constexpr int32_t kVerletSpinLimit = 1 << 22;
-
 // Search pieces shared with nlb_api.cpp.
 Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int64_t n,
                         const double* cell9, const uint8_t* pbc, double cutoff, int64_t** ei,
@@ -66,12 +63,20 @@ struct DevBuf {
 class Verlet {
  public:
   Verlet(double rc, double skin) : rc_(rc), skin_(skin) {}
+  ~Verlet() {
+    if (written_) {
+      cudaEventSynchronize(written_);
+      cudaEventDestroy(written_);
+    }
+  }
 
   // Device positions (d_pos) are used in place; host positions are uploaded
-  // first.  Results stay in the manager's buffers until the next update.
+  // first.  Results stay in the manager's buffers until the next update.  On
+  // a caller's stream, and with stream_ordered on the library's own, the call
+  // returns when their size is known: they are complete in the stream's order.
   Status update(const double* pos_host, const double* d_pos_in, int64_t n, const double* cell9,
                 const uint8_t* pbc, int* rebuilt, int64_t* m_out, int64_t** ei_out,
-                int32_t** sh_out, bool owned = false) {
+                int32_t** sh_out, bool owned, bool stream_ordered) {
     std::lock_guard<std::mutex> lk(mu_);
     *rebuilt = 0;
     *m_out = 0;
@@ -83,6 +88,11 @@ class Verlet {
     Status st = get_ctx(&c);
     if (!st.ok()) return st;
     cudaStream_t s = c->stream;
+    // (the last update may still be writing its edges, on another stream)
+    if (written_) {
+      const cudaError_t e = cudaStreamWaitEvent(s, written_, 0);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent");
+    }
     const double* d_pos = d_pos_in;
     if (n > 0 && pos_host) {
       double* up = static_cast<double*>(pos_up_.get(24 * (size_t)n));
@@ -97,7 +107,7 @@ class Verlet {
       // (one launch takes the displacement and filters the stored list; a
       // rebuild, when due, discards the filter)
       double d2 = 0.0;
-      st = filter(*c, d_pos, m_out, ei_out, sh_out, owned, &d2);
+      st = filter(*c, d_pos, m_out, ei_out, sh_out, owned, stream_ordered, &d2);
       if (!st.ok()) return st;
       last_disp_ = std::sqrt(d2);
       rebuild = last_disp_ > 0.5 * skin_;
@@ -119,7 +129,7 @@ class Verlet {
       *rebuilt = 1;
       ++rebuilds_;
     }
-    return filter(*c, d_pos, m_out, ei_out, sh_out, owned);
+    return filter(*c, d_pos, m_out, ei_out, sh_out, owned, stream_ordered);
   }
 
   // Largest displacement since the last rebuild (+inf when there is no list
@@ -227,7 +237,7 @@ class Verlet {
   // owned: the kept edges go to blocks of the result pool sized for the
   // whole stored list, handed to the caller (released again on failure).
   Status filter(Ctx& c, const double* d_pos, int64_t* m_out, int64_t** ei_out,
-                int32_t** sh_out, bool owned = false, double* disp_sq = nullptr) {
+                int32_t** sh_out, bool owned, bool stream_ordered, double* disp_sq = nullptr) {
     const int64_t m = m_list_;
     int64_t* out_ei = nullptr;
     int32_t* out_sh = nullptr;
@@ -246,11 +256,15 @@ class Verlet {
       out_sh = static_cast<int32_t*>(out_sh_.get(12 * (size_t)m));
       if (!out_ei || !out_sh) return fail(NLB_ERR_NOMEM, "device allocation failed");
     }
-    int32_t* dst_tmp = static_cast<int32_t*>(dst_tmp_.get(4 * (size_t)m));
-    const size_t state_bytes = 8 * (size_t)verlet_compact_state_words(m);
+    // [done, disp, total, tile bases] and the masks
     const size_t state_cap = state_.cap;
-    uint64_t* state = static_cast<uint64_t*>(state_.get(state_bytes));
-    if (!dst_tmp || !state) {
+    uint64_t* state = static_cast<uint64_t*>(state_.get(8 * (size_t)(3 + verlet_tiles(m))));
+    uint32_t* masks = static_cast<uint32_t*>(masks_.get(4 * (size_t)verlet_mask_words(m)));
+    if (!written_ && cudaEventCreateWithFlags(&written_, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      written_ = nullptr;
+    }
+    if (!state || !masks || !written_) {
       if (owned) {
         release_owned_device(out_ei, c.stream);
         release_owned_device(out_sh, c.stream);
@@ -274,25 +288,33 @@ class Verlet {
     list.plain = static_cast<const int32_t*>(list_plain_.p);
     list.wide = static_cast<const int32_t*>(list_wide_.p);
     list.m = m;
-    // (the launch leaves the state cleared; a new or a failed one is not)
-    if (!state_clean_ || state_.cap != state_cap)
-      cudaMemsetAsync(state, 0, state_.cap, c.stream);
+    // (the launch leaves the counters cleared; new ones and a failed launch's
+    // are not)
+    if (!state_clean_ || state_.cap != state_cap) cudaMemsetAsync(state, 0, 16, c.stream);
     state_clean_ = false;
+    VerletWork work;
+    work.done = state;
+    work.disp = state + 1;
+    work.total = reinterpret_cast<int64_t*>(state + 2);
+    work.base = work.total + 1;
+    work.masks = masks;
     c.h_report[0] = 0;
-    launch_verlet_compact(d_pos, static_cast<const double*>(ref_.p), n_, cell, list, rc_ * rc_,
-                          out_ei, out_sh, dst_tmp, state, kVerletSpinLimit, c.d_report, c.stream);
-    // (reported when everything is written: no other synchronisation)
+    launch_verlet_update(d_pos, static_cast<const double*>(ref_.p), n_, cell, list, rc_ * rc_, work,
+                         out_ei, out_sh, c.d_report, c.stream);
+    cudaError_t e = cudaEventRecord(written_, c.stream);
     Status st = wait_report(c);
     const volatile int64_t* r = c.h_report;
-    if (!st.ok() || r[2] != 0) {
+    if (st.ok() && e == cudaSuccess && !stream_ordered && c.stream == c.own_stream)
+      e = cudaStreamSynchronize(c.stream);
+    if (st.ok() && e != cudaSuccess) st = cuda_fail(e, "Verlet update");
+    if (!st.ok()) {
       if (owned) {
         release_owned_device(out_ei, c.stream);
         release_owned_device(out_sh, c.stream);
-        *ei_out = nullptr;
-        *sh_out = nullptr;
       }
-      if (!st.ok()) return st;
-      return fail(NLB_ERR_CUDA, "prefix scan gave up waiting for a tile");
+      *ei_out = nullptr;
+      *sh_out = nullptr;
+      return st;
     }
     state_clean_ = true;
     if (disp_sq) {
@@ -315,8 +337,9 @@ class Verlet {
   int64_t updates_ = 0, rebuilds_ = 0;
   double last_disp_ = 0.0;
   bool state_clean_ = false;
+  cudaEvent_t written_ = nullptr;  // the last update's edges are written
   DevBuf pos_up_, ref_, disp_, list_ij_, list_packed_, list_plain_, list_wide_, out_ei_, out_sh_,
-      dst_tmp_, state_;
+      masks_, state_;
 };
 
 }  // namespace nlb
@@ -355,7 +378,7 @@ int nlb_verlet_update(nlb_verlet* v, const double* positions, int64_t n_atoms, c
   int32_t* sh = nullptr;
   static const double kNone = 0.0;
   nlb::Status st = v->impl->update(positions ? positions : &kNone, nullptr, n_atoms, cell, pbc,
-                                   rebuilt, &m, &ei, &sh);
+                                   rebuilt, &m, &ei, &sh, false, true);
   if (!st.ok()) return st.code;
   st = nlb::alloc_result(m, out);
   if (!st.ok()) return st.code;
@@ -389,7 +412,7 @@ int nlb_verlet_update_device(nlb_verlet* v, const double* d_positions, int64_t n
   int32_t* sh = nullptr;
   static const double kNone = 0.0;
   nlb::Status st = v->impl->update(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell,
-                                   pbc, rebuilt, &m, &ei, &sh);
+                                   pbc, rebuilt, &m, &ei, &sh, false, false);
   if (!st.ok()) return st.code;
   out->n_edges = m;
   out->edge_index = ei;
@@ -410,7 +433,7 @@ int nlb_verlet_update_device_owned(nlb_verlet* v, const double* d_positions, int
   int32_t* sh = nullptr;
   static const double kNone = 0.0;
   nlb::Status st = v->impl->update(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell,
-                                   pbc, rebuilt, &m, &ei, &sh, true);
+                                   pbc, rebuilt, &m, &ei, &sh, true, false);
   if (!st.ok()) return st.code;
   if (m == 0) {
     // (blocks sized for a non-empty stored list, but nothing was kept)
