@@ -6,16 +6,22 @@
 //   k_rank_table : Morton rank of every bin, counted analytically (no sort):
 //                  rank(c) = #grid points whose 63-bit Morton code is < code(c).
 //   k_prep       : per atom: fraction, wrap, Morton key, bin rank, bin histogram.
-//   (scan)       : bin histogram -> bin starts.
+//   (scan)       : bin histogram -> bin starts: k_prep's last CTA on grids of
+//                  up to kPrepBinScanMax bins, k_bin_scan on larger ones.
 //   k_scatter    : atoms -> bin segments (arbitrary order inside a segment).
 //   k_place      : every atom to its slot (wrapped positions, wrap shifts,
 //                  original indices, packed FP32 positions, group records):
-//                  in bins of at most kRankSortMax atoms kPlaceSplit threads
-//                  per atom count the bin's (key, index) pairs below its own
-//                  (rank sort); larger bins are sorted by one CTA each -- bitonic in
-//                  shared memory up to kSortCap, merge path through global
-//                  scratch above it.
-//   k_chunk_box  : bounding box of each 32-atom chunk (dense grids only).
+//                  in bins of at most kRankSortMax atoms SPLIT threads (1 or
+//                  8) per atom count the bin's (key, index) pairs below its
+//                  own (rank sort); larger bins are sorted by one CTA each --
+//                  bitonic in shared memory up to kSortCap, merge path through
+//                  global scratch above it.
+//   k_chunk_box  : bounding box of each 32-atom chunk (dense grids of the
+//                  three-launch pipeline only).
+// Small systems (bucket_build) take two launches instead of three or four:
+//   k_prep_bucket  : per atom as k_prep, and its entry straight into its bin's
+//                    bucket;
+//   k_place_bucket : the histogram's scan (by every CTA) and the placement.
 #include "nlb_kernels.h"
 
 namespace nlb {

@@ -41,7 +41,14 @@
 // edges): count 123 us, 65 % of issue slots, 7,500 instructions per group of
 // which 4,400 the pair tests; emit 112 us against 55 us for writing the same
 // bytes from registers.  A million atoms: 2,110 -> 874 us per call, against
-// one launch that counted, waited for its offsets and moved the destinations.
+// one launch that counted, waited for its offsets and moved the destinations
+// (795 with the later changes to loads and segments: count 366, emit 352; the
+// output alone takes 173 us to fill).  The emit is bound by latency and issue
+// (49 % of slots, 20 warps an SM by shared memory; with the candidates packed
+// to four bytes 25 warps and 323 us) rather than by its stores:
+// shifts written as whole sectors, three words a lane exchanged by shuffles
+// (36 -> 12 sector writes per 32 edges), cost 372 us, and masks kept in
+// registers for more warps 375.
 //
 // Candidates on the lanes rather than atoms: bins hold 20-25 atoms at the
 // usual densities, so a third of atom lanes would idle, while the ring keeps
@@ -66,7 +73,6 @@ namespace {
 constexpr int kGThreads = 32;
 constexpr int kGRing = 64;     // candidates waiting per warp
 constexpr int kGWindow = 16;   // records expanded per emit window
-constexpr int kGStage = 1536;  // hits staged per emit window (>= one record's 1024)
 
 // A block's word: the sum of its groups' totals, and above it their number.
 constexpr int kGCountShift = 48;
@@ -695,11 +701,13 @@ __global__ void __launch_bounds__(kGThreads, 28)
 // Shared memory of one warp of the emit pass.
 struct GEmitWarp {
   uint32_t mask[32 * kGWindow];  // the window's records: hit masks
-  int2 cand[32 * kGWindow];      // and candidates {wrap + image shift (packed), original index}
+  // and candidates: original index, and wrap + image shift in the bits above
+  uint32_t cand[32 * kGWindow];
   SlotMeta meta[32];             // the group's atoms
   int64_t slot[32];              // atom's next output slot minus its place in the stage
-  uint16_t hits[kGStage];        // atom << 10 | candidate of the window, in output order
 };
+// (behind it: uint16_t hits[GroupOut::stage], atom << 10 | candidate, in output
+// order)
 static_assert(sizeof(GEmitWarp) % 16 == 0 && 32 * kGWindow <= 1024, "vector accesses, 10-bit entries");
 
 __device__ __forceinline__ void copy16(void* smem, const void* global) {
@@ -720,6 +728,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
   extern __shared__ __align__(16) unsigned char gsm[];
   const int lane = threadIdx.x;
   GEmitWarp& w_sm = *reinterpret_cast<GEmitWarp*>(gsm);
+  uint16_t* const hits = reinterpret_cast<uint16_t*>(&w_sm + 1);
   pdl_wait();
   const int32_t split = o.split;
   const int64_t item = blockIdx.x;
@@ -752,12 +761,21 @@ __global__ void __launch_bounds__(kGThreads, 28)
   for (int s = 16; s > 0; s >>= 1) base += __shfl_xor_sync(0xffffffffu, base, s);
   slot += base;
 
+  // A candidate's original index takes orig_bits, each component of its shift a
+  // third of the rest (2 bits at the most atoms, 6 at 10,000).
+  const int s_bits = (32 - out.orig_bits) / 3;
+  const int32_t s_half = 1 << (s_bits - 1);
+  const uint32_t s_mask = (1u << s_bits) - 1u, orig_mask = (1u << out.orig_bits) - 1u;
+  const int down = 32 - s_bits;
+  const int up[3] = {down - out.orig_bits, down - out.orig_bits - s_bits,
+                     down - out.orig_bits - 2 * s_bits};
+
   for (int r0 = 0; r0 < n_rec;) {
     // A window of up to kGWindow records whose hits fit the stage.
     const int n_load = n_rec - r0 < kGWindow ? n_rec - r0 : kGWindow;
     const int64_t at = (first_rec + r0) * 32;
     for (int k = lane; k < 8 * n_load; k += 32) copy16(&w_sm.mask[4 * k], &o.masks[at + 4 * k]);
-    // (the shifts of the window's candidates, packed when all fit 10 bits)
+    // (the shifts of the window's candidates, packed when all fit)
     bool wide = false;
 #pragma unroll 4
     for (int c = 0; c < n_load; ++c) {
@@ -766,12 +784,12 @@ __global__ void __launch_bounds__(kGThreads, 28)
       const SlotMeta mj = b.meta[w & 0x7fffffffu];
       const int32_t s0 = mj.sx + unpack_shift(csh, 0), s1 = mj.sy + unpack_shift(csh, 1),
                     s2 = mj.sz + unpack_shift(csh, 2);
-      wide = wide || (uint32_t)(s0 + 512) > 1023u || (uint32_t)(s1 + 512) > 1023u ||
-             (uint32_t)(s2 + 512) > 1023u;
-      w_sm.cand[32 * c + lane] = make_int2(
-          (int32_t)(((uint32_t)s0 & 1023u) | ((uint32_t)s1 & 1023u) << 10 |
-                    ((uint32_t)s2 & 1023u) << 20),
-          mj.orig);
+      wide = wide || (uint32_t)(s0 + s_half) > s_mask || (uint32_t)(s1 + s_half) > s_mask ||
+             (uint32_t)(s2 + s_half) > s_mask;
+      w_sm.cand[32 * c + lane] =
+          (uint32_t)mj.orig | (((uint32_t)s0 & s_mask) | ((uint32_t)s1 & s_mask) << s_bits |
+                               ((uint32_t)s2 & s_mask) << (2 * s_bits))
+                                  << out.orig_bits;
     }
     wide = __any_sync(0xffffffffu, wide);
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -780,7 +798,7 @@ __global__ void __launch_bounds__(kGThreads, 28)
     for (; n_win < n_load; ++n_win) {
       const int k = __popc(w_sm.mask[32 * n_win + lane]);
       const int sum = __reduce_add_sync(0xffffffffu, k);
-      if (total + sum > kGStage) break;
+      if (total + sum > out.stage) break;
       total += sum;
       mine += k;
     }
@@ -797,19 +815,19 @@ __global__ void __launch_bounds__(kGThreads, 28)
       uint32_t h = w_sm.mask[32 * c + lane];
       const uint32_t entry = (uint32_t)lane << 10 | (uint32_t)c << 5;
       while (h) {
-        w_sm.hits[pre++] = (uint16_t)(entry | (uint32_t)(__ffs(h) - 1));
+        hits[pre++] = (uint16_t)(entry | (uint32_t)(__ffs(h) - 1));
         h &= h - 1;
       }
     }
     __syncwarp();
 #pragma unroll 2
     for (int k = lane; k < total; k += 32) {
-      const uint32_t v = w_sm.hits[k];
-      const int2 cj = w_sm.cand[v & 1023u];
+      const uint32_t v = hits[k];
+      const uint32_t cj = w_sm.cand[v & 1023u];
       const SlotMeta ml = w_sm.meta[v >> 10];
       const int64_t e = w_sm.slot[v >> 10] + k;
-      int32_t s0 = unpack_shift((uint32_t)cj.x, 0), s1 = unpack_shift((uint32_t)cj.x, 1),
-              s2 = unpack_shift((uint32_t)cj.x, 2);
+      int32_t s0 = (int32_t)(cj << up[0]) >> down, s1 = (int32_t)(cj << up[1]) >> down,
+              s2 = (int32_t)(cj << up[2]) >> down;
       if (wide) {
         const uint32_t w = o.cand[at + (v & 1023u)];
         const uint32_t csh = w >> 31 ? o.cshift[at + (v & 1023u)] : 0u;
@@ -818,7 +836,8 @@ __global__ void __launch_bounds__(kGThreads, 28)
         s1 = mj.sy + unpack_shift(csh, 1);
         s2 = mj.sz + unpack_shift(csh, 2);
       }
-      write_edge<EX>(out, d_ei, M, e, ml.orig, cj.y, s0 - ml.sx, s1 - ml.sy, s2 - ml.sz);
+      write_edge<EX>(out, d_ei, M, e, ml.orig, (int32_t)(cj & orig_mask), s0 - ml.sx, s1 - ml.sy,
+                     s2 - ml.sz);
     }
     __syncwarp();
     r0 += n_win;
@@ -858,8 +877,8 @@ void launch_group_emit(const GridParams& g, const GridBuffers& b, int32_t n_cell
                        const GroupBand& band, const GroupSearch& o, const GroupOut& out,
                        cudaStream_t s) {
   const auto k = out.directed || out.vec || out.dist ? &k_group_emit<true> : &k_group_emit<false>;
-  launch_pdl(k, dim3((unsigned)(o.max_groups * o.split)), dim3(kGThreads), sizeof(GEmitWarp), s, g,
-             b, n_cells, band.rc_sq, o, out);
+  launch_pdl(k, dim3((unsigned)(o.max_groups * o.split)), dim3(kGThreads),
+             sizeof(GEmitWarp) + 2 * (size_t)out.stage, s, g, b, n_cells, band.rc_sq, o, out);
   note_launches(1);
 }
 

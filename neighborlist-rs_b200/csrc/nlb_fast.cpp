@@ -252,6 +252,22 @@ int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
   return (int32_t)std::max<int64_t>(want, 1);
 }
 
+// Hits the emit pass stages at a time.  A segment whose records hold more is
+// written in several windows, each with its own loads and scan; a larger stage
+// leaves fewer warps on an SM (25 with 1536 hits, 16 with 4096).  The small one
+// is for long launches of groups whose hits fit it: a million atoms at rc 6
+// 763 us, 836 with the large one, 300,000 276 and 293; the large one for the
+// rest: 400,000 atoms at rc 8 895 -> 774 us, 78,000 at rc 14 891 -> 760 (712
+// with 6144, but 100,000 at rc 6 137 -> 146), 10,008 at rc 14 158 -> 145, 30,000
+// at rc 8 113 -> 108, 40,000 at rc 6 84 -> 83; 2048 and 3072 are in between.
+constexpr int32_t kStageSmall = 1536, kStageLarge = 4096;
+constexpr int64_t kStageFew = 20000;  // segments
+int32_t group_stage(const SystemPlan& sp) {
+  const double hits = 32.0 * (double)estimate_edges(sp, std::sqrt(sp.rc_sq[0])) / (double)sp.n;
+  const int64_t items = sp.search.max_groups * sp.search.split;
+  return items > kStageFew && hits <= 2048.0 ? kStageSmall : kStageLarge;
+}
+
 // The group search's two launches.
 void issue_search(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t capacity, bool count) {
   const GroupBand band = group_band(sp.band);
@@ -278,6 +294,9 @@ void issue_search(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t capacity,
   out.cell = sp.ex_cell;
   out.capacity = capacity;
   out.directed = sp.ex_flags & NLB_DIRECTED ? 1 : 0;
+  out.stage = group_stage(sp);
+  out.orig_bits = 2;
+  while (((int64_t)1 << out.orig_bits) < sp.n) ++out.orig_bits;
   launch_group_emit(sp.grid, sp.gb, cells, band, sp.search, out, c.stream);
 }
 

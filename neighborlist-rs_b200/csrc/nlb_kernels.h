@@ -268,6 +268,8 @@ struct GroupOut {
   EdgeExtrasCell cell;
   int64_t capacity;
   int32_t directed;
+  int32_t orig_bits;  // bits of the largest atom index, at most 26 and at least 2
+  int32_t stage;      // hits staged per window: at least a record's 1024, a multiple of 8
 };
 void launch_group_emit(const GridParams& g, const GridBuffers& b, int32_t n_cells,
                        const GroupBand& band, const GroupSearch& o, const GroupOut& out,

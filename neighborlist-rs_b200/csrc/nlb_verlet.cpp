@@ -4,7 +4,7 @@
 // r_list = r_cut + r_skin, reference positions, rebuild when
 // max_i |r_i - r_i,ref| > r_skin / 2, update / needs_rebuild / get); the
 // reference does not implement it.  Each update:
-//   1. if a list exists for the same atom count, cell and pbc, one launch
+//   1. if a list exists for the same atom count, cell and pbc, a count pass
 //      takes the largest displacement since the last rebuild and filters the
 //      stored list with the current positions at rc, in stored order;
 //   2. if there is no list, the system changed, or that displacement is
@@ -104,8 +104,8 @@ class Verlet {
     ++updates_;
     bool rebuild = !same_system(n, cell9, pbc);
     if (!rebuild && n > 0) {
-      // (one launch takes the displacement and filters the stored list; a
-      // rebuild, when due, discards the filter)
+      // (the displacement and the filter go out together; a rebuild, when due,
+      // discards the filter)
       double d2 = 0.0;
       st = filter(*c, d_pos, m_out, ei_out, sh_out, owned, stream_ordered, &d2);
       if (!st.ok()) return st;
