@@ -680,7 +680,9 @@ def build_neighborlists_torch(cell, positions, cutoff, directed=False, vectors=F
     """GPU-resident variant of build_neighborlists for torch pipelines:
     ``positions`` is a CUDA float64 tensor (N, 3); returns
     {"edge_index": int64 (2, M), "shift": int32 (M, 3)} as CUDA tensors on the
-    same device, produced on the current torch stream.  The tensors are the
+    same device, produced on the current torch stream: the call returns when
+    the list's size is known, the tensors are complete in that stream's order,
+    and work on another stream waits for it.  The tensors are the
     library's result blocks themselves (zero-copy: the build writes them in
     place and hands them over; they return to the library's pool when the
     tensors are freed, ordered on the stream that was current for the build,
