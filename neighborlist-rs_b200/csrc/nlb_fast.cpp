@@ -255,7 +255,9 @@ int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
 // Hits the emit pass stages at a time.  A segment whose records hold more is
 // written in several windows, each with its own loads and scan; a larger stage
 // leaves fewer warps on an SM (25 with 1536 hits, 16 with 4096).  The small one
-// is for long launches of groups whose hits fit it: a million atoms at rc 6
+// is for segments so short that they cannot hold much more (10,008 atoms at
+// rc 6, 5,000 short slices: 54.5 us, 56 to 58 with the large one), and for long launches of groups
+// whose hits fit it: a million atoms at rc 6
 // 763 us, 836 with the large one, 300,000 276 and 293; the large one for the
 // rest: 400,000 atoms at rc 8 895 -> 774 us, 78,000 at rc 14 891 -> 760 (712
 // with 6144, but 100,000 at rc 6 137 -> 146), 10,008 at rc 14 158 -> 145, 30,000
@@ -265,6 +267,9 @@ constexpr int64_t kStageFew = 20000;  // segments
 int32_t group_stage(const SystemPlan& sp) {
   const double hits = 32.0 * (double)estimate_edges(sp, std::sqrt(sp.rc_sq[0])) / (double)sp.n;
   const int64_t items = sp.search.max_groups * sp.search.split;
+  const double slice = (double)stencil_cells_of(sp.grid) * (double)sp.n /
+                       ((double)sp.grid.total_bins * (double)sp.search.split);
+  if (32.0 * slice <= 2.0 * kStageSmall) return kStageSmall;
   return items > kStageFew && hits <= 2048.0 ? kStageSmall : kStageLarge;
 }
 
