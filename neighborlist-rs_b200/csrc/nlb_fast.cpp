@@ -44,6 +44,10 @@ struct FastKey {
   int32_t split;  // segments per group (0: pair tasks)
   int32_t bucket;
   int32_t ex_flags;
+  // The output options' cell: the grid does not tell an auto-box, whose
+  // vectors have no H S term, from a cell with the same matrix.
+  int32_t ex_has_cell;
+  double ex_h[9];
 };
 
 struct FastState {
@@ -440,6 +444,8 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   key.split = sp.search.split;
   key.bucket = sp.gb.bucket;
   key.ex_flags = sp.ex_flags;
+  key.ex_has_cell = sp.ex_cell.has_cell;
+  std::memcpy(key.ex_h, sp.ex_cell.h, sizeof(key.ex_h));
 
   const bool report = !c.prof;
   if (report) c.h_report[0] = 0;
