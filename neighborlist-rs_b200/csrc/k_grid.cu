@@ -139,11 +139,12 @@ constexpr uint64_t kBinAggregate = 1ull << kBinShift;
 constexpr uint64_t kBinInclusive = 2ull << kBinShift;
 constexpr uint64_t kBinValue = (1ull << kBinShift) - 1;
 constexpr uint64_t kBinAtoms = (1ull << 31) - 1;
-constexpr int kBinSpins = 1 << 22;
+constexpr int32_t kBinSpins = 1 << 22;
 
 __global__ void __launch_bounds__(kPrepThreads)
     k_bin_scan(const int32_t* __restrict__ bin_count, int64_t nb, int64_t* __restrict__ bin_start,
-               int32_t* __restrict__ group_start, uint64_t* __restrict__ state) {
+               int32_t* __restrict__ group_start, uint64_t* __restrict__ state, int32_t withhold,
+               int32_t spin_limit) {
   __shared__ uint64_t warp_tot[kPrepThreads / 32];
   __shared__ uint64_t s_prefix;
   __shared__ int64_t s_tile;
@@ -176,7 +177,8 @@ __global__ void __launch_bounds__(kPrepThreads)
   }
   if (warp == 0) {
     volatile uint64_t* tiles = state + 2;
-    if (lane == 0) {
+    const bool publish = t != withhold;  // false only under the test hook
+    if (lane == 0 && publish) {
       __threadfence();
       tiles[t] = (t == 0 ? kBinInclusive : kBinAggregate) | all;
     }
@@ -185,9 +187,9 @@ __global__ void __launch_bounds__(kPrepThreads)
       const int64_t pred = tt - lane;
       uint64_t w = kBinInclusive;
       if (pred >= 0) {
-        int spins = 0;
+        int32_t spins = 0;
         w = tiles[pred];
-        while ((w >> kBinShift) == 0 && spins < kBinSpins) {
+        while ((w >> kBinShift) == 0 && spins < spin_limit) {
           __nanosleep(32);
           w = tiles[pred];
           ++spins;
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kPrepThreads)
       if (stop >= 0) break;
     }
     if (lane == 0) {
-      if (t > 0) {
+      if (t > 0 && publish) {
         __threadfence();
         tiles[t] = kBinInclusive | (prefix + all);
       }
@@ -264,11 +266,13 @@ __global__ void __launch_bounds__(kPrepThreads)
 __global__ void k_scatter(const uint64_t* __restrict__ key, const int32_t* __restrict__ rank,
                           int64_t n, const int64_t* __restrict__ bin_start,
                           int32_t* __restrict__ bin_fill, uint64_t* __restrict__ skey,
-                          int32_t* __restrict__ sidx, const int32_t* __restrict__ fill) {
+                          int32_t* __restrict__ sidx, const int32_t* __restrict__ fill,
+                          const int64_t* __restrict__ bad) {
   pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int32_t r = rank[i];
+  if (bad && *bad != 0) return;  // (starts not valid: slots could lie anywhere)
   const int64_t slot = bin_start[r] + (fill ? fill[i] : atomicAdd(&bin_fill[r], 1));
   skey[slot] = key[i];
   sidx[slot] = (int32_t)i;
@@ -540,10 +544,14 @@ __global__ void __launch_bounds__(kSortThreads)
             GroupRec* __restrict__ groups, int32_t* __restrict__ irr_list,
             uint8_t* __restrict__ irr, int32_t* __restrict__ counters,
             float4* __restrict__ cbox, const int32_t* __restrict__ group_start,
-            int32_t* __restrict__ loose, int32_t atom_blocks, int32_t bin_span) {
+            int32_t* __restrict__ loose, int32_t atom_blocks, int32_t bin_span,
+            const int64_t* __restrict__ bad) {
   __shared__ uint64_t sk[kSortCap];
   __shared__ int32_t sv[kSortCap];
   pdl_wait();
+  // (nothing was scattered then, and no group is made: the count pass finds
+  // no work)
+  if (bad && *bad != 0) return;
   if ((int32_t)blockIdx.x >= atom_blocks) {
     const int64_t r0 = (int64_t)(blockIdx.x - atom_blocks) * bin_span;
     const int64_t end = r0 + bin_span < g.total_bins ? r0 + bin_span : g.total_bins;
@@ -861,20 +869,24 @@ void launch_grid_build(const GridParams& g, const double* pos, int64_t n, const 
     return;
   }
   const bool own_scan = b.build_done != nullptr && g.total_bins <= kPrepBinScanMax;
+  const int64_t* bad = bin_scan_error(g, b);
   k_prep<<<(unsigned)((n + kPrepThreads - 1) / kPrepThreads), kPrepThreads, 0, s>>>(
       g, pos, n, b.rank_of_bin, b.key, b.rank, b.bin_count, b.bin_start,
       own_scan ? b.build_done : nullptr, own_scan ? b.group_start : nullptr, b.fill);
   if (!own_scan && b.group_start && b.bin_scan) {
-    launch_pdl(k_bin_scan, dim3((unsigned)((g.total_bins + kBinTile - 1) / kBinTile)),
-               dim3(kPrepThreads), 0, s, (const int32_t*)b.bin_count, g.total_bins, b.bin_start,
-               b.group_start, b.bin_scan);
+    const int64_t tiles = (g.total_bins + kBinTile - 1) / kBinTile;
+    int32_t withhold = -1, spins = kBinSpins;
+    take_scan_stall(&withhold, &spins, tiles);  // failure-detection hook
+    launch_pdl(k_bin_scan, dim3((unsigned)tiles), dim3(kPrepThreads), 0, s,
+               (const int32_t*)b.bin_count, g.total_bins, b.bin_start, b.group_start, b.bin_scan,
+               withhold, spins);
     note_launches(1);
   } else if (!own_scan) {
     exclusive_scan_i32(b.bin_count, g.total_bins, b.bin_start, b.scan_tmp, s);
   }
   const bool grouped = b.group_start && (own_scan || b.bin_scan);
   launch_pdl(k_scatter, dim3((unsigned)((n + T - 1) / T)), dim3(T), 0, s, b.key, b.rank, n,
-             b.bin_start, b.bin_fill, b.skey, b.sidx, (const int32_t*)b.fill);
+             b.bin_start, b.bin_fill, b.skey, b.sidx, (const int32_t*)b.fill, bad);
   const bool whole = n >= kPlaceWhole;
   const int64_t split = whole ? 1 : 8;
   const int32_t atom_blocks = (int32_t)((split * n + kSortThreads - 1) / kSortThreads);
@@ -884,7 +896,7 @@ void launch_grid_build(const GridParams& g, const double* pos, int64_t n, const 
              pos, n, (const int32_t*)b.rank, (const int64_t*)b.bin_start, b.skey, b.sidx, b.skey2,
              b.sidx2, b.px, b.py, b.pz, b.meta, b.p32, b.sbin, b.groups, b.irr_list, b.irr,
              b.counters, b.cbox, grouped ? (const int32_t*)b.group_start : nullptr, b.loose,
-             atom_blocks, (int32_t)span);
+             atom_blocks, (int32_t)span, bad);
   note_launches(3);
   if (b.p32 && b.cbox) {
     int dev = 0, sms = 0;

@@ -195,8 +195,8 @@ void scan_impl(const TIn* in, int64_t n, int64_t* out, int64_t* tmp, cudaStream_
 
 bool scan_stall_armed() { return tl_withhold_tile >= 0; }
 
-bool take_scan_stall(int32_t* tile, int32_t* spin_limit) {
-  if (tl_withhold_tile < 0) return false;
+bool take_scan_stall(int32_t* tile, int32_t* spin_limit, int64_t tiles) {
+  if (tl_withhold_tile < 0 || tl_withhold_tile >= tiles - 1) return false;
   *tile = tl_withhold_tile;
   *spin_limit = tl_withhold_spins;
   tl_withhold_tile = -1;

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_grid_count(GridParams g, GridBuffers b, int64_t n, CutoffSet cs, uint32_t* __restrict__ counts) {
   const int64_t p = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (p >= n) return;  // warp-uniform
+  const int64_t* bad = bin_scan_error(g, b);
+  if (bad && *bad != 0) return;  // bin starts not valid (the host reads the word too)
   CountSink sink{&cs, 0u};
   visit_grid_atom(g, b, p, cs.max_sq, sink);
   const int lane = threadIdx.x & 31;

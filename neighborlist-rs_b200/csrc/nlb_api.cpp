@@ -661,12 +661,11 @@ Status count_system(Ctx& c, SystemPlan& sp, const double* d_pos) {
   if (e == cudaSuccess && pair_tasks)  // hit-mask words the count pass asked for
     e = cudaMemcpyAsync(c.h_small + k + 2, sp.gb.mask_top, sizeof(int64_t),
                         cudaMemcpyDeviceToHost, s);
-  const bool bin_scan = sp.method == Method::kCellList &&
-                        !(sp.gb.build_done && sp.grid.total_bins <= kPrepBinScanMax);
+  const int64_t* bin_bad =
+      sp.method == Method::kCellList ? bin_scan_error(sp.grid, sp.gb) : nullptr;
   c.h_small[k + 3] = 0;
-  if (e == cudaSuccess && bin_scan)  // the separate bin scan's error word
-    e = cudaMemcpyAsync(c.h_small + k + 3, sp.gb.scan_tmp + 1, sizeof(int64_t),
-                        cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess && bin_bad)  // the separate bin scan's error word
+    e = cudaMemcpyAsync(c.h_small + k + 3, bin_bad, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy2DAsync");
   e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "count pass");

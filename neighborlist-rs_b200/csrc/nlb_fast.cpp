@@ -319,8 +319,7 @@ EmitTargets fast_targets(const SystemPlan& sp, int64_t capacity, int64_t* report
   t.scan_error = sp.scan_state + 1;
   t.report = report;
   t.mask_top = sp.gb.mask_top;
-  // (grids too large for k_prep's own bin scan: the separate scan's error word)
-  t.grid_scan_error = sp.grid.total_bins > kPrepBinScanMax ? sp.gb.scan_tmp + 1 : nullptr;
+  t.grid_scan_error = bin_scan_error(sp.grid, sp.gb);
   return t;
 }
 
@@ -544,11 +543,8 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   // Grids too large for k_prep's own bin scan use a separate scan (state in
   // gb.scan_tmp): its error word too.
   c.h_small[3] = 0;
-  if (e == cudaSuccess && sp.grid.total_bins > kPrepBinScanMax)
-    e = cudaMemcpyAsync(c.h_small + 3,
-                        sp.grouped ? reinterpret_cast<int64_t*>(sp.gb.bin_scan) + 1
-                                 : sp.gb.scan_tmp + 1,
-                        sizeof(int64_t), cudaMemcpyDeviceToHost, c.stream);
+  if (const int64_t* bad = bin_scan_error(sp.grid, sp.gb); e == cudaSuccess && bad)
+    e = cudaMemcpyAsync(c.h_small + 3, bad, sizeof(int64_t), cudaMemcpyDeviceToHost, c.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
   if (e != cudaSuccess) return cuda_fail(e, "neighbour-list pipeline");
   if (c.h_small[1] != 0 || c.h_small[3] != 0)

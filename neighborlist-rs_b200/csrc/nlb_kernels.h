@@ -19,9 +19,11 @@ int64_t scan_tmp_elems(int64_t n);
 // (then record the error word and finish).  One-shot.
 void arm_scan_stall(int32_t tile, int32_t spin_limit);
 bool scan_stall_armed();
-// Takes the armed hook for a launch that is not a scan (the group
-// search's scan of its blocks); false when none is armed.
-bool take_scan_stall(int32_t* tile, int32_t* spin_limit);
+// Takes the armed hook for a launch that is not k_scan (the bin scan over
+// several CTAs, the group search's scan of its blocks); false when none is
+// armed, or when its tile is not one that another of the launch's `tiles`
+// waits for.
+bool take_scan_stall(int32_t* tile, int32_t* spin_limit, int64_t tiles = INT64_MAX);
 void exclusive_scan_u32(const uint32_t* in, int64_t n, int64_t* out, int64_t* tmp,
                         cudaStream_t s);
 void exclusive_scan_i32(const int32_t* in, int64_t n, int64_t* out, int64_t* tmp,
@@ -132,6 +134,17 @@ constexpr double kChunkPruneMinPerBin = 64.0;
 // several CTAs.
 constexpr int64_t kPrepBinScanMax = 4096;
 int64_t bin_scan_words(int64_t total_bins);
+
+// The error word of the scan that writes bin_start for this build (set when a
+// bounded wait gave up; the starts are then not valid, and neither the build's
+// later kernels nor a count pass may use them); nullptr where no tile waits for
+// another (k_prep's and the bucket build's own scans).
+__host__ __device__ inline const int64_t* bin_scan_error(const GridParams& g,
+                                                         const GridBuffers& b) {
+  if (b.bucket > 0 || (b.build_done && g.total_bins <= kPrepBinScanMax)) return nullptr;
+  if (b.group_start && b.bin_scan) return reinterpret_cast<const int64_t*>(b.bin_scan) + 1;
+  return b.scan_tmp + 1;
+}
 
 // need_rank_table = false reuses rank_of_bin from a previous build with the
 // same bins per axis.
