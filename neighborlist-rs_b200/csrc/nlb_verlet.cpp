@@ -274,8 +274,12 @@ class Verlet {
     *ei_out = out_ei;
     *sh_out = out_sh;
     if (m == 0 && !disp_sq) {
+      // Nothing to launch whose report shows that the rebuild's copy of the
+      // positions is done: wait for it, so that the caller may overwrite them
+      // and a later call on any stream finds the reference.
       m_last_ = 0;
-      return Status{NLB_OK};
+      const cudaError_t e = cudaStreamSynchronize(c.stream);
+      return e == cudaSuccess ? Status{NLB_OK} : cuda_fail(e, "Verlet rebuild");
     }
     EdgeExtrasCell cell{};
     if (has_cell_) {
