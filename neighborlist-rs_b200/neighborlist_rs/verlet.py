@@ -48,6 +48,16 @@ def _is_cuda_tensor(x) -> bool:
     return isinstance(x, torch.Tensor) and x.is_cuda
 
 
+def _cuda_positions(positions):
+    import torch
+
+    if positions.dtype != torch.float64 or positions.dim() != 2:
+        raise TypeError("positions must be a CUDA float64 tensor of shape (N, 3)")
+    if positions.shape[1] != 3:
+        raise ValueError("Positions must be (N, 3)")
+    return positions.contiguous()
+
+
 class VerletList:
     """Skin-list manager on the current CUDA device (see the module doc)."""
 
@@ -79,11 +89,7 @@ class VerletList:
         if _is_cuda_tensor(positions):
             import torch
 
-            if positions.dtype != torch.float64 or positions.dim() != 2:
-                raise TypeError("positions must be a CUDA float64 tensor of shape (N, 3)")
-            if positions.shape[1] != 3:
-                raise ValueError("Positions must be (N, 3)")
-            pos = positions.contiguous()
+            pos = _cuda_positions(positions)
             dev = pos.device
             with _on_stream_of(pos) as stream:
                 r = _DevResult()
@@ -111,18 +117,21 @@ class VerletList:
     def needs_rebuild(self, cell, positions) -> bool:
         """Whether the next update with these positions rebuilds; sets
         ``max_displacement`` (inf when the system changed or there is no
-        list yet)."""
+        list yet).  A CUDA tensor is read on the current torch stream."""
         h, pb = _cell_args(cell)
         needs = ctypes.c_int(1)
         disp = ctypes.c_double(0.0)
         if _is_cuda_tensor(positions):
-            pos = positions.contiguous()
-            ptr, n, on_dev = ctypes.c_void_p(pos.data_ptr()), pos.shape[0], 1
+            pos = _cuda_positions(positions)
+            with _on_stream_of(pos):
+                _check(_lib.nlb_verlet_needs_rebuild(
+                    self._handle(), ctypes.c_void_p(pos.data_ptr()), pos.shape[0], h, pb, 1,
+                    ctypes.byref(needs), ctypes.byref(disp)))
         else:
             pos = _positions(positions)
-            ptr, n, on_dev = ctypes.c_void_p(pos.ctypes.data), pos.shape[0], 0
-        _check(_lib.nlb_verlet_needs_rebuild(self._handle(), ptr, n, h, pb, on_dev,
-                                             ctypes.byref(needs), ctypes.byref(disp)))
+            _check(_lib.nlb_verlet_needs_rebuild(
+                self._handle(), ctypes.c_void_p(pos.ctypes.data), pos.shape[0], h, pb, 0,
+                ctypes.byref(needs), ctypes.byref(disp)))
         self.max_displacement = disp.value
         return bool(needs.value)
 
