@@ -629,7 +629,7 @@ def device_blocks() -> dict:
 
 
 _LEGACY_STREAM = 1  # cudaStreamLegacy
-_default_streams: dict = {}  # device index -> torch's default stream there
+_streams: dict = {}  # (device index, raw handle) -> torch's stream object, at most 64
 
 
 class _on_stream_of:
@@ -642,8 +642,8 @@ class _on_stream_of:
     which the library would take for its own), so the build follows the work
     that made the positions and returns when the list's size is known.  The
     last kernels may still read the positions then: a tensor that was
-    allocated on another stream is kept from reuse until they are done
-    (record_stream; 0.6 us)."""
+    allocated on another stream than the current one is kept from reuse until
+    they are done (record_stream; 0.6 us)."""
 
     __slots__ = ("tensor", "dev", "guard")
 
@@ -658,14 +658,21 @@ class _on_stream_of:
         if torch.cuda.current_device() != self.dev.index:
             self.guard = torch.cuda.device(self.dev)
             self.guard.__enter__()
-        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-        stream = (raw(self.dev.index) if raw is not None
-                  else torch.cuda.current_stream(self.dev).cuda_stream)
-        if stream == 0:
-            default = _default_streams.get(self.dev.index)
-            if default is None:
-                default = _default_streams[self.dev.index] = torch.cuda.default_stream(self.dev)
-            self.tensor.record_stream(default)
+        try:
+            raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+            stream = (raw(self.dev.index) if raw is not None
+                      else torch.cuda.current_stream(self.dev).cuda_stream)
+            key = (self.dev.index, stream)
+            current = _streams.get(key)
+            if current is None:
+                if len(_streams) >= 64:
+                    _streams.clear()
+                current = _streams[key] = torch.cuda.current_stream(self.dev)
+            self.tensor.record_stream(current)
+        except BaseException:
+            if self.guard is not None:
+                self.guard.__exit__(None, None, None)
+            raise
         _lib.nlb_set_stream(stream or _LEGACY_STREAM)
         return stream
 
