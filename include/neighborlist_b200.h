@@ -357,7 +357,10 @@ int nlb_build_noalloc(const double* d_positions, int64_t n_atoms, double cutoff,
  *   has its message).  Host results then belong to the caller (nlb_result_free) and
  *   the ticket is retired; device results stay owned by the server until
  *   nlb_server_release, which the caller issues once its own work reading
- *   them has completed.
+ *   them has completed, or after nlb_server_follow.
+ * nlb_server_follow: memory of device results freed from now on is not used
+ *   again before the work queued so far on `stream` (NULL: the legacy default
+ *   stream of the server's device) is done.
  * nlb_server_stats: fills 16 counters: submitted, completed, failed, batches,
  *   HBM bytes reserved, queued requests, largest batch, budget, then worker
  *   wall time in microseconds (all workers) spent in: batch staging and
@@ -387,6 +390,7 @@ int64_t nlb_server_submit(nlb_server* server, const double* positions, int64_t n
 int nlb_server_wait(nlb_server* server, int64_t ticket, double timeout_s, nlb_result* out,
                     double* latency_ms);
 int nlb_server_release(nlb_server* server, int64_t ticket);
+int nlb_server_follow(nlb_server* server, void* stream);
 int nlb_server_pause(nlb_server* server, int paused);
 int nlb_server_cancel(nlb_server* server, int64_t ticket);
 int nlb_server_debug_fail(nlb_server* server, int64_t ticket);

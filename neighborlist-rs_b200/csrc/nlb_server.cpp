@@ -144,6 +144,7 @@ class Server {
       e = cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&free_stream_, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&follow_ev_, cudaEventDisableTiming);
     if (e != cudaSuccess) {
       cuda_fail(e, "device result pool");
       return false;
@@ -188,6 +189,7 @@ class Server {
       cudaStreamSynchronize(free_stream_);
       cudaStreamDestroy(free_stream_);
     }
+    if (follow_ev_) cudaEventDestroy(follow_ev_);
     if (pool_) cudaMemPoolDestroy(pool_);
   }
 
@@ -340,6 +342,25 @@ class Server {
     free_req(r);
     cv_work_.notify_all();
     return NLB_OK;
+  }
+
+  // Frees of device results from now on wait for the work queued on `stream`.
+  Status follow(cudaStream_t stream) {
+    int prev = device_;
+    cudaGetDevice(&prev);
+    if (prev != device_) cudaSetDevice(device_);
+    cudaError_t e;
+    {
+      std::lock_guard<std::mutex> lk(follow_mu_);
+      e = cudaEventRecord(follow_ev_, stream);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(free_stream_, follow_ev_, 0);
+    }
+    if (e != cudaSuccess) {  // (a stream of another device)
+      cudaGetLastError();
+      e = cudaStreamSynchronize(stream);
+    }
+    if (prev != device_) cudaSetDevice(prev);
+    return e == cudaSuccess ? Status{NLB_OK} : cuda_fail(e, "nlb_server_follow");
   }
 
   // Worker wall time (microseconds, all workers) by phase of the batched
@@ -833,6 +854,8 @@ class Server {
   std::mutex dev_mu_;
   std::unordered_map<void*, int64_t> dev_refs_;  // device block -> live result slices
   cudaStream_t free_stream_ = nullptr;
+  std::mutex follow_mu_;
+  cudaEvent_t follow_ev_ = nullptr;
   size_t budget_;
   int max_batch_;
   std::mutex mu_;
@@ -904,6 +927,11 @@ int nlb_server_wait(nlb_server* s, int64_t ticket, double timeout_s, nlb_result*
 int nlb_server_release(nlb_server* s, int64_t ticket) {
   if (!s) return nlb::fail(NLB_ERR_VALUE, "server is NULL").code;
   return s->impl->release(ticket);
+}
+
+int nlb_server_follow(nlb_server* s, void* stream) {
+  if (!s) return nlb::fail(NLB_ERR_VALUE, "server is NULL").code;
+  return s->impl->follow(static_cast<cudaStream_t>(stream)).code;
 }
 
 int nlb_server_pause(nlb_server* s, int paused) {

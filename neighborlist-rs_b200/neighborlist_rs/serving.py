@@ -29,6 +29,7 @@ _lib.nlb_server_submit.restype = ctypes.c_int64
 _lib.nlb_server_wait.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_double,
                                  ctypes.POINTER(_Result), ctypes.POINTER(ctypes.c_double)]
 _lib.nlb_server_release.argtypes = [ctypes.c_void_p, ctypes.c_int64]
+_lib.nlb_server_follow.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
 _lib.nlb_server_stats.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)]
 _lib.nlb_server_pause.argtypes = [ctypes.c_void_p, ctypes.c_int]
 _lib.nlb_server_cancel.argtypes = [ctypes.c_void_p, ctypes.c_int64]
@@ -54,7 +55,9 @@ class DeviceResult:
         self.shift = int(r.shift or 0)
 
     def to_torch(self, device=None):
-        """Copies into new CUDA tensors {"edge_index": (2, M), "shift": (M, 3)}."""
+        """Copies into new CUDA tensors {"edge_index": (2, M), "shift": (M, 3)},
+        on the current torch stream; ``release`` may follow at once, the memory
+        is kept until the copies are done."""
         import torch
 
         from . import _cudart_copy
@@ -67,6 +70,7 @@ class DeviceResult:
             stream = torch.cuda.current_stream(dev).cuda_stream
             _cudart_copy(ei.data_ptr(), self.edge_index, 16 * m, stream)
             _cudart_copy(sh.data_ptr(), self.shift, 12 * m, stream)
+            _check(_lib.nlb_server_follow(self._server._handle(), stream))
         return {"edge_index": ei, "shift": sh}
 
     def release(self) -> None:
