@@ -626,7 +626,6 @@ __global__ void __launch_bounds__(kSortThreads)
                    const __grid_constant__ GridBuffers b) {
   extern __shared__ int32_t s_scan[];
   __shared__ uint64_t warp_tot[kSortThreads / 32];
-  __shared__ int32_t warp_max[kSortThreads / 32];
   const int32_t nb = (int32_t)g.total_bins;
   int32_t* const s_start = s_scan;
   int32_t* const s_group = s_scan + nb + 1;
@@ -640,11 +639,9 @@ __global__ void __launch_bounds__(kSortThreads)
     const int32_t per = (nb + kSortThreads - 1) / kSortThreads;
     const int32_t b0 = min(tid * per, nb), b1 = min(b0 + per, nb);
     uint64_t sum = 0;  // groups above, atoms below
-    int32_t most = 0;
 #pragma unroll 4
     for (int32_t c = b0; c < b1; ++c) {
       const int32_t v = b.bin_count[c];
-      most = max(most, v);
       sum += (uint64_t)((v + 31) / 32) << 32 | (uint64_t)v;
       s_start[c] = v;
     }
@@ -654,11 +651,7 @@ __global__ void __launch_bounds__(kSortThreads)
       const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    most = __reduce_max_sync(0xffffffffu, most);
-    if (lane == 31) {
-      warp_tot[warp] = x;
-      warp_max[warp] = most;
-    }
+    if (lane == 31) warp_tot[warp] = x;
     __syncthreads();
     uint64_t run = x - sum;
     for (int w = 0; w < warp; ++w) run += warp_tot[w];
@@ -673,9 +666,6 @@ __global__ void __launch_bounds__(kSortThreads)
     if (blockIdx.x == 0 && tid == kSortThreads - 1) {
       b.bin_start[nb] = n;
       b.counters[0] = (int32_t)(run >> 32);
-      int32_t top = 0;
-      for (int w = 0; w < kSortThreads / 32; ++w) top = max(top, warp_max[w]);
-      *b.max_bin = top;
     }
     __syncthreads();
   }

@@ -437,7 +437,6 @@ __device__ void finish_list(const GridBuffers& b, const GroupSearch& o, int32_t 
       r[1] = M;
       r[2] = err;
       r[3] = records;
-      r[4] = b.max_bin ? *b.max_bin : 0;
       __threadfence_system();
       r[0] = 1;
     }

@@ -58,7 +58,6 @@ struct FastState {
   int64_t last_m = 0;
   int64_t last_mask_words = 0;
   int64_t last_records = 0;  // records the last group search asked for
-  int64_t bin_n = 0, bin_nb = 0, bin_max = 0;  // largest bin of the last bucket build
 };
 
 thread_local FastState tl_states[16];
@@ -134,7 +133,7 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   // Zeroed block, so that a single memset at the start clears everything and
   // the kernels follow each other directly: bin histogram, scatter cursors, 2
   // task counters, 64-bit mask cursor (8-byte aligned: 2 nb + 2 is even),
-  // build completion count, emit task counter, loose flag, largest bin, then
+  // build completion count, emit task counter, loose flag, a word unused, then
   // (8-byte aligned) the offsets scan's state, or the group search's ticket,
   // error word, total, completion count, record cursor, block sums and segment
   // counts and the bin scan's state.
@@ -153,7 +152,6 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
   b.build_done = zeroed + 2 * nb + 4;
   b.emit_queue = reinterpret_cast<uint32_t*>(zeroed + 2 * nb + 5);
   b.loose = zeroed + 2 * nb + 6;
-  b.max_bin = zeroed + 2 * nb + 7;
   int64_t* state = reinterpret_cast<int64_t*>(zeroed + 2 * nb + 8);
   sp.scan_state = state;
   b.bin_scan = bin_scan ? reinterpret_cast<uint64_t*>(state + group_words) : nullptr;
@@ -387,16 +385,8 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   sp.search.split = sp.grouped ? group_split(sp.n, sp.grid.total_bins, cells) : 0;
   tl_last_pipeline = sp.grouped ? 0 : 1;
   sp.gb.bucket = 0;
-  if (sp.grouped && bucket_build(sp.n, sp.grid.total_bins)) {
-    // Room for four times the mean bin, and for the largest of the last
-    // system of this size; within 64 MB.
-    int64_t most = 4 * sp.n / sp.grid.total_bins;
-    if (fs.bin_n == sp.n && fs.bin_nb == sp.grid.total_bins)
-      most = std::max(most, fs.bin_max + fs.bin_max / 4);
-    int64_t bucket = 32;
-    while (bucket < most) bucket *= 2;
-    if (bucket * sp.grid.total_bins * 12 <= (int64_t)64 << 20) sp.gb.bucket = (int32_t)bucket;
-  }
+  if (sp.grouped && bucket_build(sp.n, sp.grid.total_bins))
+    sp.gb.bucket = bucket_entries(sp.n, sp.grid.total_bins);
   const double rc = std::sqrt(sp.rc_sq[0]);
   int64_t capacity = std::max<int64_t>(
       {4096, (int64_t)(1.25 * (double)fs.last_m), (int64_t)(1.5 * (double)estimate_edges(sp, rc))});
@@ -505,11 +495,6 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
     const int64_t m = r[1];
     if (r[2] != 0) return fail(NLB_ERR_CUDA, "prefix scan gave up waiting for a tile");
     if (sp.grouped) fs.last_records = r[3];
-    if (sp.gb.bucket > 0) {
-      fs.bin_n = sp.n;
-      fs.bin_nb = sp.grid.total_bins;
-      fs.bin_max = r[4];
-    }
     if (m <= capacity && (!sp.grouped || r[3] <= sp.search.chunk_cap)) {
       if (c.stream == c.own_stream) {
         if (!stream_ordered) {

@@ -109,12 +109,10 @@ struct GridBuffers {
   // (bin_scan_words(total_bins), zeroed by the caller before the build; used
   // when group_start is set); [1] is its error word.
   uint64_t* bin_scan;
-  // Bucket build (bucket > 0; see bucket_build): k_prep puts every atom
+  // Bucket build (bucket > 0; see bucket_build): k_prep_bucket puts every atom
   // straight into its bin's bucket (skey, sidx: total_bins x bucket entries),
-  // and the placement scans the histogram itself.  max_bin receives the
-  // largest bin's count.
+  // and the placement scans the histogram itself.
   int32_t bucket;
-  int32_t* max_bin;
 };
 
 // Systems that take the bucket build: small ones, where the launches saved
@@ -123,6 +121,19 @@ struct GridBuffers {
 // compares with every atom of the system).
 inline bool bucket_build(int64_t n, int64_t total_bins) {
   return n <= 32768 && total_bins <= 3072;
+}
+// Entries of a bucket: all atoms where that fits, else as many as 16 MB hold (at
+// least 432), so that a bin above its bucket holds some 40 times the mean or
+// more.  (With room for four times the mean, two phases of different density or
+// a molecule in its box had such bins and compared each of their atoms with all
+// others: 15,000 atoms in two phases at rc 6 250 -> 122 us, 10,000 156 -> 92,
+// 2,000 isolated atoms at rc 14 94 -> 71, uniform systems unchanged.)  The room
+// costs nothing but memory, since only the filled entries are touched; an odd
+// multiple of 16 keeps the buckets' heads apart in the caches.
+inline int32_t bucket_entries(int64_t n, int64_t total_bins) {
+  const int64_t room = ((int64_t)16 << 20) / (12 * total_bins);
+  const int64_t lines = (room < n ? room : n + 15) / 16;
+  return (int32_t)(16 * (lines % 2 ? lines : (room < n ? lines - 1 : lines + 1)));
 }
 
 // Grids with at least this many atoms per bin on average get chunk boxes.
