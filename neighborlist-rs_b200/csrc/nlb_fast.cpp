@@ -235,6 +235,12 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
 //     to nine), more describe the cells again (81 us with twelve); slices of
 //     at least 24 candidates (1000 isolated atoms: 70 us with 16 to 24, 78
 //     with 64; a cell of 60 atoms: 58 with 16, 57 with 24 to 32).
+//   * Runs of cells (more than 32 of them: narrow cells) of at least 96
+//     candidates: a segment per cell, of one to ten candidates in a cell of a
+//     few atoms, left the group's last warp up to 729 segments to add up (1
+//     atom in a skewed cell at rc 7: 69 us, 51 with 48 candidates, 53 with 96;
+//     16 atoms at rc 20: 74, 60, 58, and 66 with 24; 100 at rc 25: 71 with
+//     either; a limit of 64 runs 114).
 //   * Large bins (above kSplitDense atoms): slices of about 192 candidates, up
 //     to 18,000 segments.  A slice near the group is all hits, and a warp with
 //     a whole cell of them was the last to end by far (10,008 atoms at rc 14:
@@ -243,14 +249,15 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
 //     384).
 constexpr double kSplitDense = 64.0;
 constexpr int64_t kSplitTarget = 5000, kSplitDenseTarget = 18000;
-constexpr int64_t kSplitLeast = 24, kSplitSlice = 192;
+constexpr int64_t kSplitLeast = 24, kSplitCells = 96, kSplitSlice = 192;
 int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
   const int64_t groups = n / 32 + std::min<int64_t>(n, nb) + 1;  // (at most)
   const int64_t row = (int64_t)((double)cells * (double)n / (double)nb);  // candidates of a group
   int64_t want = kSplitTarget / groups;
   if ((double)n > kSplitDense * (double)nb)
     want = std::max(want, std::min(row / kSplitSlice, kSplitDenseTarget / groups));
-  want = std::min({want, cells <= 32 ? row / kSplitLeast : cells, ((int64_t)1 << 30) / groups});
+  want = std::min({want, cells <= 32 ? row / kSplitLeast : std::min(cells, row / kSplitCells),
+                   ((int64_t)1 << 30) / groups});
   return (int32_t)std::max<int64_t>(want, 1);
 }
 
