@@ -254,7 +254,7 @@ struct FastBatchArgs {
   int64_t* d_bounds;  // nullptr: no per-system offsets
   BatchItems bw;
   int64_t cap;
-  bool use_rec;          // up to four lists: count pass records hits, expansion writes the lists
+  bool use_rec;          // records_pay: count pass records hits, expansion writes the lists
   BatchRecords rec;
   int32_t* rec_flags;    // rec.seg_top / overflow / need_recompute (zeroed per batch)
 };
@@ -341,15 +341,34 @@ int64_t arena_capacity(const Ctx& c, int32_t k) {
   return cap;
 }
 
+// Whether a batch with several lists expands records instead of testing again.
+// Tests without a cell are cheap, and among few atoms cheaper than records of
+// them: two lists of systems without a cell, recomputed / expanded, us a call:
+// 300 of 64 atoms 319 / 329, 300 of 100 480 / 488, 64 of 128 222 / 218, 500 of
+// 128 929 / 941, 64 of 200 314 / 303, 20 of 900 617 / 483, 300 of 8 to 256
+// (an atom has 176 in its system) 658 / 644.  With cells records always won
+// (185 of 16 atoms 230 / 212, 20 of 900 724 / 602).
+constexpr int64_t kRecordMates = 112;  // atoms in an atom's system, on average
+bool records_pay(int32_t k, bool any_cell, const std::vector<int64_t>& sizes) {
+  if (k == 1 || any_cell) return k <= kBatchRecordLists;
+  int64_t atoms = 0, mates = 0;
+  for (int64_t n : sizes) {
+    atoms += n;
+    mates += n * n;
+  }
+  return k <= kBatchRecordLists && mates > kRecordMates * atoms;
+}
+
 // The device-sized path for a batch of small systems only (one run).
 // *handled = false (nothing issued) when the batch's kind still has launch
 // shapes to time or phases are being profiled: the caller runs the counted
 // path instead.
 Status run_small_fast(Ctx& c, const double* d_pos, const std::vector<int64_t>& starts,
                       const int64_t* d_starts, const double* d_cells, const uint8_t* d_pbcs,
-                      const uint8_t* d_has, double rc_max, const std::vector<double>& rc_sq,
-                      const std::vector<int32_t>& order, bool disjoint, bool multi,
-                      nlb_result* outs, int64_t* sys_offsets, bool* handled) {
+                      const uint8_t* d_has, bool any_cell, double rc_max,
+                      const std::vector<double>& rc_sq, const std::vector<int32_t>& order,
+                      bool disjoint, bool multi, nlb_result* outs, int64_t* sys_offsets,
+                      bool* handled) {
   *handled = false;
   cudaStream_t s = c.stream;
   const int32_t ns = (int32_t)starts.size() - 1;
@@ -399,7 +418,7 @@ Status run_small_fast(Ctx& c, const double* d_pos, const std::vector<int64_t>& s
   // record holds at least one of a list's <= cap edges.  Without the memory
   // for them the emit pass recomputes.
   const int64_t segs = run_atoms + k * (cap / 32 + 1) + 1024;
-  a.use_rec = k <= kBatchRecordLists && segs <= INT32_MAX / 2;
+  a.use_rec = records_pay(k, any_cell, sizes) && segs <= INT32_MAX / 2;
   if (a.use_rec) {
     a.rec.seg_cap = (int)segs;
     a.rec.seg_hdr = slot<int4>(c, kSlotBatch0 + 13, (size_t)segs * (k > 1 ? 2 : 1));
@@ -656,8 +675,10 @@ Status run_batch(const double* pos, int64_t n, const int32_t* batch, int64_t n_b
   if (all_small) {
     const double t_up = wall_ms();
     bool handled = false;
-    st = run_small_fast(*c, d_pos, starts, d_starts, d_cells, d_pbcs, d_has, rc_max, rc_sq, order,
-                        disjoint, multi, outs, sys_offsets, &handled);
+    const bool any_cell =
+        cells && (!has_cell || std::any_of(has_cell, has_cell + n_sys, [](uint8_t h) { return h; }));
+    st = run_small_fast(*c, d_pos, starts, d_starts, d_cells, d_pbcs, d_has, any_cell, rc_max, rc_sq,
+                        order, disjoint, multi, outs, sys_offsets, &handled);
     if (c->prof && handled) {
       c->prof_host_ms[0] += t_up - t_call;
       c->prof_host_ms[3] += wall_ms() - t_call;
