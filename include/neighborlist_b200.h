@@ -182,9 +182,10 @@ int64_t nlb_graph_replays(void);
 
 /* Single-system, single-cutoff pipeline choice (no counterpart in the
  * reference).  mode 0 (the default): the group search, two launches (count
- * with hit masks, emit); mode 1: the pair-task pipeline, three launches
- * (count, offsets scan, emit).  Both give identical results.  mode < 0 only
- * queries.  Returns the previous mode, or -1 for an unknown mode. */
+ * with hit masks, emit), except for narrow cells of up to 128 atoms (more
+ * than 125 stencil cells, no output options); mode 1, and those: the
+ * pair-task pipeline, three launches (count, offsets scan, emit).  Both give
+ * identical results.  mode < 0 only queries.  Returns the previous mode, or -1 for an unknown mode. */
 int32_t nlb_single_pipeline(int32_t mode);
 /* The pipeline the calling thread's last single-cutoff cell-list build took:
  * 0 = group search, 1 = pair tasks, -1 = none yet. */

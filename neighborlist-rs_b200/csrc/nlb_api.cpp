@@ -968,7 +968,7 @@ Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int
   Status st = plan_system(pos_host, n, cell9, pb, cs, false, false, sp, bptr);
   if (!st.ok()) return st;
   if (fast_eligible(sp)) {
-    const bool direct = ex && flags && takes_group_search(sp);
+    const bool direct = ex && flags && takes_group_search(sp, flags);
     if (direct) {
       sp.ex_flags = flags;
       if (cell9) {

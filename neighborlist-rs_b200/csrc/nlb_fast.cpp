@@ -9,8 +9,9 @@
 // the count's records were too small does it grow them and run the missing
 // passes again.
 //
-// Mode 1 (nlb_single_pipeline) takes the pair-task kernels of the
-// multi-cutoff path instead: count per (atom, stencil cell), scan, emit.
+// Mode 1 (nlb_single_pipeline), and narrow cells of a few atoms, take the
+// pair-task kernels of the multi-cutoff path instead: count per (atom, stencil
+// cell), scan, emit.
 //
 // The first call with a given set of launch parameters runs the work
 // directly; a repeated call with identical parameters (same positions
@@ -237,10 +238,11 @@ Status prepare_fast(Ctx& c, SystemPlan& sp, int64_t capacity, int64_t mask_cap) 
 //     with 64; a cell of 60 atoms: 58 with 16, 57 with 24 to 32).
 //   * Runs of cells (more than 32 of them: narrow cells) of at least 96
 //     candidates: a segment per cell, of one to ten candidates in a cell of a
-//     few atoms, left the group's last warp up to 729 segments to add up (1
+//     few atoms, leaves the group's last warp up to 729 segments to add up (1
 //     atom in a skewed cell at rc 7: 69 us, 51 with 48 candidates, 53 with 96;
-//     16 atoms at rc 20: 74, 60, 58, and 66 with 24; 100 at rc 25: 71 with
-//     either; a limit of 64 runs 114).
+//     16 atoms at rc 20: 74, 60, 58, and 66 with 24; 60 at rc 25: 78, 76, 76,
+//     and 83 with a limit of 64 runs; all without the pair tasks that narrow
+//     cells take unless output options are wanted).
 //   * Large bins (above kSplitDense atoms): slices of about 192 candidates, up
 //     to 18,000 segments.  A slice near the group is all hits, and a warp with
 //     a whole cell of them was the last to end by far (10,008 atoms at rc 14:
@@ -375,8 +377,18 @@ Status wait_report(Ctx& c) {
 //
 // (The group search counts a row of candidates -- at most 32 images of all
 // atoms -- in 32 bits.)
-bool takes_group_search(const SystemPlan& sp) {
-  return fast_eligible(sp) && single_pipeline_mode() == 0 && sp.n < ((int64_t)1 << 26);
+// Narrow cells, whose stencils have hundreds of cells, keep the pair tasks up to
+// 128 atoms: one to four groups leave the group search with long runs of nearly
+// empty cells and one warp that adds them up, while a warp per (group, cell)
+// spreads them over the chip.  Device time of a repeated build, pair tasks / group
+// search, us: 1 atom, 729 cells 39 / 41, 16 atoms, 729 cells 39 / 46, 32 atoms,
+// 343 cells 39 / 46, 60 atoms, 567 cells 48 / 55, 100 atoms, 343 cells 56 / 58;
+// 200 atoms, 245 cells 73 / 64, 100 atoms, 125 cells 54 / 47.  With output
+// options the group search's one pass wins (66 / 62 to 75 / 80 us a call).
+constexpr int64_t kNarrowCells = 125, kNarrowAtoms = 128;
+bool takes_group_search(const SystemPlan& sp, int ex_flags) {
+  if (!fast_eligible(sp) || single_pipeline_mode() != 0 || sp.n >= ((int64_t)1 << 26)) return false;
+  return ex_flags || sp.n > kNarrowAtoms || stencil_cells_of(sp.grid) <= kNarrowCells;
 }
 
 // M reaches the host through host-mapped memory as soon as it is known: when
@@ -388,7 +400,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
                 bool stream_ordered) {
   FastState& fs = state_for(c);
   const int64_t cells = stencil_cells_of(sp.grid);
-  sp.grouped = takes_group_search(sp);
+  sp.grouped = takes_group_search(sp, sp.ex_flags);
   sp.search.split = sp.grouped ? group_split(sp.n, sp.grid.total_bins, cells) : 0;
   tl_last_pipeline = sp.grouped ? 0 : 1;
   sp.gb.bucket = 0;

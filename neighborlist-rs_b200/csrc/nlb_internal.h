@@ -253,10 +253,12 @@ Status device_bounds(Ctx& c, const double* d_pos, int64_t n, double bounds6[6]);
 // report (c.h_report[0] = 1), polling the stream now and then: a stream that
 // failed, or ended without a report, ends the wait with an error.
 Status wait_report(Ctx& c);
-// Whether run_fast takes the group search for this system.
-bool takes_group_search(const SystemPlan& sp);
-// Single-system pipeline choice: 0 = the two-launch group search, 1 = the
-// three-launch pair-task pipeline.
+// Whether run_fast takes the group search for this system, with these output
+// options.
+bool takes_group_search(const SystemPlan& sp, int ex_flags);
+// Single-system pipeline choice: 0 = the two-launch group search (pair tasks
+// for narrow cells of a few atoms), 1 = always the three-launch pair-task
+// pipeline.
 int32_t single_pipeline_mode();
 int32_t set_single_pipeline_mode(int32_t mode);  // returns the previous mode
 // Pipeline of the calling thread's last single-cutoff cell-list build:

@@ -505,8 +505,9 @@ def last_single_pipeline() -> int:
 
 def set_single_pipeline(mode: int | None) -> int:
     """Single-system pipeline: 0 (or None) = the two-launch group search (count
-    with hit masks, emit), 1 = the three-launch pair-task pipeline.  Identical
-    results either way; returns the previous mode."""
+    with hit masks, emit; narrow cells of up to 128 atoms take pair tasks), 1 =
+    always the three-launch pair-task pipeline.  Identical results either way;
+    returns the previous mode."""
     r = int(_lib.nlb_single_pipeline(0 if mode is None else int(mode)))
     if r < 0:
         raise ValueError(f"no single-system pipeline mode {mode}")
