@@ -265,23 +265,31 @@ int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
 
 // Hits the emit pass stages at a time.  A segment whose records hold more is
 // written in several windows, each with its own loads and scan; a larger stage
-// leaves fewer warps on an SM (25 with 1536 hits, 16 with 4096).  The small one
-// is for segments so short that they cannot hold much more (10,008 atoms at
-// rc 6, 5,000 short slices: 54.5 us, 56 to 58 with the large one), and for long launches of groups
-// whose hits fit it: a million atoms at rc 6
-// 763 us, 836 with the large one, 300,000 276 and 293; the large one for the
-// rest: 400,000 atoms at rc 8 895 -> 774 us, 78,000 at rc 14 891 -> 760 (712
-// with 6144, but 100,000 at rc 6 137 -> 146), 10,008 at rc 14 158 -> 145, 30,000
-// at rc 8 113 -> 108, 40,000 at rc 6 84 -> 83; 2048 and 3072 are in between.
+// leaves fewer warps on an SM (25 with 1536 hits, 16 with 4096).  By the most a
+// segment can be expected to hold: all pairs of its slice, or all hits of its
+// group.  The small stage (us a call, small / large stage):
+//   * groups in several segments, up to 2560 hits: 10,008 atoms at rc 6 59.4 /
+//     61.4, 10,000 at rc 5 54.0 / 56.5, at rc 7 65.3 / 67.1, 15,000 at rc 6 63.9 /
+//     66.8, 20,001 with vectors at rc 5 87.2 / 88.9, 2,000 at rc 8 56.0 / 57.2;
+//   * groups in one segment, up to 1024 hits: 40,000 atoms at rc 5 83 / 87,
+//     80,000 107 / 112; at rc 6, with 1,480, some gain and some lose (40,000 97 /
+//     95, 60,000 115 / 119, 100,000 153 / 149);
+//   * long launches of groups whose hits mostly fit it: a million atoms at rc 6
+//     763 / 836, 300,000 276 / 293.
+// The large one for the rest: 400,000 atoms at rc 8 895 / 774, 78,000 at rc 14
+// 891 / 760 (712 with 6144, but 100,000 at rc 6 137 -> 146), 10,008 at rc 14 158
+// / 145, 30,000 at rc 8 113 / 108.
 constexpr int32_t kStageSmall = 1536, kStageLarge = 4096;
+constexpr double kStageSplit = 2560.0, kStageWhole = 1024.0, kStageLong = 2048.0;  // hits
 constexpr int64_t kStageFew = 20000;  // segments
 int32_t group_stage(const SystemPlan& sp) {
   const double hits = 32.0 * (double)estimate_edges(sp, std::sqrt(sp.rc_sq[0])) / (double)sp.n;
   const int64_t items = sp.search.max_groups * sp.search.split;
   const double slice = (double)stencil_cells_of(sp.grid) * (double)sp.n /
                        ((double)sp.grid.total_bins * (double)sp.search.split);
-  if (32.0 * slice <= 2.0 * kStageSmall) return kStageSmall;
-  return items > kStageFew && hits <= 2048.0 ? kStageSmall : kStageLarge;
+  const double most = std::min(32.0 * slice, hits);
+  if (most <= (sp.search.split > 1 ? kStageSplit : kStageWhole)) return kStageSmall;
+  return items > kStageFew && hits <= kStageLong ? kStageSmall : kStageLarge;
 }
 
 // The group search's two launches.
