@@ -202,6 +202,12 @@ int32_t nlb_last_single_pipeline(void);
  * shot; builds whose scan has fewer tiles are unaffected.  Returns NLB_OK,
  * or NLB_ERR_VALUE for tile < 0 or spin_limit < 1. */
 int nlb_debug_scan_stall(int32_t tile, int32_t spin_limit);
+/* Failure-detection hook: `count` of the calling thread's workspace
+ * allocations fail as if the device had no memory, after the next `nth` have
+ * succeeded (count 0: none, which also takes the hook back).  The call that
+ * meets one returns NLB_ERR_NOMEM and the next one is exact again.
+ * Returns NLB_OK, or NLB_ERR_VALUE for a negative argument. */
+int nlb_debug_fail_alloc(int32_t nth, int32_t count);
 
 /* Per-thread phase timing with CUDA events on the launching stream.
  * enable != 0 starts (and resets) it.  nlb_profile_read fills ms[0..3] with

@@ -421,9 +421,11 @@ void* Ctx::raw(int slot, size_t bytes) {
         cudaFree(b.p);
     }
     b = Buf{};
+    if (slot == kSlotRankTab) rank_nb[0] = -1;  // (no table in it, whatever follows)
     const size_t cap = std::max<size_t>(bytes + bytes / 4, 4096);
     cudaMemPool_t pool = result_pool_for(device);
-    if (!pool || cudaMallocFromPoolAsync(&b.p, cap, pool, stream) != cudaSuccess) {
+    if (!pool || take_alloc_failure() ||
+        cudaMallocFromPoolAsync(&b.p, cap, pool, stream) != cudaSuccess) {
       cudaGetLastError();
       b = Buf{};
       return nullptr;
@@ -437,7 +439,18 @@ void* Ctx::raw(int slot, size_t bytes) {
 
 namespace {
 thread_local std::unordered_map<int, Ctx*> tl_ctxs;
+thread_local int32_t tl_fail_skip = 0, tl_fail_count = 0;
 }  // namespace
+
+bool take_alloc_failure() {
+  if (tl_fail_count == 0) return false;
+  if (tl_fail_skip > 0) {
+    --tl_fail_skip;
+    return false;
+  }
+  --tl_fail_count;
+  return true;
+}
 
 void release_thread_ctx() {
   release_fast_states();
@@ -1392,6 +1405,14 @@ int32_t nlb_single_pipeline(int32_t mode) {
   if (mode < 0) return single_pipeline_mode();
   if (mode > 1) return -1;
   return set_single_pipeline_mode(mode);
+}
+
+int nlb_debug_fail_alloc(int32_t nth, int32_t count) {
+  if (nth < 0 || count < 0)
+    return fail(NLB_ERR_VALUE, "nth and count must not be negative").code;
+  tl_fail_skip = nth;
+  tl_fail_count = count;
+  return NLB_OK;
 }
 
 int nlb_debug_scan_stall(int32_t tile, int32_t spin_limit) {

@@ -623,11 +623,12 @@ Status run_brute_rows(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_ou
   // zero)
   const bool fresh = c.bufs[kSlotBruteRows].p == nullptr;
   rows.offs = slot<int64_t>(c, kSlotBruteRows, 2 * (size_t)kBruteRowAtoms + 2);
-  if (!rows.masks || !rows.offs || !out_arrays(c, sp, capacity))
-    return fail(NLB_ERR_NOMEM, "device allocation failed");
   rows.counts = reinterpret_cast<int32_t*>(rows.offs + kBruteRowAtoms + 1);
   rows.done = rows.counts + kBruteRowAtoms;
-  if (fresh) cudaMemsetAsync(rows.done, 0, sizeof(int32_t), c.stream);
+  // (before anything can fail: the next call finds the block there)
+  if (fresh && rows.offs) cudaMemsetAsync(rows.done, 0, sizeof(int32_t), c.stream);
+  if (!rows.masks || !rows.offs || !out_arrays(c, sp, capacity))
+    return fail(NLB_ERR_NOMEM, "device allocation failed");
   c.h_report[0] = 0;
   c.mark(0);
   c.mark(1);

@@ -135,6 +135,9 @@ struct Ctx {
 };
 
 Status get_ctx(Ctx** out);
+// Failure-detection hook: whether the calling thread's next workspace
+// allocation fails (nlb_debug_fail_alloc).
+bool take_alloc_failure();
 // Hands the context's single-system result arrays (slots kSlotOutEi and
 // kSlotOutSh, allocated from the per-device result pool) over to the caller:
 // the context forgets them and its next build allocates fresh ones from the

@@ -45,8 +45,9 @@ struct DevBuf {
       if (p) cudaFree(p);
       p = nullptr;
       cap = 0;
-      if (cudaMalloc(&p, bytes + bytes / 4) != cudaSuccess) {
+      if (take_alloc_failure() || cudaMalloc(&p, bytes + bytes / 4) != cudaSuccess) {
         cudaGetLastError();
+        p = nullptr;
         return nullptr;
       }
       cap = bytes + bytes / 4;
@@ -259,6 +260,7 @@ class Verlet {
     // [done, disp, total, tile bases] and the masks
     const size_t state_cap = state_.cap;
     uint64_t* state = static_cast<uint64_t*>(state_.get(8 * (size_t)(3 + verlet_tiles(m))));
+    if (state_.cap != state_cap) state_clean_ = false;  // (before anything can fail)
     uint32_t* masks = static_cast<uint32_t*>(masks_.get(4 * (size_t)verlet_mask_words(m)));
     if (!written_ && cudaEventCreateWithFlags(&written_, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
@@ -294,7 +296,7 @@ class Verlet {
     list.m = m;
     // (the launch leaves the counters cleared; new ones and a failed launch's
     // are not)
-    if (!state_clean_ || state_.cap != state_cap) cudaMemsetAsync(state, 0, 16, c.stream);
+    if (!state_clean_) cudaMemsetAsync(state, 0, 16, c.stream);
     state_clean_ = false;
     VerletWork work;
     work.done = state;
