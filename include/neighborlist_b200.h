@@ -204,8 +204,9 @@ int32_t nlb_last_single_pipeline(void);
 int nlb_debug_scan_stall(int32_t tile, int32_t spin_limit);
 /* Failure-detection hook: `count` of the calling thread's workspace
  * allocations fail as if the device had no memory, after the next `nth` have
- * succeeded (count 0: none, which also takes the hook back).  The call that
- * meets one returns NLB_ERR_NOMEM and the next one is exact again.
+ * succeeded (count 0: none, which also takes the hook back).  A build whose
+ * search does not find its memory takes one that needs less; any other call
+ * that meets one returns NLB_ERR_NOMEM, and the next one is exact again.
  * Returns NLB_OK, or NLB_ERR_VALUE for a negative argument. */
 int nlb_debug_fail_alloc(int32_t nth, int32_t count);
 

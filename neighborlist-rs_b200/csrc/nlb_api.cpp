@@ -437,6 +437,17 @@ void* Ctx::raw(int slot, size_t bytes) {
   return b.p;
 }
 
+void Ctx::drop(int slot) {
+  Buf& b = bufs[slot];
+  if (!b.p) return;
+  cudaStreamSynchronize(stream);
+  if (b.pooled)
+    cudaFreeAsync(b.p, stream);
+  else
+    cudaFree(b.p);
+  b = Buf{};
+}
+
 namespace {
 thread_local std::unordered_map<int, Ctx*> tl_ctxs;
 thread_local int32_t tl_fail_skip = 0, tl_fail_count = 0;
@@ -993,7 +1004,7 @@ Status half_list_device(Ctx& c, const double* pos_host, const double* d_pos, int
     if (!st.ok()) return st;
     *ei = sp.out_src;
     *sh = sp.out_sh;
-    if (direct) {
+    if (direct && sp.ex_flags) {  // (not written where the workspace did not fit)
       ex->n_edges = flags & NLB_DIRECTED ? 2 * *m : *m;
       ex->edge_index = sp.out_src;
       ex->shift = sp.out_sh;

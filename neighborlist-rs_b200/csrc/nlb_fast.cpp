@@ -399,6 +399,44 @@ bool takes_group_search(const SystemPlan& sp, int ex_flags) {
   return ex_flags || sp.n > kNarrowAtoms || stencil_cells_of(sp.grid) <= kNarrowCells;
 }
 
+// The build without the memory that the searches above ask for: the group
+// search's records, or result arrays by the density's estimate.  FP64 per-atom
+// passes with 12 bytes an atom besides the cell list, and result arrays of
+// exactly M edges; the output options are left to the caller (sp.ex_flags 0).
+Status run_lean(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
+                bool stream_ordered) {
+  FastState& fs = state_for(c);
+  fs.have_key = false;
+  for (int s : {kSlotMasks, kSlotCand, kSlotCshift, kSlotAtomBase, kSlotSegCnt, kSlotSegRec,
+                kSlotTaskHdr, kSlotCounts, kSlotOffs, kSlotSkey, kSlotOutEi, kSlotOutSh,
+                kSlotOutVec, kSlotOutDist})
+    c.drop(s);
+  sp.gb = GridBuffers{};
+  sp.fp32 = false;
+  sp.grouped = false;
+  sp.ex_flags = 0;
+  Status st = count_system(c, sp, d_pos);
+  if (!st.ok()) return st;
+  DevLists L;
+  st = device_outputs(c, sp.m, L);
+  if (!st.ok()) return st;
+  const int64_t zero = 0;
+  st = emit_system(c, sp, d_pos, L, &zero, 0);
+  if (!st.ok()) return st;
+  sp.out_src = L.src[0];
+  sp.out_sh = L.sh[0];
+  if (c.stream == c.own_stream) {
+    const cudaError_t e = stream_ordered ? cudaSuccess : cudaStreamSynchronize(c.stream);
+    if (e != cudaSuccess) return cuda_fail(e, "neighbour-list pipeline");
+  } else {
+    const cudaError_t e = cudaEventRecord(c.early_ev, c.stream);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
+    c.early_stream = c.stream;
+  }
+  *m_out = sp.m[0];
+  return Status{NLB_OK};
+}
+
 // M reaches the host through host-mapped memory as soon as it is known: when
 // the count pass ends (mode 1: when its emit pass starts).  On a caller's
 // stream the call then returns at once: the emit is queued on that stream
@@ -443,6 +481,7 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
                           (int64_t)(c.bufs[kSlotCshift].cap / sizeof(uint32_t))});
   if (mask_have > mask_cap) mask_cap = mask_have;
   Status st = prepare_fast(c, sp, capacity, mask_cap);
+  if (st.code == NLB_ERR_NOMEM) return run_lean(c, sp, d_pos, m_out, stream_ordered);
   if (!st.ok()) return st;
 
   FastKey key;
@@ -573,14 +612,13 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
     // Too little room: grow it (outside any capture) and run what is missing
     // again.  The records: the count pass once more, its state cleared first.
     const int64_t cap2 = m > capacity ? m + m / 8 + 1024 : capacity;
-    if (!out_arrays(c, sp, cap2))
-      return fail(NLB_ERR_NOMEM, "device allocation for the edge lists failed");
+    if (!out_arrays(c, sp, cap2)) return run_lean(c, sp, d_pos, m_out, stream_ordered);
     if (recount) {
       GroupSearch& o = sp.search;
       o.masks = slot<uint32_t>(c, kSlotMasks, 32 * (size_t)records);
       o.cand = slot<uint32_t>(c, kSlotCand, 32 * (size_t)records);
       o.cshift = slot<uint32_t>(c, kSlotCshift, 32 * (size_t)records);
-      if (!o.masks || !o.cand || !o.cshift) return fail(NLB_ERR_NOMEM, "device allocation failed");
+      if (!o.masks || !o.cand || !o.cshift) return run_lean(c, sp, d_pos, m_out, stream_ordered);
       o.chunk_cap = records;
       cudaMemsetAsync(o.state, 0, sizeof(uint64_t) * (size_t)group_state_words(o.max_groups), c.stream);
     }

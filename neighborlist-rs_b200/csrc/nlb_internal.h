@@ -132,6 +132,8 @@ struct Ctx {
   // Returns a device buffer of at least `bytes` for `slot` (contents are not
   // preserved on growth), or nullptr if the allocation failed.
   void* raw(int slot, size_t bytes);
+  // Gives a slot's buffer back to the pool.
+  void drop(int slot);
 };
 
 Status get_ctx(Ctx** out);
@@ -229,6 +231,8 @@ Status plan_system(const double* pos_host, int64_t n, const double* cell9, const
                    const std::vector<double>& cutoffs, bool disjoint, bool multi,
                    SystemPlan& sp, const double* bounds6 = nullptr);
 Status count_system(Ctx& c, SystemPlan& sp, const double* d_pos);
+// Result arrays of exactly m[q] edges per list, each [src | dst].
+Status device_outputs(Ctx& c, const std::vector<int64_t>& m, DevLists& L);
 Status emit_system(Ctx& c, SystemPlan& sp, const double* d_pos, const DevLists& L,
                    const int64_t* base, int64_t index_offset);
 
