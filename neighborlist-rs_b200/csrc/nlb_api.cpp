@@ -407,9 +407,9 @@ void* Ctx::raw(int slot, size_t bytes) {
     // be handed over; the others so that a grown slot's old memory stays
     // mapped for the next allocation instead of being unmapped by cudaFree
     // and mapped again by cudaMalloc).  Growth waits for this context's own
-    // work: every call has either synchronised its stream before it returned
-    // or is followed by this stream (early_ev).  It must not wait for the
-    // whole device: with several server workers making their streams at the
+    // work: every call has synchronised its stream before it returned (one
+    // that failed too: settle) or is followed by this stream (early_ev).  It
+    // must not wait for the whole device: with several server workers making their streams at the
     // same time, cudaDeviceSynchronize crashed inside the driver (a null
     // stream in cuCtxSynchronize, about one process in ten), and it held up
     // every other worker.
@@ -535,6 +535,18 @@ Status get_ctx(Ctx** out) {
   return Status{NLB_OK};
 }
 
+void settle() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  const auto it = tl_ctxs.find(dev);
+  if (it == tl_ctxs.end()) return;
+  Ctx* c = it->second;
+  // (a call that failed before it took its stream leaves an earlier one here)
+  if (c->stream == (tl_user_stream ? tl_user_stream : c->own_stream))
+    cudaStreamSynchronize(c->stream);
+  cudaGetLastError();
+}
+
 // Accumulates the phase times of completed (synchronized) profiled work.
 void Ctx::harvest() {
   float ms = 0.f;
@@ -572,6 +584,7 @@ void ensure_smem_attr(const void* func, int bytes) {
 Status count_system(Ctx& c, SystemPlan& sp, const double* d_pos) {
   const int64_t n = sp.n;
   const int32_t k = (int32_t)sp.rc_sq.size();
+  if (k + 4 > kSmallHost) return fail(NLB_ERR_VALUE, "too many cutoffs");
   cudaStream_t s = c.stream;
   // Count layout: k rows of n + 1 per-atom counts, or (pair tasks) one row of
   // n * S per-(atom, stencil cell) counts plus a trailing zero.
@@ -676,7 +689,6 @@ Status count_system(Ctx& c, SystemPlan& sp, const double* d_pos) {
   exclusive_scan_u32(sp.counts, (int64_t)k * row, sp.offs, scan_tmp, s);
   c.mark(3);
   // Row starts offs[q * row], q = 0..k, in one strided copy.
-  if (k + 4 > kSmallHost) return fail(NLB_ERR_VALUE, "too many cutoffs");
   cudaError_t e = cudaMemcpy2DAsync(c.h_small, sizeof(int64_t), sp.offs, sizeof(int64_t) * row,
                                     sizeof(int64_t), (size_t)k + 1, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)  // the scan's bounded-wait error word
@@ -880,7 +892,10 @@ Status download_results(Ctx& c, const std::vector<int64_t>& m, const DevLists& L
   for (int32_t q = 0; q < k; ++q) {
     nlb_result& r = outs[order[q]];
     Status st = alloc_result(m[q], &r);
-    if (!st.ok()) return st;
+    if (!st.ok()) {
+      cudaStreamSynchronize(c.stream);  // (the caller releases the results queued so far)
+      return st;
+    }
     if (m[q] == 0) continue;
     // [src | dst] in one copy when the destinations follow the sources.
     const bool joined = L.dst[q] == L.src[q] + m[q];
@@ -1253,24 +1268,23 @@ const char* nlb_version(void) { return "neighborlist-b200 0.1.0 (sm_100a)"; }
 int nlb_build(const double* positions, int64_t n_atoms, double cutoff, const double* cell,
               const uint8_t* pbc, int /*parallel*/, nlb_result* out) {
   if (!out) return fail(NLB_ERR_VALUE, "out is NULL").code;
-  return run_single(positions, n_atoms, cell, pbc, &cutoff, 1, false, false, out).code;
+  return done(run_single(positions, n_atoms, cell, pbc, &cutoff, 1, false, false, out));
 }
 
 int nlb_build_multi(const double* positions, int64_t n_atoms, const double* cutoffs,
                     int32_t n_cutoffs, const double* cell, const uint8_t* pbc, int disjoint,
                     nlb_result* outs) {
   if (n_cutoffs > 0 && (!outs || !cutoffs)) return fail(NLB_ERR_VALUE, "outs is NULL").code;
-  return run_single(positions, n_atoms, cell, pbc, cutoffs, n_cutoffs, disjoint != 0, true, outs)
-      .code;
+  return done(run_single(positions, n_atoms, cell, pbc, cutoffs, n_cutoffs, disjoint != 0, true,
+                         outs));
 }
 
 int nlb_build_batch(const double* positions, int64_t n_atoms, const int32_t* batch,
                     int64_t n_batch, double cutoff, const double* cells, const uint8_t* pbcs,
                     const uint8_t* has_cell, int64_t n_cells, int /*parallel*/, nlb_result* out) {
   if (!out) return fail(NLB_ERR_VALUE, "out is NULL").code;
-  return run_batch(positions, n_atoms, batch, n_batch, &cutoff, 1, cells, pbcs, has_cell, n_cells,
-                   false, false, out)
-      .code;
+  return done(run_batch(positions, n_atoms, batch, n_batch, &cutoff, 1, cells, pbcs, has_cell,
+                        n_cells, false, false, out));
 }
 
 int nlb_build_batch_multi(const double* positions, int64_t n_atoms, const int32_t* batch,
@@ -1278,9 +1292,8 @@ int nlb_build_batch_multi(const double* positions, int64_t n_atoms, const int32_
                           const double* cells, const uint8_t* pbcs, const uint8_t* has_cell,
                           int64_t n_cells, int disjoint, nlb_result* outs) {
   if (n_cutoffs > 0 && (!outs || !cutoffs)) return fail(NLB_ERR_VALUE, "outs is NULL").code;
-  return run_batch(positions, n_atoms, batch, n_batch, cutoffs, n_cutoffs, cells, pbcs, has_cell,
-                   n_cells, disjoint != 0, true, outs)
-      .code;
+  return done(run_batch(positions, n_atoms, batch, n_batch, cutoffs, n_cutoffs, cells, pbcs,
+                        has_cell, n_cells, disjoint != 0, true, outs));
 }
 
 int nlb_build_batch_ex(const double* positions, int64_t n_atoms, const int32_t* batch,
@@ -1289,15 +1302,14 @@ int nlb_build_batch_ex(const double* positions, int64_t n_atoms, const int32_t* 
                        int64_t n_cells, int disjoint, int multi, nlb_result* outs,
                        int64_t* system_offsets) {
   if (n_cutoffs > 0 && (!outs || !cutoffs)) return fail(NLB_ERR_VALUE, "outs is NULL").code;
-  return run_batch(positions, n_atoms, batch, n_batch, cutoffs, n_cutoffs, cells, pbcs, has_cell,
-                   n_cells, disjoint != 0, multi != 0, outs, system_offsets)
-      .code;
+  return done(run_batch(positions, n_atoms, batch, n_batch, cutoffs, n_cutoffs, cells, pbcs,
+                        has_cell, n_cells, disjoint != 0, multi != 0, outs, system_offsets));
 }
 
 int nlb_build_ex(const double* positions, int64_t n_atoms, double cutoff, const double* cell,
                  const uint8_t* pbc, int flags, nlb_result_ex* out) {
   if (!out) return fail(NLB_ERR_VALUE, "out is NULL").code;
-  return run_single_ex(positions, nullptr, n_atoms, cell, pbc, cutoff, flags, out).code;
+  return done(run_single_ex(positions, nullptr, n_atoms, cell, pbc, cutoff, flags, out));
 }
 
 int nlb_build_device_ex(const double* d_positions, int64_t n_atoms, double cutoff,
@@ -1309,9 +1321,8 @@ int nlb_build_device_ex(const double* d_positions, int64_t n_atoms, double cutof
   }
   // A non-null placeholder selects the device-result path for empty input.
   static const double kNone = 0.0;
-  return run_single_ex(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell, pbc, cutoff,
-                       flags, out)
-      .code;
+  return done(run_single_ex(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell, pbc, cutoff,
+                            flags, out));
 }
 
 int nlb_build_device_ex_owned(const double* d_positions, int64_t n_atoms, double cutoff,
@@ -1323,9 +1334,8 @@ int nlb_build_device_ex_owned(const double* d_positions, int64_t n_atoms, double
     return fail(NLB_ERR_VALUE, "positions is NULL").code;
   }
   static const double kNone = 0.0;
-  return run_single_ex(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell, pbc, cutoff,
-                       flags, out, true)
-      .code;
+  return done(run_single_ex(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell, pbc, cutoff,
+                            flags, out, true));
 }
 
 void nlb_result_ex_free(nlb_result_ex* r) {
@@ -1355,13 +1365,13 @@ void nlb_pinned_stats(int64_t* out) {
 int nlb_build_device(const double* d_positions, int64_t n_atoms, double cutoff,
                      const double* cell, const uint8_t* pbc, nlb_device_result* out) {
   if (!out) return fail(NLB_ERR_VALUE, "out is NULL").code;
-  return run_single_device(d_positions, n_atoms, cell, pbc, cutoff, out).code;
+  return done(run_single_device(d_positions, n_atoms, cell, pbc, cutoff, out));
 }
 
 int nlb_build_device_owned(const double* d_positions, int64_t n_atoms, double cutoff,
                            const double* cell, const uint8_t* pbc, nlb_device_result* out) {
   if (!out) return fail(NLB_ERR_VALUE, "out is NULL").code;
-  return run_single_device(d_positions, n_atoms, cell, pbc, cutoff, out, true).code;
+  return done(run_single_device(d_positions, n_atoms, cell, pbc, cutoff, out, true));
 }
 
 int nlb_device_free(void* p, void* stream) {

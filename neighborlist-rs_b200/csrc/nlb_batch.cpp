@@ -103,6 +103,7 @@ Status run_small(Ctx& c, const double* d_pos, const std::vector<int64_t>& starts
   cudaStream_t s = c.stream;
   const int32_t ns = b - a;
   const int32_t k = (int32_t)rc_sq.size();
+  if (k + 3 > kSmallHost) return fail(NLB_ERR_VALUE, "too many cutoffs");
   const int64_t run_start = starts[a];
   const int64_t run_atoms = starts[b] - run_start;
   const int64_t row = run_atoms + 1;
@@ -156,7 +157,6 @@ Status run_small(Ctx& c, const double* d_pos, const std::vector<int64_t>& starts
     cudaMemcpyAsync(run_bounds.data(), d_bounds, sizeof(int64_t) * run_bounds.size(),
                     cudaMemcpyDeviceToHost, s);
   }
-  if (k + 3 > kSmallHost) return fail(NLB_ERR_VALUE, "too many cutoffs");
   cudaError_t e = cudaMemcpy2DAsync(c.h_small, sizeof(int64_t), offs, sizeof(int64_t) * row,
                                     sizeof(int64_t), (size_t)k + 1, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)
@@ -373,6 +373,7 @@ Status run_small_fast(Ctx& c, const double* d_pos, const std::vector<int64_t>& s
   cudaStream_t s = c.stream;
   const int32_t ns = (int32_t)starts.size() - 1;
   const int32_t k = (int32_t)rc_sq.size();
+  if (k + 4 > kSmallHost) return fail(NLB_ERR_VALUE, "too many cutoffs");
   const int64_t run_atoms = starts[ns];
   std::vector<int64_t> sizes(ns);
   for (int32_t i = 0; i < ns; ++i) sizes[i] = starts[i + 1] - starts[i];
@@ -490,7 +491,6 @@ Status run_small_fast(Ctx& c, const double* d_pos, const std::vector<int64_t>& s
   const double t_issue = wall_ms();
   // One synchronisation: list totals, plan errors, the scan's error word,
   // per-system offsets.
-  if (k + 4 > kSmallHost) return fail(NLB_ERR_VALUE, "too many cutoffs");
   cudaError_t e = cudaMemcpy2DAsync(c.h_small, sizeof(int64_t), a.offs, sizeof(int64_t) * a.row,
                                     sizeof(int64_t), (size_t)k + 1, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)

@@ -137,6 +137,15 @@ struct Ctx {
 };
 
 Status get_ctx(Ctx** out);
+// Waits for what a failed call left queued on the calling thread's active
+// stream: it may still use the workspace, which the next call may use, and
+// free, on another stream.
+void settle();
+// The code of a call that ends with st.
+inline int done(const Status& st) {
+  if (st.code == NLB_ERR_NOMEM || st.code == NLB_ERR_CUDA) settle();
+  return st.code;
+}
 // Failure-detection hook: whether the calling thread's next workspace
 // allocation fails (nlb_debug_fail_alloc).
 bool take_alloc_failure();

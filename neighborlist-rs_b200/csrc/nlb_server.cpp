@@ -479,16 +479,23 @@ class Server {
         const double t0 = now_s();
         st[0] = run_large(items[0]);
         us_large += us_since(t0);
-        if (!st[0].ok()) msg[0] = g_last_error;
+        if (!st[0].ok()) {
+          settle();  // (copies into the results that are freed below)
+          msg[0] = g_last_error;
+        }
       } else {
         const Status all = run_batch_items(items);
+        if (!all.ok()) settle();
         if (!all.ok() && items.size() > 1) {
           // Rerun one by one so that only the offending request fails.
           for (size_t i = 0; i < items.size(); ++i) {
             discard(items[i]);
             std::vector<Req*> one(1, items[i]);
             st[i] = run_batch_items(one);
-            if (!st[i].ok()) msg[i] = g_last_error;
+            if (!st[i].ok()) {
+              settle();
+              msg[i] = g_last_error;
+            }
           }
         } else if (!all.ok()) {
           st[0] = all;

@@ -385,12 +385,12 @@ int nlb_verlet_update(nlb_verlet* v, const double* positions, int64_t n_atoms, c
   static const double kNone = 0.0;
   nlb::Status st = v->impl->update(positions ? positions : &kNone, nullptr, n_atoms, cell, pbc,
                                    rebuilt, &m, &ei, &sh, false, true);
-  if (!st.ok()) return st.code;
+  if (!st.ok()) return nlb::done(st);
   st = nlb::alloc_result(m, out);
-  if (!st.ok()) return st.code;
+  if (!st.ok()) return nlb::done(st);
   nlb::Ctx* c = nullptr;
   st = nlb::get_ctx(&c);
-  if (!st.ok()) return st.code;
+  if (!st.ok()) return nlb::done(st);
   cudaError_t e = cudaSuccess;
   if (m > 0) {
     e = cudaMemcpyAsync(out->edge_index, ei, 16 * (size_t)m, cudaMemcpyDeviceToHost, c->stream);
@@ -400,7 +400,7 @@ int nlb_verlet_update(nlb_verlet* v, const double* positions, int64_t n_atoms, c
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     nlb_result_free(out);
-    return nlb::cuda_fail(e, "result copy").code;
+    return nlb::done(nlb::cuda_fail(e, "result copy"));
   }
   return NLB_OK;
 }
@@ -419,7 +419,7 @@ int nlb_verlet_update_device(nlb_verlet* v, const double* d_positions, int64_t n
   static const double kNone = 0.0;
   nlb::Status st = v->impl->update(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell,
                                    pbc, rebuilt, &m, &ei, &sh, false, false);
-  if (!st.ok()) return st.code;
+  if (!st.ok()) return nlb::done(st);
   out->n_edges = m;
   out->edge_index = ei;
   out->shift = sh;
@@ -440,7 +440,7 @@ int nlb_verlet_update_device_owned(nlb_verlet* v, const double* d_positions, int
   static const double kNone = 0.0;
   nlb::Status st = v->impl->update(nullptr, d_positions ? d_positions : &kNone, n_atoms, cell,
                                    pbc, rebuilt, &m, &ei, &sh, true, false);
-  if (!st.ok()) return st.code;
+  if (!st.ok()) return nlb::done(st);
   if (m == 0) {
     // (blocks sized for a non-empty stored list, but nothing was kept)
     nlb::Ctx* c = nullptr;
@@ -460,11 +460,9 @@ int nlb_verlet_needs_rebuild(nlb_verlet* v, const double* positions, int64_t n_a
                              const double* cell, const uint8_t* pbc, int positions_on_device,
                              int* needs, double* max_displacement) {
   if (!v || !needs || !max_displacement) return nlb::fail(NLB_ERR_VALUE, "NULL argument").code;
-  return v->impl
-      ->needs_rebuild(positions_on_device ? nullptr : positions,
-                      positions_on_device ? positions : nullptr, n_atoms, cell, pbc, needs,
-                      max_displacement)
-      .code;
+  return nlb::done(v->impl->needs_rebuild(positions_on_device ? nullptr : positions,
+                                          positions_on_device ? positions : nullptr, n_atoms, cell,
+                                          pbc, needs, max_displacement));
 }
 
 void nlb_verlet_stats(nlb_verlet* v, int64_t* stats) {

@@ -148,3 +148,30 @@ def test_every_allocation_of_a_skin_list(nl, oracle):
 
     for nth in range(0, 60, 1):
         in_thread(lambda: attempt(nth))
+
+
+def test_the_next_call_may_take_another_stream(nl, oracle):
+    """A call that fails has waited for what it queued: the next one frees and
+    writes the same workspace on another stream."""
+    import torch
+
+    sides = [torch.cuda.Stream() for _ in range(2)]
+    systems = []
+    for kind in ("brute", "bucket", "bins"):
+        pos, rows, rc = system(kind)
+        systems.append((nl.PyCell(rows.tolist()), torch.from_numpy(pos).cuda(), rc,
+                        oracle.search_single(pos, rows, PBC3, rc, nthreads=8)))
+    torch.cuda.synchronize()
+
+    def attempt(nth):
+        for k, (cell, pos, rc, ref) in enumerate(systems):  # (each larger: the workspace grows)
+            assert nl._lib.nlb_debug_fail_alloc(nth, 1000) == 0
+            with torch.cuda.stream(sides[k % 2]), pytest.raises(RuntimeError, match="alloc"):
+                nl.build_neighborlists_torch(cell, pos, rc, vectors=True)
+            assert nl._lib.nlb_debug_fail_alloc(0, 0) == 0
+            with torch.cuda.stream(sides[(k + 1) % 2]):
+                r = nl.build_neighborlists_torch(cell, pos, rc)
+                assert_same({q: v.cpu().numpy() for q, v in r.items()}, ref, f"{nth}, {k}")
+
+    for nth in (0, 1, 2, 3):
+        in_thread(lambda: attempt(nth))
