@@ -263,6 +263,28 @@ int32_t group_split(int64_t n, int64_t nb, int64_t cells) {
   return (int32_t)std::max<int64_t>(want, 1);
 }
 
+// Records the group search asks room for: one per 32 candidates of a segment,
+// with the groups and candidates of a uniform density.
+int64_t group_records(int64_t n, int64_t nb, int64_t cells, int32_t split) {
+  const double per_bin = (double)n / (double)nb;
+  const double filled = (double)nb * (1.0 - std::exp(-per_bin));
+  const double groups = std::max(filled, (double)n / 32.0 + 0.5 * filled) + 1.0;
+  const double records = groups * ((double)cells * per_bin / 32.0 + split);
+  return (int64_t)std::min(1.25 * records, 1e12) + 64 * kGroupRegions;
+}
+
+double group_search_bytes(int64_t n, double volume, double rc) {
+  // (bins at least rc wide, 27 stencil cells)
+  const double bins = volume / (rc * rc * rc);
+  const int64_t nb = bins > 1.0 ? (int64_t)std::min(bins, 1e9) : 1;
+  const int32_t split = group_split(n, nb, 27);
+  const double groups = (double)n / 32.0 + (double)std::min<int64_t>(n, nb) + 1.0;
+  double bytes = 384.0 * (double)group_records(n, nb, 27, split) +  // masks, candidates, shifts
+                 groups * (280.0 + 144.0 * split);                  // offsets, segment counts
+  if (bucket_build(n, nb)) bytes += 12.0 * (double)nb * bucket_entries(n, nb);
+  return 1.25 * bytes;
+}
+
 // Hits the emit pass stages at a time.  A segment whose records hold more is
 // written in several windows, each with its own loads and scan; a larger stage
 // leaves fewer warps on an SM (25 with 1536 hits, 16 with 4096).  By the most a
@@ -464,17 +486,13 @@ Status run_fast(Ctx& c, SystemPlan& sp, const double* d_pos, int64_t* m_out,
   if (sp.ex_flags & NLB_DISTANCES) have = std::min(have, c.bufs[kSlotOutDist].cap / sizeof(double));
   if ((int64_t)(have / per) > capacity) capacity = (int64_t)(have / per);
   // Hit-mask arena: the last run's need x 1.25, at least 64 words per atom;
-  // the group search's records (32 words each): one per 32 candidates of a
-  // segment, with the groups and candidates of a uniform density.
+  // the group search's records (32 words each) by the density, or the last
+  // run's need.
   int64_t mask_cap = std::max<int64_t>(64 * sp.n + 4096, fs.last_mask_words + fs.last_mask_words / 4);
-  if (sp.grouped) {
-    const double per_bin = (double)sp.n / (double)sp.grid.total_bins;
-    const double filled = (double)sp.grid.total_bins * (1.0 - std::exp(-per_bin));
-    const double groups = std::max(filled, (double)sp.n / 32.0 + 0.5 * filled) + 1.0;
-    const double records = groups * ((double)cells * per_bin / 32.0 + sp.search.split);
-    mask_cap = 32 * std::max<int64_t>((int64_t)std::min(1.25 * records, 1e12) + 64 * kGroupRegions,
-                                      fs.last_records + fs.last_records / 8);
-  }
+  if (sp.grouped)
+    mask_cap = 32 * std::max<int64_t>(
+                        group_records(sp.n, sp.grid.total_bins, cells, sp.search.split),
+                        fs.last_records + fs.last_records / 8);
   int64_t mask_have = (int64_t)(c.bufs[kSlotMasks].cap / sizeof(uint32_t));
   if (sp.grouped)
     mask_have = std::min({mask_have, (int64_t)(c.bufs[kSlotCand].cap / sizeof(uint32_t)),

@@ -272,6 +272,9 @@ Status wait_report(Ctx& c);
 // Whether run_fast takes the group search for this system, with these output
 // options.
 bool takes_group_search(const SystemPlan& sp, int ex_flags);
+// Workspace of the group search for n atoms in a volume, besides the cell
+// list's (an estimate, with room to grow).
+double group_search_bytes(int64_t n, double volume, double rc);
 // Single-system pipeline choice: 0 = the two-launch group search (pair tasks
 // for narrow cells of a few atoms), 1 = always the three-launch pair-task
 // pipeline.

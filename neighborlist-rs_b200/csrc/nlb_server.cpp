@@ -88,10 +88,11 @@ size_t block_class(size_t bytes) {
   return c;
 }
 
-// Returns the estimated device footprint; sets *result to the estimated
-// result bytes.
-size_t estimate_bytes(const Req& r, size_t* result) {
-  *result = 0;
+// Returns the estimated device footprint (positions, cell list, result); sets
+// *result to the estimated result bytes and *search to those of the
+// single-system search of a large request.
+size_t estimate_bytes(const Req& r, size_t* result, size_t* search) {
+  *result = *search = 0;
   if (r.n == 0) return 4096;
   // Density-based edge estimate: half the neighbours within rc at the mean
   // density of the system's box (its cell, or the auto-box of its span).
@@ -116,6 +117,8 @@ size_t estimate_bytes(const Req& r, size_t* result) {
   const double edges = 1.3 * (double)r.n * per_atom + 64.0;
   const double work = 24.0 * r.n + 220.0 * r.n + 12.0 * 27.0 * r.n;
   *result = (size_t)std::min(edges * 28.0, 1e15);
+  if (r.n > kBatchMaxAtoms)
+    *search = (size_t)std::min(group_search_bytes(r.n, vol, r.rc), 1e15);
   return (size_t)std::min(edges * 28.0 + work, 1e15);
 }
 
@@ -234,12 +237,16 @@ class Server {
       }
       std::memcpy(r->pos, pos, sizeof(double) * 3 * (size_t)n);
     }
-    r->est_bytes = estimate_bytes(*r, &r->est_result);
+    size_t search = 0;
+    r->est_bytes = estimate_bytes(*r, &r->est_result, &search);
     if (r->est_bytes > budget_) {
       free_req(r);
       fail(NLB_ERR_VALUE, "request exceeds the server's HBM budget");
       return -NLB_ERR_VALUE;
     }
+    // (a search that does not find its memory takes one that needs less: its
+    // share is reserved where it can be, but a request runs alone without it)
+    r->est_bytes = std::min(r->est_bytes + search, budget_);
     r->t_submit = now_s();
     std::lock_guard<std::mutex> lk(mu_);
     r->id = next_id_++;
