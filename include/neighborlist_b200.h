@@ -365,10 +365,12 @@ int nlb_build_noalloc(const double* d_positions, int64_t n_atoms, double cutoff,
  *   has its message).  Host results then belong to the caller (nlb_result_free) and
  *   the ticket is retired; device results stay owned by the server until
  *   nlb_server_release, which the caller issues once its own work reading
- *   them has completed, or after nlb_server_follow.
+ *   them has completed, or after nlb_server_follow or nlb_server_copy.
  * nlb_server_follow: memory of device results freed from now on is not used
  *   again before the work queued so far on `stream` (NULL: the legacy default
  *   stream of the server's device) is done.
+ * nlb_server_copy: queues the copies of a device result (edge_index and shift
+ *   of n_edges edges) into the caller's arrays on `stream`, then follows it.
  * nlb_server_stats: fills 16 counters: submitted, completed, failed, batches,
  *   HBM bytes reserved, queued requests, largest batch, budget, then worker
  *   wall time in microseconds (all workers) spent in: batch staging and
@@ -399,6 +401,8 @@ int nlb_server_wait(nlb_server* server, int64_t ticket, double timeout_s, nlb_re
                     double* latency_ms);
 int nlb_server_release(nlb_server* server, int64_t ticket);
 int nlb_server_follow(nlb_server* server, void* stream);
+int nlb_server_copy(nlb_server* server, int64_t* dst_edge_index, const int64_t* edge_index,
+                    int32_t* dst_shift, const int32_t* shift, int64_t n_edges, void* stream);
 int nlb_server_pause(nlb_server* server, int paused);
 int nlb_server_cancel(nlb_server* server, int64_t ticket);
 int nlb_server_debug_fail(nlb_server* server, int64_t ticket);

@@ -948,6 +948,19 @@ int nlb_server_follow(nlb_server* s, void* stream) {
   return s->impl->follow(static_cast<cudaStream_t>(stream)).code;
 }
 
+int nlb_server_copy(nlb_server* s, int64_t* dst_edge_index, const int64_t* edge_index,
+                    int32_t* dst_shift, const int32_t* shift, int64_t n_edges, void* stream) {
+  if (!s) return nlb::fail(NLB_ERR_VALUE, "server is NULL").code;
+  if (n_edges <= 0) return NLB_OK;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemcpyAsync(dst_edge_index, edge_index, 16 * (size_t)n_edges,
+                                  cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(dst_shift, shift, 12 * (size_t)n_edges, cudaMemcpyDeviceToDevice, st);
+  if (e != cudaSuccess) return nlb::cuda_fail(e, "nlb_server_copy").code;
+  return s->impl->follow(st).code;
+}
+
 int nlb_server_pause(nlb_server* s, int paused) {
   if (!s) return nlb::fail(NLB_ERR_VALUE, "server is NULL").code;
   s->impl->pause(paused != 0);

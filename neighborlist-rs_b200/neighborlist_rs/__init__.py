@@ -633,6 +633,14 @@ _LEGACY_STREAM = 1  # cudaStreamLegacy
 _streams: dict = {}  # (device index, raw handle) -> torch's stream object, at most 64
 
 
+def _raw_stream(index: int) -> int:
+    """The current torch stream of a device as its raw handle."""
+    import torch
+
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(index) if raw is not None else torch.cuda.current_stream(index).cuda_stream
+
+
 class _on_stream_of:
     """The device and the current torch stream of a CUDA tensor for the calls
     inside: ``with _on_stream_of(t) as stream``.  The device is switched only
@@ -660,9 +668,7 @@ class _on_stream_of:
             self.guard = torch.cuda.device(self.dev)
             self.guard.__enter__()
         try:
-            raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-            stream = (raw(self.dev.index) if raw is not None
-                      else torch.cuda.current_stream(self.dev).cuda_stream)
+            stream = _raw_stream(self.dev.index)
             key = (self.dev.index, stream)
             current = _streams.get(key)
             if current is None:
@@ -782,11 +788,6 @@ def build_neighborlists_ex(cell, positions, cutoff, directed=False, vectors=Fals
     if distances:
         out["distances"] = _arr(r.distances, m, np.float64)
     return out
-
-
-def _cudart_copy(dst, src, nbytes, stream):
-    _check(_lib.nlb_copy_device(ctypes.c_void_p(dst), ctypes.c_void_p(src), nbytes,
-                                ctypes.c_void_p(stream)))
 
 
 def _torch_ex(cell, positions, cutoff, directed, vectors, distances):

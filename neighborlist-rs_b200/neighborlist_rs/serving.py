@@ -18,8 +18,8 @@ from __future__ import annotations
 import ctypes
 import threading
 
-from . import (_Result, _cell_args, _check, _check_cutoff, _dp, _lib, _positions, _to_dict,
-               _u8p)
+from . import (_Result, _cell_args, _check, _check_cutoff, _dp, _lib, _positions, _raw_stream,
+               _to_dict, _u8p)
 
 _lib.nlb_server_create.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int, ctypes.c_int]
 _lib.nlb_server_create.restype = ctypes.c_void_p
@@ -29,7 +29,8 @@ _lib.nlb_server_submit.restype = ctypes.c_int64
 _lib.nlb_server_wait.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_double,
                                  ctypes.POINTER(_Result), ctypes.POINTER(ctypes.c_double)]
 _lib.nlb_server_release.argtypes = [ctypes.c_void_p, ctypes.c_int64]
-_lib.nlb_server_follow.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+_lib.nlb_server_copy.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+                                 ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]
 _lib.nlb_server_stats.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int64)]
 _lib.nlb_server_pause.argtypes = [ctypes.c_void_p, ctypes.c_int]
 _lib.nlb_server_cancel.argtypes = [ctypes.c_void_p, ctypes.c_int64]
@@ -60,17 +61,14 @@ class DeviceResult:
         is kept until the copies are done."""
         import torch
 
-        from . import _cudart_copy
-
         dev = torch.device("cuda", self._server.device) if device is None else device
         m = self.n_edges
         ei = torch.empty((2, m), dtype=torch.int64, device=dev)
         sh = torch.empty((m, 3), dtype=torch.int32, device=dev)
         if m:
-            stream = torch.cuda.current_stream(dev).cuda_stream
-            _cudart_copy(ei.data_ptr(), self.edge_index, 16 * m, stream)
-            _cudart_copy(sh.data_ptr(), self.shift, 12 * m, stream)
-            _check(_lib.nlb_server_follow(self._server._handle(), stream))
+            _check(_lib.nlb_server_copy(self._server._handle(), ei.data_ptr(), self.edge_index,
+                                        sh.data_ptr(), self.shift, m,
+                                        _raw_stream(ei.device.index)))
         return {"edge_index": ei, "shift": sh}
 
     def release(self) -> None:
