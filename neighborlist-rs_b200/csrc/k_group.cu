@@ -42,10 +42,10 @@
 // which 4,400 the pair tests; emit 112 us against 55 us for writing the same
 // bytes from registers.  A million atoms: 2,110 -> 874 us per call, against
 // one launch that counted, waited for its offsets and moved the destinations
-// (795 with the later changes to loads and segments: count 366, emit 352; the
-// output alone takes 173 us to fill).  The emit is bound by latency and issue
-// (49 % of slots, 20 warps an SM by shared memory; with the candidates packed
-// to four bytes 25 warps and 323 us) rather than by its stores:
+// (761 with the later changes to loads, segments, stage and recheck: count 346,
+// emit 319; the output alone takes 173 us to fill).  The emit is bound by latency
+// and issue (49 % of slots, 20 warps an SM by shared memory: 352 us; with the
+// candidates packed to four bytes 25 warps and 319) rather than by its stores:
 // shifts written as whole sectors, three words a lane exchanged by shuffles
 // (36 -> 12 sector writes per 32 edges), cost 372 us, and masks kept in
 // registers for more warps 375.
