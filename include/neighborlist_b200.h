@@ -368,7 +368,7 @@ int nlb_build_noalloc(const double* d_positions, int64_t n_atoms, double cutoff,
  *   them has completed, or after nlb_server_follow or nlb_server_copy.
  * nlb_server_follow: memory of device results freed from now on is not used
  *   again before the work queued so far on `stream` (NULL: the legacy default
- *   stream of the server's device) is done.
+ *   stream of the current device) is done.
  * nlb_server_copy: queues the copies of a device result (edge_index and shift
  *   of n_edges edges) into the caller's arrays on `stream`, then follows it.
  * nlb_server_stats: fills 16 counters: submitted, completed, failed, batches,

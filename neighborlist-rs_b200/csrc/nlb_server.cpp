@@ -353,9 +353,6 @@ class Server {
 
   // Frees of device results from now on wait for the work queued on `stream`.
   Status follow(cudaStream_t stream) {
-    int prev = device_;
-    cudaGetDevice(&prev);
-    if (prev != device_) cudaSetDevice(device_);
     cudaError_t e;
     {
       std::lock_guard<std::mutex> lk(follow_mu_);
@@ -366,7 +363,6 @@ class Server {
       cudaGetLastError();
       e = cudaStreamSynchronize(stream);
     }
-    if (prev != device_) cudaSetDevice(prev);
     return e == cudaSuccess ? Status{NLB_OK} : cuda_fail(e, "nlb_server_follow");
   }
 

@@ -633,10 +633,8 @@ _LEGACY_STREAM = 1  # cudaStreamLegacy
 _streams: dict = {}  # (device index, raw handle) -> torch's stream object, at most 64
 
 
-def _raw_stream(index: int) -> int:
+def _raw_stream(torch, index: int) -> int:
     """The current torch stream of a device as its raw handle."""
-    import torch
-
     raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
     return raw(index) if raw is not None else torch.cuda.current_stream(index).cuda_stream
 
@@ -668,7 +666,7 @@ class _on_stream_of:
             self.guard = torch.cuda.device(self.dev)
             self.guard.__enter__()
         try:
-            stream = _raw_stream(self.dev.index)
+            stream = _raw_stream(torch, self.dev.index)
             key = (self.dev.index, stream)
             current = _streams.get(key)
             if current is None:

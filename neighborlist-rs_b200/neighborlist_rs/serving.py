@@ -66,9 +66,12 @@ class DeviceResult:
         ei = torch.empty((2, m), dtype=torch.int64, device=dev)
         sh = torch.empty((m, 3), dtype=torch.int32, device=dev)
         if m:
+            if ei.device.index != torch.cuda.current_device():
+                with torch.cuda.device(ei.device):
+                    return self.to_torch(ei.device)
             _check(_lib.nlb_server_copy(self._server._handle(), ei.data_ptr(), self.edge_index,
                                         sh.data_ptr(), self.shift, m,
-                                        _raw_stream(ei.device.index)))
+                                        _raw_stream(torch, ei.device.index)))
         return {"edge_index": ei, "shift": sh}
 
     def release(self) -> None:
