@@ -226,8 +226,10 @@ int64_t nlb_profile_host(double* ms);
  * (cutoff count, power-of-two buckets of the system count, the largest and
  * the mean system, quarter-octave bucket of the largest cutoff): the first
  * batch of a kind runs its count pass once in every candidate shape, timed
- * with CUDA events, and the kind keeps the fastest.  Every shape gives
- * identical results.
+ * with CUDA events, and the kind keeps the fastest.  Batches that leave the
+ * GPU mostly idle (at most 128 atoms per SM in about as many systems as SMs)
+ * are cut finer by a rule instead, without trials, and are no kind of the
+ * tuner's.  Every shape gives identical results.
  *
  * nlb_batch_shape(i) pins shape i (0 = the default) for every batched
  * launch of the process, -1 returns to tuning; it returns the number of

@@ -533,7 +533,8 @@ def batch_shape_info(shape: int) -> dict:
 
 def batch_tuner_state() -> list:
     """One dict per kind of batch seen: its key, the chosen shape (-1: not
-    decided yet) and the number of candidate shapes it was timed in."""
+    decided yet) and the number of candidate shapes it was timed in.  Batches
+    that leave the GPU mostly idle are cut by a rule and are not listed."""
     n = int(_lib.nlb_batch_tuner_state(None, 0))
     buf = np.zeros(8 * max(n, 1), np.int64)
     n = min(n, int(_lib.nlb_batch_tuner_state(buf.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)), n)))
